@@ -198,12 +198,16 @@ LBRB_API int lbrb_set_pairs(lbrb_t *h, int mode);
  * on first use (-1).  Tiles with a one-node ring recomputed around each:
  * 0: 32x8, 1: 32x4, 2: 32x16, 3: 64x4, 4: 32x8 with a thread per node of
  * the tile and its ring, 5: 30x8 likewise, 6: 32x8 at 5 blocks per SM,
- * 7: 32x6, 8: 64x8.  Strips of 32 columns walked down a chunk of rows,
- * recomputing only two halo columns and two rows per chunk (tile_y: rows
- * per group): 9: 8 rows, 3 blocks per SM; 10: 8 rows, 3 blocks, the next
- * group's loads issued before this group's second step (software
- * pipelining); 11: likewise, 2 blocks; 12: 6 rows, 4 blocks, pipelined;
- * 13: 4 rows, 6 blocks, pipelined; 14: 6 rows, 3 blocks, pipelined. */
+ * 7: 32x6, 8: 64x8.  9-14, marching.  FP64: strips of 32 columns walked
+ * down a chunk of rows, recomputing only two halo columns and two rows per
+ * chunk (tile_y: rows per group): 9: 8 rows, 3 blocks per SM; 10: 8 rows,
+ * 3 blocks, the next group's loads issued before this group's second step
+ * (software pipelining); 11: likewise, 2 blocks; 12: 6 rows, 4 blocks,
+ * pipelined; 13: 4 rows, 6 blocks, pipelined; 14: 6 rows, 3 blocks,
+ * pipelined.  FP32: strips of 60 columns, one warp each, two nodes per
+ * thread, walked row by row up a chunk (tile_y: 1): 9-12: 8 warps per SM,
+ * chunks for 1, 2, 3, 6 waves of warps; 13, 14: 12 warps per SM, 4 and 9
+ * waves. */
 LBRB_API int lbrb_set_pair_shape(lbrb_t *h, int shape);
 /* the number of launch shapes of the two-step kernel (0 .. n-1) */
 LBRB_API int lbrb_pair_shapes(void);

@@ -968,6 +968,13 @@ int lbrb_step(lbrb_t* h, int n) {
     h->istep = istep;
     return LBRB_OK;
   };
+  // a nudged run's in-launch sums (the tuner's trials read them too: the
+  // launch with them is another kernel)
+  auto with_sums = [&](auto& V) {
+    if (h->p.nudge != LBRB_NUDGE_BILINEAR) return;
+    V.nmask = h->nmask;
+    V.nacc = reinterpret_cast<const unsigned long long*>(h->acc2);
+  };
   // Two plain steps n, n+1 in one launch (lb_pair_kernel), then the particles
   // of each.  Step n's T goes to the source buffer T[cur] (its particle
   // records read it there), step n+1's to T[cur ^ 1]; u, v of step n go to
@@ -1010,20 +1017,14 @@ int lbrb_step(lbrb_t* h, int n) {
         LBView<float> V1 = make_view<float>(h, src, dst, A, wuv, rec1 ? 1 : 0);
         V1.T = (float*)h->T[src];
         V1.rho = (float*)h->rho[src];
-        if (nud) {
-          V1.nmask = h->nmask;
-          V1.nacc = reinterpret_cast<const unsigned long long*>(h->acc2);
-        }
+        with_sums(V1);
         CK(h, launch_pair_fp32(V1, make_view<float>(h, dst, dst, B, wuv || last, rt2), h->pair_shape, h->stream,
                                pdl_ok));
       } else {
         LBView<double> V1 = make_view<double>(h, src, dst, A, wuv, rec1 ? 1 : 0);
         V1.T = (double*)h->T[src];
         V1.rho = (double*)h->rho[src];
-        if (nud) {
-          V1.nmask = h->nmask;
-          V1.nacc = reinterpret_cast<const unsigned long long*>(h->acc2);
-        }
+        with_sums(V1);
         CK(h, launch_pair_fp64(V1, make_view<double>(h, dst, dst, B, wuv || last, rt2), h->pair_shape, h->stream,
                                pdl_ok));
       }
@@ -1084,9 +1085,11 @@ int lbrb_step(lbrb_t* h, int n) {
       if (!tuned_get(g_tuned_pair, h, &sh, &ms)) {
         if (f32) {
           LBView<float> t1 = make_view<float>(h, src, dst, A, wuv, 0), t2 = make_view<float>(h, dst, dst, B, wuv, 0);
+          with_sums(t1);
           sh = tune_pair_fp32(t1, t2, h->stream, &ms);
         } else {
           LBView<double> t1 = make_view<double>(h, src, dst, A, wuv, 0), t2 = make_view<double>(h, dst, dst, B, wuv, 0);
+          with_sums(t1);
           sh = tune_pair_fp64(t1, t2, h->stream, &ms);
         }
         CK(h, cudaGetLastError());
@@ -2546,15 +2549,17 @@ int lbrb_set_pair_shape(lbrb_t* h, int shape) {
 
 int lbrb_get_pair_shape(const lbrb_t* h, int* shape, int* tile_x, int* tile_y, float* ms) {
   if (!h) return LBRB_ERR_ARG;
-  // (lb_kernels.cu: PAIR_SHAPES, then MARCH_SHAPES: a strip of 32 columns
-  // walked in groups of tile_y rows)
+  // (lb_kernels.cu: PAIR_SHAPES, then for FP64 MARCH_SHAPES: a strip of 32
+  // columns walked in groups of tile_y rows; for FP32 WAVE_SHAPES: strips of
+  // 60 columns, one row at a time)
   static const int TXS[] = {32, 32, 32, 64, 32, 30, 32, 32, 64, 32, 32, 32, 32, 32, 32},
                    TYS[] = {8, 4, 16, 4, 8, 8, 8, 6, 8, 8, 8, 8, 6, 4, 6};
   static_assert(sizeof(TXS) / sizeof(int) == NUM_PAIR_SHAPES, "pair shape table");
   const int sh = h->pair_shape;
   if (shape) *shape = sh;
-  if (tile_x) *tile_x = sh < 0 ? 0 : TXS[sh];
-  if (tile_y) *tile_y = sh < 0 ? 0 : TYS[sh];
+  const bool wave = sh >= NUM_PAIR_TILES && fp32(h);
+  if (tile_x) *tile_x = sh < 0 ? 0 : (wave ? 60 : TXS[sh]);
+  if (tile_y) *tile_y = sh < 0 ? 0 : (wave ? 1 : TYS[sh]);
   if (ms) *ms = h->pair_ms;
   return LBRB_OK;
 }

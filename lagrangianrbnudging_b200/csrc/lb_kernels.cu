@@ -87,6 +87,20 @@ __global__ void __launch_bounds__(32 * (R + 1), MINB)
   march_block<Real, R, PRE, Off>(V1, V2, strip * 32, ya, min(H, V1.ny - ya), march_smem);
 }
 
+template <int NW, int MINB, int D, bool NUD>
+__global__ void __launch_bounds__(32 * NW, MINB)
+    lb_wave2_kernel(const LBView<float> V1, const LBView<float> V2, int H, int nitems) {
+  pdl_wait();
+  extern __shared__ __align__(16) float wave_smem[];
+  const int w = threadIdx.x >> 5, item = blockIdx.x * NW + w;
+  if (item >= nitems) return;
+  const int nstrips = (V1.nx + WAVE_COLS<2> - 1) / WAVE_COLS<2>;
+  const int strip = item % nstrips, ya = item / nstrips * H;
+  wave_march<2, D, NUD>([&](auto s) -> const LBView<float>& { return decltype(s)::value == 0 ? V1 : V2; },
+                        strip * WAVE_COLS<2> + WAVE_X0<2>, min(WAVE_COLS<2>, V1.nx - strip * WAVE_COLS<2>), ya,
+                        min(H, V1.ny - ya), wave_smem + w * wave_smem_floats<2, D>());
+}
+
 // pair launch shapes: (tile columns, tile rows, threads, min blocks per SM)
 struct PairShape { int tx, ty, nt, minb; };
 constexpr PairShape PAIR_SHAPES[] = {{32, 8, 256, 4}, {32, 4, 128, 6}, {32, 16, 512, 2}, {64, 4, 256, 3},
@@ -113,7 +127,7 @@ static cudaError_t launch_pair_t(const LBView<Real>& V1, const LBView<Real>& V2,
   return go(lb_pair_kernel<Real, TX, TY, NT, MB, size_t>);
 }
 
-// marching launch shapes: (rows per group R, min blocks per SM, waves): the
+// FP64 marching launch shapes: (rows per group R, min blocks per SM, waves): the
 // chunk height H = kR - 2 (whole groups) is chosen so that the grid of
 // strips x chunks holds about `waves` waves of resident blocks
 struct MarchShape { int r, minb, waves, pre; };
@@ -151,22 +165,66 @@ static cudaError_t launch_march_t(const LBView<Real>& V1, const LBView<Real>& V2
   return go(lb_march_kernel<Real, R, MB, PRE, size_t>);
 }
 
-template <typename Real>
-static cudaError_t launch_march(const LBView<Real>& V1, const LBView<Real>& V2, int m, cudaStream_t s, bool pdl) {
+// The FP32 marching shapes: wave_march, one warp per strip and chunk, (warps
+// per block, min blocks per SM, waves).  The chunk height is chosen so that
+// the items (strips x chunks) fill at most `waves` waves of resident warps:
+// few waves recompute fewer rows (two per chunk), many keep the warps of a
+// row band together, which the DRAM pages reward.  8 or 12 warps per SM: 15
+// of them (128 registers) ran 10% slower (128 against 118 us per step at
+// 4096x2048), their copies queueing behind one another.
+struct WaveShape { int nw, minb, waves; };
+constexpr WaveShape WAVE_SHAPES[NMARCH] = {{8, 1, 1}, {8, 1, 2}, {8, 1, 3}, {8, 1, 6}, {4, 3, 4}, {4, 3, 9}};
+constexpr int WAVE2_STAGES = 2;  // rows of inputs in flight per warp
+
+template <int NW, int MINB, bool NUD>
+static cudaError_t launch_wave2_t(const LBView<float>& V1, const LBView<float>& V2, int waves, cudaStream_t s,
+                                  bool pdl) {
+  constexpr auto kernel = lb_wave2_kernel<NW, MINB, WAVE2_STAGES, NUD>;
+  constexpr size_t smem = NW * wave_smem_floats<2, WAVE2_STAGES>() * sizeof(float);
+  static std::atomic<unsigned long long> attr_set{0};
+  static std::atomic<int> occ_cache[MAX_DEVICES] = {};
+  cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
+  if (e != cudaSuccess) return e;
+  int occ = 0, dev = 0, nsm = 0;
+  e = occupancy_once((const void*)kernel, 32 * NW, smem, occ_cache, &occ);
+  if (e == cudaSuccess) e = current_device(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int ny = V1.ny;
+  const long nstrips = (V1.nx + WAVE_COLS<2> - 1) / WAVE_COLS<2>;
+  const long chunks = std::min((long)ny, std::max(1L, (long)waves * occ * nsm * NW / nstrips));
+  const int H = (int)((ny + chunks - 1) / chunks);
+  const long nitems = nstrips * ((ny + H - 1) / H);
+  return launch_k(kernel, dim3((unsigned)((nitems + NW - 1) / NW)), 32 * NW, smem, s, pdl, V1, V2, H, (int)nitems);
+}
+
+static cudaError_t launch_wave2(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
+  const WaveShape w = WAVE_SHAPES[m];
+  if (w.nw == 8)
+    return V1.nmask ? launch_wave2_t<8, 1, true>(V1, V2, w.waves, s, pdl)
+                    : launch_wave2_t<8, 1, false>(V1, V2, w.waves, s, pdl);
+  return V1.nmask ? launch_wave2_t<4, 3, true>(V1, V2, w.waves, s, pdl)
+                  : launch_wave2_t<4, 3, false>(V1, V2, w.waves, s, pdl);
+}
+
+static cudaError_t launch_march(const LBView<double>& V1, const LBView<double>& V2, int m, cudaStream_t s, bool pdl) {
   const int waves = MARCH_SHAPES[m].waves;
   switch (m) {
-    case 1: return launch_march_t<Real, 8, 3, true>(V1, V2, waves, s, pdl);
-    case 2: return launch_march_t<Real, 8, 2, true>(V1, V2, waves, s, pdl);
-    case 3: return launch_march_t<Real, 6, 4, true>(V1, V2, waves, s, pdl);
-    case 4: return launch_march_t<Real, 4, 6, true>(V1, V2, waves, s, pdl);
-    case 5: return launch_march_t<Real, 6, 3, true>(V1, V2, waves, s, pdl);
-    default: return launch_march_t<Real, 8, 3, false>(V1, V2, waves, s, pdl);
+    case 1: return launch_march_t<double, 8, 3, true>(V1, V2, waves, s, pdl);
+    case 2: return launch_march_t<double, 8, 2, true>(V1, V2, waves, s, pdl);
+    case 3: return launch_march_t<double, 6, 4, true>(V1, V2, waves, s, pdl);
+    case 4: return launch_march_t<double, 4, 6, true>(V1, V2, waves, s, pdl);
+    case 5: return launch_march_t<double, 6, 3, true>(V1, V2, waves, s, pdl);
+    default: return launch_march_t<double, 8, 3, false>(V1, V2, waves, s, pdl);
   }
+}
+static cudaError_t launch_march(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
+  return launch_wave2(V1, V2, m, s, pdl);
 }
 
 template <typename Real>
 static cudaError_t launch_pair(const LBView<Real>& V1, const LBView<Real>& V2, int shape, cudaStream_t s, bool pdl) {
-  if (shape >= NPAIR) return launch_march<Real>(V1, V2, shape - NPAIR, s, pdl);
+  if (shape >= NPAIR) return launch_march(V1, V2, shape - NPAIR, s, pdl);
   switch (shape) {
     case 1: return launch_pair_t<Real, 32, 4, 128, 6>(V1, V2, s, pdl);
     case 2: return launch_pair_t<Real, 32, 16, 512, 2>(V1, V2, s, pdl);

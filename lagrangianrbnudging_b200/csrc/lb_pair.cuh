@@ -347,4 +347,263 @@ __device__ __forceinline__ void march_block(const LBView<Real>& V1, const LBView
   }
 }
 
+// -------------------- S steps per launch, one warp per strip, two FP32 nodes per thread
+// A warp owns a strip of up to WAVE_COLS<S> columns [x0, x0 + ncols) and a
+// chunk of rows [ya, ya + Hc), and walks up it one row per iteration: level 1
+// computes step n at row y, level 2 step n+1 at row y - 1, ..., level S step
+// n+S-1 at row y - S + 1, which it stores.  No other warp takes part, so
+// there is no block barrier.  Lane l holds a pair of columns at every level,
+// (p, p + 1) with p = x0 - (S - s) + 2l at level s: a level's pair starts one
+// column right of the level's before it, so of the populations streaming
+// into it those with c_x = +1 come from the lane's own pair of the level
+// before, those with c_x = -1 from lane l + 1's pair, and those with c_x = 0
+// one from each.  In y, populations with c_y = -1 come from the row the level
+// before has just computed (registers, shuffles), c_y = 0 from the row before
+// it and c_y = +1 from the one before that: those wait in the warp's shared
+// memory (1 and 2 rows deep).  Level s has 32 - s lanes, so a strip is
+// 2 (32 - S) columns, and recomputes S - s rows beyond each end of its chunk.
+// Level 1's inputs come through D stages of shared memory filled by 16-byte
+// asynchronous copies: a row's 64 columns from x0 - S (a multiple of 4, so x0
+// is 2 mod 4 for S = 2 and 0 mod 4 for S = 4) of one population of f (lanes
+// 0-15) and of g (lanes 16-31), each from the row it streams out of, per
+// instruction.  Strips wrap around in x, pair by pair.
+// Wall rows bounce back from the node's own populations: at row 0 the slot
+// of row -1 takes the level's f4, f7, f8 instead (read at the node's own
+// columns); at the top the c_y = +1 populations of the row itself are there.
+// Level 1 takes the domain's first and last row, and the ghost rows of a
+// y-slab (S = 2), by pull_node / pull_ghost_row instead of a stage.
+template <int S>
+constexpr int WAVE_COLS = 2 * (32 - S);
+template <int S>
+constexpr int WAVE_X0 = S % 4;  // first strip's x0
+
+// shared memory of one warp: D stages of 19 planes; per level but the last,
+// c_y = 0 populations and F of a row, c_y = +1 populations of 2 rows
+constexpr int WAVE_SLOTS = 7 + 2 * 6, WAVE_STAGE = 2 * NPOP + 1;
+template <int S, int D>
+constexpr size_t wave_smem_floats() {
+  return (size_t)((S - 1) * WAVE_SLOTS + D * WAVE_STAGE) * 64;
+}
+
+__device__ __forceinline__ void stcs2(char* p, unsigned o, float2 a) { __stcs(reinterpret_cast<float2*>(p + o), a); }
+__device__ __forceinline__ void cp16(unsigned dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// a level's moments at its strip's aligned pairs (ODD: the lane's second
+// column with its right neighbour's first)
+template <bool ODD>
+__device__ __forceinline__ void wave_put(float* p, float2 a, bool ok) {
+  const float2 b = ODD ? make_float2(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)) : a;
+  if (ok) *reinterpret_cast<float2*>(p) = b;
+}
+
+template <int S, int D, bool NUD, typename GetV>
+__device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int ya, int Hc, float* sm) {
+  static_assert(S == 2 || S == 4, "x0 - S a multiple of 4 and aligned pairs");
+  const LBView<float>& V1 = view(std::integral_constant<int, 0>{});
+  const int nx = V1.nx, ny = V1.ny;
+  const unsigned pitch = (unsigned)V1.pitch;
+  const size_t plane = V1.plane;
+  const bool glo = S == 2 && V1.gh2_lo != nullptr, ghi = S == 2 && V1.gh2_hi != nullptr;
+  const int ylo = glo ? -1 : 0, yhi = ghi ? ny : ny - 1;
+  const int lane = threadIdx.x & 31;
+  const int l1 = min(lane + 1, 31);
+  float* const lag = sm + D * WAVE_STAGE * 64;
+  const unsigned sm_addr = (unsigned)__cvta_generic_to_shared(sm);
+
+  // this lane's 4 columns of a staged row
+  const int cq = 4 * (lane & 15);
+  const bool cp_ok = cq < ncols + 2 * S;
+  const unsigned cp_col = (unsigned)((x0 - S + cq + 16 * nx) % nx);
+  const float* const cp_base = (lane < 16 ? V1.fsrc : V1.gsrc) + cp_col;
+  const unsigned cp_dst = sm_addr + (lane < 16 ? 0 : NPOP * 256) + cq * 4;
+  auto issue = [&](int y, int stage) {
+    if (y > 0 && y < ny - 1 && cp_ok) {
+      const float* p = cp_base + (size_t)((unsigned)y * pitch);
+      const unsigned d = cp_dst + stage * (WAVE_STAGE * 256);
+      static_for<NPOP>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        cp16(d + k * 256, p + ((ptrdiff_t)(k * plane) - (ptrdiff_t)icy(k) * (ptrdiff_t)pitch));
+      });
+      if (lane < 16) cp16(d + 2 * NPOP * 256, V1.Fin + ((unsigned)y * pitch + cp_col));
+    }
+    cp_commit();
+  };
+
+  const int nit = Hc + 2 * (S - 1);
+  int y = ya - (S - 1);
+  // a nudged run's sums of step n at the lane's level-1 pair: the mask bits of
+  // a row are loaded two iterations ahead, its sums (where a bit is set) one
+  const int nxa = (x0 - (S - 1) + 2 * lane + 16 * nx) % nx, nxb = nxa + 1 == nx ? 0 : nxa + 1;
+  auto mask_bits = [&](int yy) -> unsigned {
+    if (yy < 0 || yy >= ny) return 0;
+    const unsigned* m = V1.nmask + (size_t)yy * (pitch >> 5);
+    return ((m[nxa >> 5] >> (nxa & 31)) & 1u) | (((m[nxb >> 5] >> (nxb & 31)) & 1u) << 1);
+  };
+  auto sum_at = [&](int yy, int x, bool on) -> long long {
+    return on ? (long long)V1.nacc[(size_t)yy * pitch + x] : 0;
+  };
+  long long na = 0, nb = 0;
+  unsigned bits = 0;
+  if constexpr (NUD) {
+    bits = mask_bits(y);
+    na = sum_at(y, nxa, bits & 1u), nb = sum_at(y, nxb, bits & 2u);
+    bits = mask_bits(y + 1);
+  }
+#pragma unroll
+  for (int d = 0; d < D; d++) issue(d < nit ? y + d : -1, d);
+  int stage = 0;
+  int p0 = 0, p1 = 6 * 64;  // c_y = +1 slot of this iteration's row (and of the row two before it), and of the row before
+  for (int it = 0; it < nit; it++, y++) {
+    float2 f[NPOP], g[NPOP], F, r, u, v, t;
+    const bool on1 = y >= ylo && y <= yhi;
+    cp_wait<D - 1>();
+    __syncwarp();
+    const float* st = sm + stage * WAVE_STAGE * 64;
+    auto own = [&](const float* s, int i) { return reinterpret_cast<const float2*>(s + i * 64)[lane]; };
+    auto nxt = [&](const float* s, int i) { return reinterpret_cast<const float2*>(s + i * 64)[l1]; };
+    auto mid = [&](const float* s, int i) { return make_float2(s[i * 64 + 2 * lane + 1], s[i * 64 + 2 * l1]); };
+    if (y > 0 && y < ny - 1) {
+      static_for<NPOP>([&](auto kc) {
+        constexpr int k = decltype(kc)::value;
+        f[k] = icx(k) == 1 ? own(st, k) : (icx(k) == -1 ? nxt(st, k) : mid(st, k));
+        g[k] = icx(k) == 1 ? own(st, NPOP + k) : (icx(k) == -1 ? nxt(st, NPOP + k) : mid(st, NPOP + k));
+      });
+      F = mid(st, 2 * NPOP);
+    } else if (on1) {
+      float a[2 * NPOP], b[2 * NPOP];
+      auto one = [&](int x, float* p, float& Fx) {
+        x = (x + 16 * nx) % nx;
+        if (S == 2 && (y < 0 || y >= ny)) {
+          pull_ghost_row<float, size_t>(V1, y < 0, x, p, p + NPOP, Fx);
+        } else {
+          pull_node<float, LBRB_TWALL_DIRICHLET, size_t, false>(V1, y, x, p, p + NPOP);
+          dirichlet_walls(V1, y, p + NPOP);
+          Fx = V1.Fin[(unsigned)y * pitch + x];
+        }
+      };
+      one(x0 - (S - 1) + 2 * lane, a, F.x);
+      one(x0 - (S - 1) + 2 * lane + 1, b, F.y);
+#pragma unroll
+      for (int k = 0; k < NPOP; k++) {
+        f[k] = make_float2(a[k], b[k]);
+        g[k] = make_float2(a[NPOP + k], b[NPOP + k]);
+      }
+    }
+    __syncwarp();
+    issue(it + D < nit ? y + D : -1, stage);
+    stage = stage + 1 == D ? 0 : stage + 1;
+    if (on1) {
+      node_shift2(V1, f, g, F, r, u, v, t);
+      if constexpr (NUD) {
+        if (na != 0) {
+          const double sv = (double)na * (1.0 / FIX_SCALE);
+#pragma unroll
+          for (int k = 0; k < NPOP; k++) g[k].x = g[k].x + nudge_increment<float>(k, sv);
+        }
+        if (nb != 0) {
+          const double sv = (double)nb * (1.0 / FIX_SCALE);
+#pragma unroll
+          for (int k = 0; k < NPOP; k++) g[k].y = g[k].y + nudge_increment<float>(k, sv);
+        }
+      }
+    }
+    if constexpr (NUD) {
+      na = sum_at(y + 1, nxa, bits & 1u), nb = sum_at(y + 1, nxb, bits & 2u);
+      bits = mask_bits(y + 2);
+    }
+    static_for<S>([&](auto sc) {
+      constexpr int s = decltype(sc)::value + 1;  // level, whose row yr is now in f, g, F and r, u, v, t
+      constexpr int off = S - s;
+      const LBView<float>& V = view(std::integral_constant<int, s - 1>{});
+      const int yr = y - (s - 1);
+      const bool on = s == 1 ? on1 : (yr >= max(ya - off, 0) && yr <= min(ya + Hc - 1 + off, ny - 1));
+      // the level's moments (and the last level's state) in its strip and chunk
+      if (on && yr >= ya && yr < ya + Hc) {
+        const int c = 2 * lane - off + (off & 1);  // column in the strip of the aligned pair
+        const bool ok = c >= 0 && c < ncols;
+        const int xc = x0 + c;
+        const unsigned o = (unsigned)yr * pitch + (unsigned)(xc >= nx ? xc - nx : xc);
+        const unsigned ob = o * 4u;  // (bytes within a plane)
+        constexpr bool ODD = (off & 1) != 0;
+        if constexpr (s == S) {
+          if (ok) {
+#pragma unroll
+            for (int k = 0; k < NPOP; k++) {
+              stcs2(reinterpret_cast<char*>(V.fdst) + k * plane * 4, ob, f[k]);
+              stcs2(reinterpret_cast<char*>(V.gdst) + k * plane * 4, ob, g[k]);
+            }
+          }
+        }
+        if (s == S || V.write_F) wave_put<ODD>(V.Fout + o, F, ok);
+        if (V.write_uv) {
+          wave_put<ODD>(V.u + o, u, ok);
+          wave_put<ODD>(V.v + o, v, ok);
+        }
+        if (V.write_rt & 1) wave_put<ODD>(V.T + o, t, ok);
+        if (V.write_rt & 2) wave_put<ODD>(V.rho + o, r, ok);
+      }
+      if constexpr (s < S) {
+        // the next level's inputs at row yn; this level's row takes their place
+        const int yn = yr - 1;
+        const bool lo = yn == 0 && !glo, hi = yn == ny - 1 && !ghi;
+        float* w0 = lag + (s - 1) * WAVE_SLOTS * 64;
+        float* w1 = w0 + 7 * 64 + p0;
+        float* wp = w0 + 7 * 64 + p1;
+        const float2 a0 = mid(w0, 0), a1 = own(w0, 1), a3 = nxt(w0, 2);
+        const float2 b0 = mid(w0, 3), b1 = own(w0, 4), b3 = nxt(w0, 5);
+        const float2 Fn = mid(w0, 6);
+        float2 a2 = mid(w1, 0), a5 = own(w1, 1), a6 = nxt(w1, 2);
+        if (lo) a5 = mid(w1, 1), a6 = mid(w1, 2);
+        float2 b2 = mid(w1, 3), b5 = own(w1, 4), b6 = nxt(w1, 5);
+        __syncwarp();
+        if (on) {
+          auto put = [&](float* slot, int i, float2 a) { reinterpret_cast<float2*>(slot + i * 64)[lane] = a; };
+          put(w0, 0, f[0]), put(w0, 1, f[1]), put(w0, 2, f[3]);
+          put(w0, 3, g[0]), put(w0, 4, g[1]), put(w0, 5, g[3]);
+          put(w0, 6, F);
+          put(w1, 0, f[2]), put(w1, 1, f[5]), put(w1, 2, f[6]);
+          put(w1, 3, g[2]), put(w1, 4, g[5]), put(w1, 5, g[6]);
+          if (yr == 0 && !glo) put(wp, 0, f[4]), put(wp, 1, f[7]), put(wp, 2, f[8]);
+        }
+        auto shm = [&](float2 a) { return make_float2(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)); };
+        auto shn = [&](float2 a) {
+          return make_float2(__shfl_down_sync(0xffffffffu, a.x, 1), __shfl_down_sync(0xffffffffu, a.y, 1));
+        };
+        f[4] = shm(f[4]), f[7] = shn(f[7]);  // (f[8]: the lane's own)
+        g[4] = shm(g[4]), g[7] = shn(g[7]);
+        f[0] = a0, f[1] = a1, f[3] = a3, f[2] = a2, f[5] = a5, f[6] = a6;
+        g[0] = b0, g[1] = b1, g[3] = b3, g[2] = b2, g[5] = b5, g[6] = b6;
+        F = Fn;
+        const LBView<float>& VN = view(std::integral_constant<int, s>{});
+        if (lo || hi) {
+          if (lo) {
+            g[2] = g[5] = g[6] = make_float2(0.f, 0.f);
+          } else {
+            f[4] = mid(wp, 0), f[7] = mid(wp, 1), f[8] = mid(wp, 2);
+            g[4] = g[7] = g[8] = make_float2(0.f, 0.f);
+          }
+          float ga[NPOP], gb[NPOP];
+#pragma unroll
+          for (int k = 0; k < NPOP; k++) ga[k] = g[k].x, gb[k] = g[k].y;
+          dirichlet_walls(VN, yn, ga);
+          dirichlet_walls(VN, yn, gb);
+#pragma unroll
+          for (int k = 0; k < NPOP; k++) g[k] = make_float2(ga[k], gb[k]);
+        }
+        __syncwarp();
+        if (yn >= max(ya - off + 1, 0) && yn <= min(ya + Hc - 2 + off, ny - 1)) node_shift2(VN, f, g, F, r, u, v, t);
+      }
+    });
+    const int pt = p0;
+    p0 = p1;
+    p1 = pt;
+  }
+  cp_wait<0>();
+}
+
 }  // namespace lbrb
