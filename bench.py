@@ -441,7 +441,7 @@ def run_ours(args, torch, dist, rank: int, world: int, device: int) -> dict | No
     mlups64 = whole_job_mlups(world, nodes, K64, ms64)
     peak, peak_kind = measured_peak()
     # the fused launches of the instrumented window: node-steps per launch
-    # (2 for a two-step launch; the call's last step is a single one)
+    # (4 and 2 for four- and two-step launches)
     avg_lb = lb_ms / max(lb_n, 1)
     spl = K / max(lb_n, 1)
     achieved = ALG_BYTES["fp32"] * nodes * spl / (avg_lb * 1e-3) / 1e9
@@ -449,8 +449,10 @@ def run_ours(args, torch, dist, rank: int, world: int, device: int) -> dict | No
     spl64 = K64 / max(timing64["lb_step"][1], 1)
     avg_lb64 = timing64["lb_step"][0] / max(timing64["lb_step"][1], 1)
     achieved64 = ALG_BYTES["fp64"] * nodes * spl64 / (avg_lb64 * 1e-3) / 1e9
-    if pair32["shape"] >= 0 and spl > 1.5:
-        kernel32 = "lb_march_kernel<float>" if pair32["shape"] >= 9 else "lb_pair_kernel<float>"
+    if spl > 2.5:
+        kernel32 = "lb_wave4_kernel"
+    elif pair32["shape"] >= 0 and spl > 1.5:
+        kernel32 = "lb_wave2_kernel" if pair32["shape"] >= 9 else "lb_pair_kernel<float>"
     else:
         kernel32 = "lb_node_kernel<float>"
     tr = profiled_traffic("fp32" if spl > 1.5 else "fp32_single", kernel32)
@@ -487,8 +489,8 @@ def run_ours(args, torch, dist, rank: int, world: int, device: int) -> dict | No
                      "traffic_gbs": (round(tr * nodes / (avg_lb * 1e-3) / 1e9, 1) if tr else None),
                      "share_of_step": round(lb_ms / timing["window_ms"][0], 4),
                      "launch_shape": shape32, "pair_shape": pair32,
-                     "note": "achieved = 144 B x node-steps per launch / launch time (a two-step launch moves "
-                             "the populations through HBM once for two steps); per-kernel times from an "
+                     "note": "achieved = 144 B x node-steps per launch / launch time (a four-step launch moves "
+                             "the populations through HBM once for four steps); per-kernel times from an "
                              "instrumented second window of the same K steps"},
         "fp64": {"value": round(mlups64, 1), "unit": "MLUPS", "steps": K64,
                  "lb_achieved_gbs": round(achieved64, 1),

@@ -191,7 +191,12 @@ LBRB_API int lbrb_set_graph(lbrb_t *h, int mode);
  * The launch shape is timed on first use (once per process for handles
  * of the same kind, as for autotune); lbrb_get_pair_shape reports it
  * (shape index, tile columns and rows, ms per launch; shape -1 before).
- * Replaces, for two steps at a time, the reference's per-step sweeps
+ * FP32 runs without nudging also take four steps per launch where that is
+ * timed faster than two two-step launches and the shape was not fixed by
+ * lbrb_set_pair_shape: the same steps, again with identical results, while
+ * more than four steps of the call remain and at most one of the four is a
+ * record step.
+ * Replaces, for two or four steps at a time, the reference's per-step sweeps
  * (stream, moments, collide: temppart_dump.c:1674-1759). */
 LBRB_API int lbrb_set_pairs(lbrb_t *h, int mode);
 /* fix the launch shape of the two-step kernel instead of timing the shapes

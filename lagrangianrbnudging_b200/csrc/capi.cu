@@ -54,7 +54,7 @@ struct TuneVal {
   float ms;
 };
 static std::mutex g_tune_mu;
-static std::map<TuneKey, TuneVal> g_tuned_single, g_tuned_pair;
+static std::map<TuneKey, TuneVal> g_tuned_single, g_tuned_pair, g_tuned_quad;
 // the steps store u, v every step (and T on record steps) for particles:
 // the whole domain's, or a slab's own (lbrb_slab_particles_set)
 static bool moves_particles(const lbrb_t* h) { return h->np > 0 || (h->sp && h->sp->cap > 0); }
@@ -250,6 +250,7 @@ static void free_all(lbrb_t* h) {
   F(h->pops[0]); F(h->pops[1]); F(h->F[0]); F(h->F[1]);
   F(h->rho[0]); F(h->rho[1]); F(h->T[0]); F(h->T[1]);
   for (int a = 0; a < 3; a++) for (int b = 0; b < 2; b++) F(h->uv[a][b]);
+  F(h->uv_extra);
   F(h->px); F(h->pid); F(h->ptype); F(h->d_ring);
   if (h->h_ring) cudaFreeHost(h->h_ring);
   delete[] h->h_ring_step;
@@ -351,6 +352,22 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
       for (int s = 0; s < h->p.record_slots; s++)
         if (cudaEventCreateWithFlags(&h->ring_ev[s], cudaEventDisableTiming) != cudaSuccess)
           return done(LBRB_ERR_CUDA);
+    }
+  }
+  // the two extra u, v slots of four-step launches with particles, unless an
+  // earlier handle of this kind timed pairs as faster (lbrb_step); a run
+  // without memory for them steps in pairs
+  if (h->np > 0 && fp32(h) && p.twall == LBRB_TWALL_DIRICHLET && p.nudge == LBRB_NUDGE_NONE) {
+    int sh = 0;
+    float ms = 0.f;
+    const size_t pb1 = h->plane * h->esize;
+    if (!tuned_get(g_tuned_quad, h, &sh, &ms) || sh >= 0) {
+      if (cudaMalloc(&h->uv_extra, 4 * pb1) != cudaSuccess) {
+        cudaGetLastError();
+        h->uv_extra = nullptr;
+      } else {
+        for (int q = 0; q < 4; q++) h->uv[3 + q / 2][q % 2] = (char*)h->uv_extra + q * pb1;
+      }
     }
   }
   h->nobs = p.nobs;
@@ -1102,6 +1119,78 @@ int lbrb_step(lbrb_t* h, int n) {
     }
     return LBRB_OK;
   };
+  // Four plain steps n .. n+3 in one launch (lb_wave4_kernel), then the
+  // particles of all four.  As `two`: u, v of n+2 and n+3 go to the slots two
+  // pairs would leave them in, those of n and n+1 to the extra slots; at most
+  // one of the steps is a record step, whose T goes to the source buffer, or
+  // for step n+3 to the destination's.  Never the call's last step.
+  auto quad_views = [&](const bool* rec, LBView<float> (&V)[4]) {
+    const int src = h->cur, dst = h->cur ^ 1;
+    const bool parts = h->np > 0;
+    const int slot[4] = {3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
+    for (int q = 0; q < 4; q++) {
+      V[q] = make_view<float>(h, src, dst, parts ? slot[q] : h->uvcur, parts ? 1 : 0, rec[q] ? 1 : 0);
+      if (q < 3) V[q].T = (float*)h->T[src];
+    }
+  };
+  auto four = [&]() -> int {
+    const bool parts = h->np > 0;
+    bool rec[4];
+    for (int q = 0; q < 4; q++) rec[q] = parts && h->p.noutconfig > 0 && (h->istep + 1 + q) % h->p.noutconfig == 0;
+    LBView<float> V[4];
+    quad_views(rec, V);
+    const int tm = tmark_begin(h, 0, h->stream);
+    CK(h, launch_quad_fp32(V, h->quad_shape, h->stream, pdl_ok));
+    tmark_end(h, tm, h->stream);
+    if (parts) {
+      const int slot[5] = {h->uvcur, 3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
+      const void* fields[4][5];
+      double* r[4] = {};
+      const int rslot = (int)(h->rec_head % h->p.record_slots);
+      for (int q = 0; q < 4; q++) {
+        for (int c = 0; c < 2; c++) fields[q][c] = h->uv[slot[q + 1]][c], fields[q][2 + c] = h->uv[slot[q]][c];
+        fields[q][4] = V[q].T;
+        if (rec[q]) r[q] = h->d_ring + (size_t)rslot * h->nrec_fields * h->np;
+      }
+      const int tp = tmark_begin(h, 1, h->stream);
+      CK(h, launch_particles_quad(fields, true, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full,
+                                  r, h->dflags, h->stream, pdl_ok));
+      tmark_end(h, tp, h->stream);
+      for (int q = 0; q < 4; q++)
+        if (rec[q]) {
+          const int rc = record_copy(h->istep + 1 + q, rslot, r[q], h->stream);
+          if (rc) return rc;
+        }
+      h->uvprev = slot[3];
+      h->uvcur = slot[4];
+    }
+    h->cur ^= 1;
+    h->prev_valid = false;
+    h->prev_pair = false;
+    h->istep += 4;
+    return LBRB_OK;
+  };
+  // four steps per launch where a timed launch beats two timed pair launches
+  auto quads_ok = [&]() {
+    return f32 && step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed;
+  };
+  auto tune_quads = [&]() -> int {
+    h->quad_shape = -1;
+    if (h->np > 0 && !h->uv_extra) return LBRB_OK;  // (no memory for the slots: pairs)
+    float ms = 0.f;
+    int sh = 0;
+    if (!tuned_get(g_tuned_quad, h, &sh, &ms)) {
+      const bool none[4] = {};
+      LBView<float> V[4];
+      quad_views(none, V);
+      sh = tune_quad_fp32(V, h->stream, &ms);
+      CK(h, cudaGetLastError());
+      if (ms >= 2.f * h->pair_ms) sh = -1;
+      tuned_put(g_tuned_quad, h, sh, ms);
+    }
+    h->quad_shape = sh;
+    return LBRB_OK;
+  };
   bool graphs_on = graph_ok(h);  // (refined below for a caller's capture)
   if (step_pairs_ok(h) && h->pair_shape < 0 && n >= 3) {
     // the pair shape is timed on the first call that can use pairs (trial
@@ -1110,6 +1199,14 @@ int lbrb_step(lbrb_t* h, int n) {
     CK(h, cudaStreamIsCapturing(h->stream, &cs));
     if (cs == cudaStreamCaptureStatusNone && !(graphs_on && n - 1 >= GRAPH_STEPS)) {
       const int rc = tune_pairs();
+      if (rc) return rc;
+    }
+  }
+  if (n >= 5 && h->quad_shape == -2 && quads_ok() && !graphs_on) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(h->stream, &cs));
+    if (cs == cudaStreamCaptureStatusNone) {
+      const int rc = tune_quads();
       if (rc) return rc;
     }
   }
@@ -1166,6 +1263,19 @@ int lbrb_step(lbrb_t* h, int n) {
         h->prev_pair = false;
         h->istep += GRAPH_STEPS;
         s += GRAPH_STEPS;
+        continue;
+      }
+    }
+    if (!graphs && n - s >= 5 && h->quad_shape >= 0 && quads_ok()) {
+      // (a group with two record steps, or whose record would not fit in the
+      // ring, goes in pairs or single steps, which report the overflow)
+      int need = 0;
+      for (int q = 1; q <= 4; q++)
+        need += h->np > 0 && h->p.noutconfig > 0 && (h->istep + q) % h->p.noutconfig == 0;
+      if (need <= 1 && h->rec_head - h->rec_tail + need <= h->p.record_slots) {
+        const int rc = four();
+        if (rc) return rc;
+        s += 4;
         continue;
       }
     }
@@ -2543,6 +2653,7 @@ int lbrb_set_pair_shape(lbrb_t* h, int shape) {
   if (!h || shape < -1 || shape >= NUM_PAIR_SHAPES)
     return fail(h, LBRB_ERR_ARG, "set_pair_shape: shape must be -1 (tune) or a shape index");
   h->pair_shape = shape;
+  h->pair_fixed = shape >= 0;
   h->pair_ms = 0.f;
   return LBRB_OK;
 }

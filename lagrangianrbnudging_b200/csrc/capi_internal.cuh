@@ -32,6 +32,9 @@ cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, i
 cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s, bool pdl);
 int tune_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, cudaStream_t s, float* best_ms);
 int tune_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, cudaStream_t s, float* best_ms);
+// four steps per launch (as pairs; FP32, no nudging, no y-slab): one view per step
+cudaError_t launch_quad_fp32(const LBView<float> (&V)[4], int shape, cudaStream_t s, bool pdl);
+int tune_quad_fp32(const LBView<float> (&V)[4], cudaStream_t s, float* best_ms);
 cudaError_t launch_particles(const void* u, const void* v, const void* ub, const void* vb,
                              const void* T, bool fp32, int nx, int ny, int pitch, double* P,
                              const int* ptype, int np, double beta, int record, int full,
@@ -42,6 +45,10 @@ cudaError_t launch_particles(const void* u, const void* v, const void* ub, const
 cudaError_t launch_particles_pair(const void* const* fields_a, const void* const* fields_b, bool fp32, int nx,
                                   int ny, int pitch, double* P, const int* ptype, int np, double beta, int full,
                                   double* rec_a, double* rec_b, unsigned* dflags, cudaStream_t s, bool pdl);
+// the same for four steps (after a four-step fused launch)
+cudaError_t launch_particles_quad(const void* const (*fields)[5], bool fp32, int nx, int ny, int pitch, double* P,
+                                  const int* ptype, int np, double beta, int full, double* const* rec,
+                                  unsigned* dflags, cudaStream_t s, bool pdl);
 // y-slabs: rows5 = device tables of row pointers (u, v, ub, vb, T), one
 // entry per global row
 // y-slabs holding their own particles (particle_kernels.cu): the moment

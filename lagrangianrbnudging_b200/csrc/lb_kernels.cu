@@ -101,6 +101,28 @@ __global__ void __launch_bounds__(32 * NW, MINB)
                         min(H, V1.ny - ya), wave_smem + w * wave_smem_floats<2, D>());
 }
 
+// four steps per launch: the populations and F cross HBM once per four steps
+template <int NW, int MINB, int D>
+__global__ void __launch_bounds__(32 * NW, MINB)
+    lb_wave4_kernel(const LBView<float> V1, const LBView<float> V2, const LBView<float> V3, const LBView<float> V4,
+                    int H, int nitems) {
+  pdl_wait();
+  extern __shared__ __align__(16) float wave_smem[];
+  const int w = threadIdx.x >> 5, item = blockIdx.x * NW + w;
+  if (item >= nitems) return;
+  const int nstrips = (V1.nx + WAVE_COLS<4> - 1) / WAVE_COLS<4>;
+  const int strip = item % nstrips, ya = item / nstrips * H;
+  wave_march<4, D, false>(
+      [&](auto s) -> const LBView<float>& {
+        if constexpr (decltype(s)::value == 0) return V1;
+        else if constexpr (decltype(s)::value == 1) return V2;
+        else if constexpr (decltype(s)::value == 2) return V3;
+        else return V4;
+      },
+      strip * WAVE_COLS<4> + WAVE_X0<4>, min(WAVE_COLS<4>, V1.nx - strip * WAVE_COLS<4>), ya, min(H, V1.ny - ya),
+      wave_smem + w * wave_smem_floats<4, D>());
+}
+
 // pair launch shapes: (tile columns, tile rows, threads, min blocks per SM)
 struct PairShape { int tx, ty, nt, minb; };
 constexpr PairShape PAIR_SHAPES[] = {{32, 8, 256, 4}, {32, 4, 128, 6}, {32, 16, 512, 2}, {64, 4, 256, 3},
@@ -196,6 +218,30 @@ static cudaError_t launch_wave2_t(const LBView<float>& V1, const LBView<float>& 
   const int H = (int)((ny + chunks - 1) / chunks);
   const long nitems = nstrips * ((ny + H - 1) / H);
   return launch_k(kernel, dim3((unsigned)((nitems + NW - 1) / NW)), 32 * NW, smem, s, pdl, V1, V2, H, (int)nitems);
+}
+
+// four-step launch shapes: waves of resident warps the chunk height aims at
+constexpr int QUAD_WAVES[NUM_QUAD_SHAPES] = {1, 2, 4};
+cudaError_t launch_quad_fp32(const LBView<float> (&V)[4], int shape, cudaStream_t s, bool pdl) {
+  constexpr int NW = 4, MINB = 3, D = 1;
+  constexpr auto kernel = lb_wave4_kernel<NW, MINB, D>;
+  constexpr size_t smem = NW * wave_smem_floats<4, D>() * sizeof(float);
+  static std::atomic<unsigned long long> attr_set{0};
+  static std::atomic<int> occ_cache[MAX_DEVICES] = {};
+  cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
+  if (e != cudaSuccess) return e;
+  int occ = 0, dev = 0, nsm = 0;
+  e = occupancy_once((const void*)kernel, 32 * NW, smem, occ_cache, &occ);
+  if (e == cudaSuccess) e = current_device(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int ny = V[0].ny;
+  const long nstrips = (V[0].nx + WAVE_COLS<4> - 1) / WAVE_COLS<4>;
+  const long chunks = std::min((long)ny, std::max(1L, (long)QUAD_WAVES[shape] * occ * nsm * NW / nstrips));
+  const int H = (int)((ny + chunks - 1) / chunks);
+  const long nitems = nstrips * ((ny + H - 1) / H);
+  return launch_k(kernel, dim3((unsigned)((nitems + NW - 1) / NW)), 32 * NW, smem, s, pdl, V[0], V[1], V[2], V[3], H,
+                  (int)nitems);
 }
 
 static cudaError_t launch_wave2(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
@@ -400,6 +446,36 @@ static int tune_pair(const LBView<Real>& A, const LBView<Real>& B, cudaStream_t 
   float bt = 1e30f;
   for (int sh = 0; sh < NUM_PAIR_SHAPES; sh++)
     if (shape_ms[sh] < bt) { bt = shape_ms[sh]; best = sh; }
+  cudaEventDestroy(a);
+  cudaEventDestroy(b);
+  if (best_ms) *best_ms = bt / reps;
+  return best;
+}
+// the four-step launch shapes, timed as tune_pair's (no T or rho stored)
+int tune_quad_fp32(const LBView<float> (&Vin)[4], cudaStream_t s, float* best_ms) {
+  LBView<float> V[4] = {Vin[0], Vin[1], Vin[2], Vin[3]};
+  for (auto& v : V) v.write_rt = 0;
+  cudaEvent_t a, b;
+  cudaEventCreate(&a);
+  cudaEventCreate(&b);
+  const int reps = std::max(3, tune_reps(V[0]) / 2);
+  int best = 0;
+  float bt = 1e30f;
+  for (int round = 0; round < 2; round++) {
+    for (int sh = 0; sh < NUM_QUAD_SHAPES; sh++) {
+      if (launch_quad_fp32(V, sh, s, false) != cudaSuccess) {
+        cudaGetLastError();
+        continue;
+      }
+      cudaEventRecord(a, s);
+      for (int r = 0; r < reps; r++) launch_quad_fp32(V, sh, s, false);
+      cudaEventRecord(b, s);
+      cudaEventSynchronize(b);
+      float ms = 1e30f;
+      cudaEventElapsedTime(&ms, a, b);
+      if (ms < bt) bt = ms, best = sh;
+    }
+  }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (best_ms) *best_ms = bt / reps;

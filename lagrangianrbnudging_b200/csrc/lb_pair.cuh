@@ -377,12 +377,16 @@ constexpr int WAVE_COLS = 2 * (32 - S);
 template <int S>
 constexpr int WAVE_X0 = S % 4;  // first strip's x0
 
-// shared memory of one warp: D stages of 19 planes; per level but the last,
-// c_y = 0 populations and F of a row, c_y = +1 populations of 2 rows
+// shared memory of one warp: D stages of 19 planes of 64 columns; per level s
+// but the last, c_y = 0 populations and F of a row and c_y = +1 populations
+// of 2 rows, 2 (32 - s) columns each; a few floats that lanes past a level's
+// last pair may read (12 warps of S = 4, D = 1 just fit an SM this way)
 constexpr int WAVE_SLOTS = 7 + 2 * 6, WAVE_STAGE = 2 * NPOP + 1;
+constexpr int wave_cols(int level) { return 2 * (32 - level); }
+constexpr int wave_lag(int level) { return level == 0 ? 0 : wave_lag(level - 1) + WAVE_SLOTS * wave_cols(level); }
 template <int S, int D>
 constexpr size_t wave_smem_floats() {
-  return (size_t)((S - 1) * WAVE_SLOTS + D * WAVE_STAGE) * 64;
+  return ((size_t)D * WAVE_STAGE * 64 + wave_lag(S - 1) + 8 + 3) / 4 * 4;
 }
 
 __device__ __forceinline__ void stcs2(char* p, unsigned o, float2 a) { __stcs(reinterpret_cast<float2*>(p + o), a); }
@@ -457,23 +461,24 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
 #pragma unroll
   for (int d = 0; d < D; d++) issue(d < nit ? y + d : -1, d);
   int stage = 0;
-  int p0 = 0, p1 = 6 * 64;  // c_y = +1 slot of this iteration's row (and of the row two before it), and of the row before
+  int p0 = 0, p1 = 6;  // c_y = +1 slots of this iteration's row (and of the row two before it), and of the row before
   for (int it = 0; it < nit; it++, y++) {
     float2 f[NPOP], g[NPOP], F, r, u, v, t;
     const bool on1 = y >= ylo && y <= yhi;
     cp_wait<D - 1>();
     __syncwarp();
     const float* st = sm + stage * WAVE_STAGE * 64;
-    auto own = [&](const float* s, int i) { return reinterpret_cast<const float2*>(s + i * 64)[lane]; };
-    auto nxt = [&](const float* s, int i) { return reinterpret_cast<const float2*>(s + i * 64)[l1]; };
-    auto mid = [&](const float* s, int i) { return make_float2(s[i * 64 + 2 * lane + 1], s[i * 64 + 2 * l1]); };
+    // a staged plane at the lane's pair, its right neighbour's, and one column right of its own
+    auto sown = [&](int i) { return reinterpret_cast<const float2*>(st + i * 64)[lane]; };
+    auto snxt = [&](int i) { return reinterpret_cast<const float2*>(st + i * 64)[l1]; };
+    auto smid = [&](int i) { return make_float2(st[i * 64 + 2 * lane + 1], st[i * 64 + 2 * l1]); };
     if (y > 0 && y < ny - 1) {
       static_for<NPOP>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        f[k] = icx(k) == 1 ? own(st, k) : (icx(k) == -1 ? nxt(st, k) : mid(st, k));
-        g[k] = icx(k) == 1 ? own(st, NPOP + k) : (icx(k) == -1 ? nxt(st, NPOP + k) : mid(st, NPOP + k));
+        f[k] = icx(k) == 1 ? sown(k) : (icx(k) == -1 ? snxt(k) : smid(k));
+        g[k] = icx(k) == 1 ? sown(NPOP + k) : (icx(k) == -1 ? snxt(NPOP + k) : smid(NPOP + k));
       });
-      F = mid(st, 2 * NPOP);
+      F = smid(2 * NPOP);
     } else if (on1) {
       float a[2 * NPOP], b[2 * NPOP];
       auto one = [&](int x, float* p, float& Fx) {
@@ -551,9 +556,13 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         // the next level's inputs at row yn; this level's row takes their place
         const int yn = yr - 1;
         const bool lo = yn == 0 && !glo, hi = yn == ny - 1 && !ghi;
-        float* w0 = lag + (s - 1) * WAVE_SLOTS * 64;
-        float* w1 = w0 + 7 * 64 + p0;
-        float* wp = w0 + 7 * 64 + p1;
+        constexpr int CW = wave_cols(s);
+        float* w0 = lag + wave_lag(s - 1);
+        float* w1 = w0 + (7 + p0) * CW;
+        float* wp = w0 + (7 + p1) * CW;
+        auto own = [&](const float* q, int i) { return reinterpret_cast<const float2*>(q + i * CW)[lane]; };
+        auto nxt = [&](const float* q, int i) { return reinterpret_cast<const float2*>(q + i * CW)[l1]; };
+        auto mid = [&](const float* q, int i) { return make_float2(q[i * CW + 2 * lane + 1], q[i * CW + 2 * l1]); };
         const float2 a0 = mid(w0, 0), a1 = own(w0, 1), a3 = nxt(w0, 2);
         const float2 b0 = mid(w0, 3), b1 = own(w0, 4), b3 = nxt(w0, 5);
         const float2 Fn = mid(w0, 6);
@@ -561,8 +570,8 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         if (lo) a5 = mid(w1, 1), a6 = mid(w1, 2);
         float2 b2 = mid(w1, 3), b5 = own(w1, 4), b6 = nxt(w1, 5);
         __syncwarp();
-        if (on) {
-          auto put = [&](float* slot, int i, float2 a) { reinterpret_cast<float2*>(slot + i * 64)[lane] = a; };
+        if (on && 2 * lane < CW) {
+          auto put = [&](float* q, int i, float2 a) { reinterpret_cast<float2*>(q + i * CW)[lane] = a; };
           put(w0, 0, f[0]), put(w0, 1, f[1]), put(w0, 2, f[3]);
           put(w0, 3, g[0]), put(w0, 4, g[1]), put(w0, 5, g[3]);
           put(w0, 6, F);

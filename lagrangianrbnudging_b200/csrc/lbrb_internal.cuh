@@ -59,6 +59,8 @@ inline bool off32_ok(size_t plane) { return plane * 2 * NPOP < (size_t(1) << 32)
 // (MARCH_SHAPES)
 constexpr int NUM_PAIR_TILES = 9;
 constexpr int NUM_PAIR_SHAPES = NUM_PAIR_TILES + 6;
+// launch shapes of the FP32 four-step kernel (QUAD_WAVES)
+constexpr int NUM_QUAD_SHAPES = 3;
 // planes (of nx values) of a y-slab's ghost block for two steps per launch
 // (aux_kernels.cu: slab_pack2_kernel)
 constexpr int SLAB_GH2_PLANES = 19;
@@ -305,6 +307,11 @@ struct Handle {
   int pair_mode = -1;
   int pair_shape = -1;
   float pair_ms = 0.f;
+  bool pair_fixed = false;  // lbrb_set_pair_shape chose the shape: two steps per launch, no four-step launches
+  // four steps per launch (lb_wave4_kernel): -2 not timed yet, -1 not used
+  // (two pair launches are faster, or no memory for the u, v slots), else
+  // the launch shape
+  int quad_shape = -2;
   int pair_save[3] = {0, 0, 0};  // y-slab pairs: cur, uvcur, uvprev before the launch
   int graph_mode = -1;
   size_t esize = 8;   // bytes per population value
@@ -325,7 +332,9 @@ struct Handle {
   // particle kernel of step n can run beside the fused kernel of step n+1
   void* rho[2] = {nullptr, nullptr};
   void* T[2] = {nullptr, nullptr};
-  void* uv[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
+  // (slots 3 and 4, in uv_extra: u^n, u^{n+1} inside a four-step launch with particles)
+  void* uv[5][2] = {};
+  void* uv_extra = nullptr;
   int uvcur = 0, uvprev = 1;
   // second stream: the adjoint window's segment recompute (events order it
   // against `stream`)

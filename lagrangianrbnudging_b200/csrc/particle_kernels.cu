@@ -50,6 +50,20 @@ __global__ void __launch_bounds__(128) particle_pair_kernel(const PView<Real> Va
   particle_update<Real, DERIVS>(Vb, p);
 }
 
+// four steps likewise, after a four-step fused launch
+template <typename Real>
+struct PView4 {
+  PView<Real> V[4];
+};
+template <typename Real, bool DERIVS>
+__global__ void __launch_bounds__(128) particle_quad_kernel(const __grid_constant__ PView4<Real> A) {
+  pdl_wait();
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= A.V[0].np) return;
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) particle_update<Real, DERIVS>(A.V[q], p);
+}
+
 // ------------------------------------------------------------- y-slabs
 // A domain held as y-slabs, one handle each (one process per GPU, or several
 // in one process): each slab holds the particles whose cell lies in its rows,
@@ -350,6 +364,25 @@ cudaError_t launch_particles_pair(const void* const* fields_a, const void* const
     const int g = (np + 127) / 128;
     if (beta != 0.0 || full) return launch_k(particle_pair_kernel<Real, true>, g, 128, 0, s, pdl, Va, Vb);
     return launch_k(particle_pair_kernel<Real, false>, g, 128, 0, s, pdl, Va, Vb);
+  };
+  return fp32 ? go(0.f) : go(0.0);
+}
+
+cudaError_t launch_particles_quad(const void* const (*fields)[5], bool fp32, int nx, int ny, int pitch, double* P,
+                                  const int* ptype, int np, double beta, int full, double* const* rec,
+                                  unsigned* dflags, cudaStream_t s, bool pdl) {
+  if (np <= 0) return cudaSuccess;
+  auto go = [&](auto zero) -> cudaError_t {
+    using Real = decltype(zero);
+    PView4<Real> A;
+    for (int q = 0; q < 4; q++) {
+      const void* const* f = fields[q];
+      A.V[q] = PView<Real>{(const Real*)f[0], (const Real*)f[1], (const Real*)f[2], (const Real*)f[3],
+                           (const Real*)f[4], nx, ny, pitch, P, ptype, np, beta, rec[q] ? 1 : 0, full, rec[q], dflags};
+    }
+    const int g = (np + 127) / 128;
+    if (beta != 0.0 || full) return launch_k(particle_quad_kernel<Real, true>, g, 128, 0, s, pdl, A);
+    return launch_k(particle_quad_kernel<Real, false>, g, 128, 0, s, pdl, A);
   };
   return fp32 ? go(0.f) : go(0.0);
 }

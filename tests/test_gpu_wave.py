@@ -62,3 +62,28 @@ def test_strip_edges(nx, ny, shape):
 def test_strip_edges_with_particles_and_nudging(nx, ny):
     with make(nx, ny, 0, -1, 30, 40) as a, make(nx, ny, 1, 12, 30, 40) as b:
         same(a, b, (2, 3, 12))
+
+
+@pytest.mark.parametrize("nx,ny", [(4, 5), (56, 3), (60, 8), (64, 33), (232, 700), (512, 256)])
+@pytest.mark.parametrize("nprtcl,every", [(0, 0), (30, 2), (30, 5)])
+def test_four_steps_per_launch(nx, ny, nprtcl, every):
+    """automatic launches (four, two and one steps, whichever the tuner
+    keeps) against single steps: calls around multiples of four, records on
+    every step of a group (every = 2: two in a group, so pairs)"""
+    def run(pairs):
+        kw = dict(lb.closure(nx, ny, Ra=1e5, Pr=1.0, U=0.05), precision="fp32", nprtcl=nprtcl, noutconfig=every,
+                  record_slots=64, beta=0.5, record_full=1)
+        r = lb.Run(**kw)
+        r.set_graph(0)
+        r.set_pairs(pairs)
+        r.init_conduction(7, 5e-2)
+        if nprtcl:
+            rng = np.random.default_rng(7)
+            ptype = (np.arange(nprtcl) % 2).astype(np.int32)
+            z = np.zeros(nprtcl)
+            r.set_particles(np.arange(nprtcl, dtype=np.int32), rng.uniform(0.5, nx, nprtcl),
+                            rng.uniform(1.0, ny, nprtcl), z, z, ptype, np.where(ptype == 1, 0.05, 0.0))
+        return r
+
+    with run(0) as a, run(1) as b:
+        same(a, b, (5, 6, 7, 8, 9, 23))
