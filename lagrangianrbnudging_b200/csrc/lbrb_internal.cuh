@@ -26,8 +26,7 @@ namespace lbrb {
 constexpr int NPOP = 9;
 constexpr int WARP = 32;
 
-// D2Q9 as the reference's dellar() builds it (temppart_dump.c:1363-1401);
-// cy[3] = -cy[1] and cx[4] = -cx[2] are negative zeros there.
+// D2Q9 as the reference's dellar() builds it (temppart_dump.c:1363-1401)
 __host__ __device__ constexpr double w_of(int k) {
   return k == 0 ? 16. / 36. : (k < 5 ? 4. / 36. : 1. / 36.);
 }
@@ -36,12 +35,6 @@ __host__ __device__ constexpr int icx(int k) {
 }
 __host__ __device__ constexpr int icy(int k) {
   return (k == 2 || k == 5 || k == 6) ? 1 : ((k == 4 || k == 7 || k == 8) ? -1 : 0);
-}
-__host__ __device__ constexpr double dcx(int k) {
-  return k == 4 ? -0.0 : (double)icx(k);
-}
-__host__ __device__ constexpr double dcy(int k) {
-  return k == 3 ? -0.0 : (double)icy(k);
 }
 __host__ __device__ constexpr int opp(int k) {
   return k == 0 ? 0 : (k <= 4 ? ((k + 1) % 4) + 1 : ((k - 5 + 2) % 4) + 5);
@@ -179,6 +172,39 @@ __device__ __forceinline__ void equil_ref(double r1, double u, double v, double 
   feq[6] = r1 * w_of(6) * (1. + sumsq2 - ui + vi - uv);
   feq[7] = r1 * w_of(7) * (1. + sumsq2 - ui - vi + uv);
   feq[8] = r1 * w_of(8) * (1. + sumsq2 + ui - vi - uv);
+}
+
+// div_const where only the value of a zero quotient matters, not its sign:
+// the correction step alone gives RN(x / c) for every x != 0 (r = 0 adds
+// nothing) and a zero for x = +-0.  Every quotient of the collision is used
+// this way: it is multiplied, squared, or added to a sum that is not a zero.
+__device__ __forceinline__ double div_sum(double x, double c, double rc) {
+  const double q0 = __dmul_rn(x, rc);
+  return __fma_rn(__fma_rn(-q0, c, x), rc, q0);
+}
+
+// The velocity part of equilif / equilig in the reference's operation order
+// (temppart_dump.c:1097-1180): f_k^eq = (rho w_k) b[k], g_k^eq = (T w_k) b[k],
+// the brackets b[] of f and g being the same expressions of u and v.
+__device__ __forceinline__ void equil_brackets(double u, double v, double b[NPOP]) {
+  const double usq = u * u;
+  const double vsq = v * v;
+  const double sumsq = div_sum(usq + vsq, DIV_2CS2, RCP_2CS2);
+  const double sumsq2 = div_sum(sumsq * (1. - CS2), CS2, RCP_CS2);
+  const double u2 = div_sum(usq, DIV_2_9, RCP_2_9);
+  const double v2 = div_sum(vsq, DIV_2_9, RCP_2_9);
+  const double ui = div_sum(u, CS2, RCP_CS2);
+  const double vi = div_sum(v, CS2, RCP_CS2);
+  const double uv = ui * vi;
+  b[0] = 1. - sumsq;
+  b[1] = 1. - sumsq + u2 + ui;
+  b[2] = 1. - sumsq + v2 + vi;
+  b[3] = 1. - sumsq + u2 - ui;
+  b[4] = 1. - sumsq + v2 - vi;
+  b[5] = 1. + sumsq2 + ui + vi + uv;
+  b[6] = 1. + sumsq2 - ui + vi - uv;
+  b[7] = 1. + sumsq2 - ui - vi + uv;
+  b[8] = 1. + sumsq2 + ui - vi - uv;
 }
 
 
