@@ -191,7 +191,7 @@ LBRB_API int lbrb_set_graph(lbrb_t *h, int mode);
  * The launch shape is timed on first use (once per process for handles
  * of the same kind, as for autotune); lbrb_get_pair_shape reports it
  * (shape index, tile columns and rows, ms per launch; shape -1 before).
- * FP32 runs without nudging also take four steps per launch where that is
+ * Runs without nudging also take four steps per launch where that is
  * timed faster than two two-step launches and the shape was not fixed by
  * lbrb_set_pair_shape: the same steps, again with identical results, while
  * more than four steps of the call remain and at most one of the four is a
@@ -203,15 +203,10 @@ LBRB_API int lbrb_set_pairs(lbrb_t *h, int mode);
  * on first use (-1).  Tiles with a one-node ring recomputed around each:
  * 0: 32x8, 1: 32x4, 2: 32x16, 3: 64x4, 4: 32x8 with a thread per node of
  * the tile and its ring, 5: 30x8 likewise, 6: 32x8 at 5 blocks per SM,
- * 7: 32x6, 8: 64x8.  9-14, marching.  FP64: strips of 32 columns walked
- * down a chunk of rows, recomputing only two halo columns and two rows per
- * chunk (tile_y: rows per group): 9: 8 rows, 3 blocks per SM; 10: 8 rows,
- * 3 blocks, the next group's loads issued before this group's second step
- * (software pipelining); 11: likewise, 2 blocks; 12: 6 rows, 4 blocks,
- * pipelined; 13: 4 rows, 6 blocks, pipelined; 14: 6 rows, 3 blocks,
- * pipelined.  FP32: strips of 60 columns, one warp each, two nodes per
- * thread, walked row by row up a chunk (tile_y: 1): 9-12: 8 warps per SM,
- * chunks for 1, 2, 3, 6 waves of warps; 13, 14: 12 warps per SM, 4 and 9
+ * 7: 32x6, 8: 64x8.  9-14, marching: strips of 60 columns, one warp each,
+ * two nodes per thread, walked row by row up a chunk of rows (tile_y: 1).
+ * FP32: 9-12: 8 warps per SM, chunks for 1, 2, 3, 6 waves of warps; 13, 14:
+ * 12 warps per SM, 4 and 9 waves.  FP64: 8 warps per SM, 1, 2, 3, 4, 6 and 9
  * waves. */
 LBRB_API int lbrb_set_pair_shape(lbrb_t *h, int shape);
 /* the number of launch shapes of the two-step kernel (0 .. n-1) */
@@ -357,17 +352,17 @@ LBRB_API int lbrb_ensemble_get_schedule(const lbrb_ensemble_t *e, int *variant, 
 /* Two steps per launch for every member (as lbrb_set_pairs, with Dirichlet
  * walls; bilinear-nudged members too): every step of a call but its last
  * (and one more when an even count remains) goes in pairs, each pair one
- * launch over all members -- marching over strips of 32 columns x chunks of
- * rows (lb_march_kernel's block) or over tiles (lb_pair_kernel's block), the
- * members' views in shared memory -- with the nudged members' step-n
+ * launch over all members -- marching over strips of 60 columns x chunks of
+ * rows (one warp each, as lb_wave2_kernel) or over tiles (lb_pair_kernel's
+ * block), the members' views in shared memory -- with the nudged members' step-n
  * innovations formed before it and every member's particles, step n+1
  * innovations and nudging apply after it; 12 steps are replayed from a CUDA
  * graph.  Members end bit-identical to lbrb_step.
  * mode -1 (the default) and 1: on; 0: one step per launch.  The launch
- * variant (lbrb_ensemble_pair_variants() of them: marching with 6 or 8 rows
- * per group, tiles of 32 x 8 or 30 x 8 nodes) is timed at the first paired
- * call unless set; lbrb_ensemble_get_pairs reports its rows per group or per
- * tile (0 before) and ms per launch (0 when set rather than timed). */
+ * variant (lbrb_ensemble_pair_variants() of them: marching over chunks of 64,
+ * 32 or 16 rows, tiles of 32 x 8 or 30 x 8 nodes) is timed at the first paired
+ * call unless set; lbrb_ensemble_get_pairs reports the rows a block marches
+ * at a time (one per warp) or a tile's rows (0 before) and ms per launch (0 when set rather than timed). */
 LBRB_API int lbrb_ensemble_set_pairs(lbrb_ensemble_t *e, int mode);
 LBRB_API int lbrb_ensemble_get_pairs(const lbrb_ensemble_t *e, int *mode, int *rows, float *ms);
 LBRB_API int lbrb_ensemble_pair_variants(void);

@@ -357,7 +357,7 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
   // the two extra u, v slots of four-step launches with particles, unless an
   // earlier handle of this kind timed pairs as faster (lbrb_step); a run
   // without memory for them steps in pairs
-  if (h->np > 0 && fp32(h) && p.twall == LBRB_TWALL_DIRICHLET && p.nudge == LBRB_NUDGE_NONE) {
+  if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge == LBRB_NUDGE_NONE) {
     int sh = 0;
     float ms = 0.f;
     const size_t pb1 = h->plane * h->esize;
@@ -1124,23 +1124,30 @@ int lbrb_step(lbrb_t* h, int n) {
   // pairs would leave them in, those of n and n+1 to the extra slots; at most
   // one of the steps is a record step, whose T goes to the source buffer, or
   // for step n+3 to the destination's.  Never the call's last step.
-  auto quad_views = [&](const bool* rec, LBView<float> (&V)[4]) {
+  auto quad_views = [&](auto zero, const bool* rec, auto& V) {
+    using Real = decltype(zero);
     const int src = h->cur, dst = h->cur ^ 1;
     const bool parts = h->np > 0;
     const int slot[4] = {3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
     for (int q = 0; q < 4; q++) {
-      V[q] = make_view<float>(h, src, dst, parts ? slot[q] : h->uvcur, parts ? 1 : 0, rec[q] ? 1 : 0);
-      if (q < 3) V[q].T = (float*)h->T[src];
+      V[q] = make_view<Real>(h, src, dst, parts ? slot[q] : h->uvcur, parts ? 1 : 0, rec[q] ? 1 : 0);
+      if (q < 3) V[q].T = (Real*)h->T[src];
     }
   };
   auto four = [&]() -> int {
     const bool parts = h->np > 0;
     bool rec[4];
     for (int q = 0; q < 4; q++) rec[q] = parts && h->p.noutconfig > 0 && (h->istep + 1 + q) % h->p.noutconfig == 0;
-    LBView<float> V[4];
-    quad_views(rec, V);
     const int tm = tmark_begin(h, 0, h->stream);
-    CK(h, launch_quad_fp32(V, h->quad_shape, h->stream, pdl_ok));
+    if (f32) {
+      LBView<float> V[4];
+      quad_views(0.f, rec, V);
+      CK(h, launch_quad_fp32(V, h->quad_shape, h->stream, pdl_ok));
+    } else {
+      LBView<double> V[4];
+      quad_views(0.0, rec, V);
+      CK(h, launch_quad_fp64(V, h->quad_shape, h->stream, pdl_ok));
+    }
     tmark_end(h, tm, h->stream);
     if (parts) {
       const int slot[5] = {h->uvcur, 3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
@@ -1149,11 +1156,11 @@ int lbrb_step(lbrb_t* h, int n) {
       const int rslot = (int)(h->rec_head % h->p.record_slots);
       for (int q = 0; q < 4; q++) {
         for (int c = 0; c < 2; c++) fields[q][c] = h->uv[slot[q + 1]][c], fields[q][2 + c] = h->uv[slot[q]][c];
-        fields[q][4] = V[q].T;
+        fields[q][4] = h->T[q < 3 ? h->cur : h->cur ^ 1];
         if (rec[q]) r[q] = h->d_ring + (size_t)rslot * h->nrec_fields * h->np;
       }
       const int tp = tmark_begin(h, 1, h->stream);
-      CK(h, launch_particles_quad(fields, true, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full,
+      CK(h, launch_particles_quad(fields, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full,
                                   r, h->dflags, h->stream, pdl_ok));
       tmark_end(h, tp, h->stream);
       for (int q = 0; q < 4; q++)
@@ -1172,7 +1179,7 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   // four steps per launch where a timed launch beats two timed pair launches
   auto quads_ok = [&]() {
-    return f32 && step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed;
+    return step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed;
   };
   auto tune_quads = [&]() -> int {
     h->quad_shape = -1;
@@ -1181,9 +1188,15 @@ int lbrb_step(lbrb_t* h, int n) {
     int sh = 0;
     if (!tuned_get(g_tuned_quad, h, &sh, &ms)) {
       const bool none[4] = {};
-      LBView<float> V[4];
-      quad_views(none, V);
-      sh = tune_quad_fp32(V, h->stream, &ms);
+      if (f32) {
+        LBView<float> V[4];
+        quad_views(0.f, none, V);
+        sh = tune_quad_fp32(V, h->stream, &ms);
+      } else {
+        LBView<double> V[4];
+        quad_views(0.0, none, V);
+        sh = tune_quad_fp64(V, h->stream, &ms);
+      }
       CK(h, cudaGetLastError());
       if (ms >= 2.f * h->pair_ms) sh = -1;
       tuned_put(g_tuned_quad, h, sh, ms);
@@ -2660,17 +2673,15 @@ int lbrb_set_pair_shape(lbrb_t* h, int shape) {
 
 int lbrb_get_pair_shape(const lbrb_t* h, int* shape, int* tile_x, int* tile_y, float* ms) {
   if (!h) return LBRB_ERR_ARG;
-  // (lb_kernels.cu: PAIR_SHAPES, then for FP64 MARCH_SHAPES: a strip of 32
-  // columns walked in groups of tile_y rows; for FP32 WAVE_SHAPES: strips of
-  // 60 columns, one row at a time)
-  static const int TXS[] = {32, 32, 32, 64, 32, 30, 32, 32, 64, 32, 32, 32, 32, 32, 32},
-                   TYS[] = {8, 4, 16, 4, 8, 8, 8, 6, 8, 8, 8, 8, 6, 4, 6};
+  // (lb_kernels.cu: PAIR_SHAPES, then WAVE_SHAPES: strips of 60 columns, one
+  // row at a time)
+  static const int TXS[] = {32, 32, 32, 64, 32, 30, 32, 32, 64, 60, 60, 60, 60, 60, 60},
+                   TYS[] = {8, 4, 16, 4, 8, 8, 8, 6, 8, 1, 1, 1, 1, 1, 1};
   static_assert(sizeof(TXS) / sizeof(int) == NUM_PAIR_SHAPES, "pair shape table");
   const int sh = h->pair_shape;
   if (shape) *shape = sh;
-  const bool wave = sh >= NUM_PAIR_TILES && fp32(h);
-  if (tile_x) *tile_x = sh < 0 ? 0 : (wave ? 60 : TXS[sh]);
-  if (tile_y) *tile_y = sh < 0 ? 0 : (wave ? 1 : TYS[sh]);
+  if (tile_x) *tile_x = sh < 0 ? 0 : TXS[sh];
+  if (tile_y) *tile_y = sh < 0 ? 0 : TYS[sh];
   if (ms) *ms = h->pair_ms;
   return LBRB_OK;
 }

@@ -32,9 +32,11 @@ cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, i
 cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s, bool pdl);
 int tune_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, cudaStream_t s, float* best_ms);
 int tune_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, cudaStream_t s, float* best_ms);
-// four steps per launch (as pairs; FP32, no nudging, no y-slab): one view per step
+// four steps per launch (as pairs; no nudging, no y-slab): one view per step
 cudaError_t launch_quad_fp32(const LBView<float> (&V)[4], int shape, cudaStream_t s, bool pdl);
+cudaError_t launch_quad_fp64(const LBView<double> (&V)[4], int shape, cudaStream_t s, bool pdl);
 int tune_quad_fp32(const LBView<float> (&V)[4], cudaStream_t s, float* best_ms);
+int tune_quad_fp64(const LBView<double> (&V)[4], cudaStream_t s, float* best_ms);
 cudaError_t launch_particles(const void* u, const void* v, const void* ub, const void* vb,
                              const void* T, bool fp32, int nx, int ny, int pitch, double* P,
                              const int* ptype, int np, double beta, int record, int full,

@@ -45,19 +45,16 @@ struct lbrb_ensemble_s {
   cudaGraphExec_t gexec = nullptr;
   int graph_variant = -1;
   // two steps per launch: pair_mode -1 (default) / 1 on, 0 off; pair views
-  // [6 phases][2 steps][n] and their EnsAux, items of the marching kernel
-  // (member, first column, first row, rows) and of each tile variant
-  // (member, first column, first row, 0), the variant (-1: tune), a graph
+  // [6 phases][2 steps][n] and their EnsAux, items of each pair variant
+  // (member, first column, first row, rows), the variant (-1: tune), a graph
   // of 6 pairs (12 steps, the period of the buffer cycle)
   int pair_mode = -1;
   int pair_variant = -1;
   float pair_ms = 0.f;
   void* d_pviews = nullptr;
   void* d_paux = nullptr;
-  int4* d_pitems = nullptr;
-  int npitems = 0;
-  int4* d_titems[ENS_PAIR_VARIANTS - ENS_MARCH_VARIANTS] = {};
-  int ntitems[ENS_PAIR_VARIANTS - ENS_MARCH_VARIANTS] = {};
+  int4* d_pitems[ENS_PAIR_VARIANTS] = {};
+  int npitems[ENS_PAIR_VARIANTS] = {};
   cudaGraph_t pgraph = nullptr;
   cudaGraphExec_t pgexec = nullptr;
   int pgraph_variant = -1;
@@ -339,10 +336,8 @@ const char* paux_at(const lbrb_ensemble_t* e, int ph, int step) {
 
 // the two-step LB launch of variant v over every member, pair phase ph
 static cudaError_t launch_pair_lb(lbrb_ensemble_t* e, int v, int ph) {
-  const bool tile = v >= ENS_MARCH_VARIANTS;
-  return launch_ens_march(e->f32, e->off32, v, pview_at(e, ph, 0), pview_at(e, ph, 1),
-                          tile ? e->d_titems[v - ENS_MARCH_VARIANTS] : e->d_pitems,
-                          tile ? e->ntitems[v - ENS_MARCH_VARIANTS] : e->npitems, e->d_ctr, e->stream);
+  return launch_ens_pair(e->f32, e->off32, v, pview_at(e, ph, 0), pview_at(e, ph, 1), e->d_pitems[v], e->npitems[v],
+                         e->d_ctr, e->stream);
 }
 
 // two steps of every member, pair phase ph (0..5)
@@ -372,10 +367,8 @@ cudaError_t launch_pair(lbrb_ensemble_t* e, int ph) {
   return c;
 }
 
-// work items of the marching kernel: every member's strips of 32 columns x
-// chunks of PAIR_CHUNK rows (whole groups of 6 or 8 rows with the two ring
-// rows); of a tile variant: every member's tiles, row by row
-constexpr int PAIR_CHUNK = 62;
+// work items of the pair variants: every member's strips x chunks of rows, or
+// its tiles, row by row
 static int upload_items(lbrb_ensemble_t* e, const std::vector<int4>& it, int4** d, int* n) {
   EK(e, cudaMalloc(d, it.size() * sizeof(int4)));
   EK(e, cudaMemcpyAsync(*d, it.data(), it.size() * sizeof(int4), cudaMemcpyHostToDevice, e->stream));
@@ -385,23 +378,18 @@ static int upload_items(lbrb_ensemble_t* e, const std::vector<int4>& it, int4** 
 }
 
 int set_pair_items(lbrb_ensemble_t* e) {
-  if (e->d_pitems) return LBRB_OK;
-  std::vector<int4> it;
-  for (size_t i = 0; i < e->m.size(); i++) {
-    const lbrb_t* h = e->m[i];
-    for (int y = 0; y < h->p.ny; y += PAIR_CHUNK)
-      for (int x = 0; x < h->p.nx; x += 32) it.push_back(make_int4((int)i, x, y, std::min(PAIR_CHUNK, h->p.ny - y)));
-  }
-  int rc = upload_items(e, it, &e->d_pitems, &e->npitems);
-  for (int v = ENS_MARCH_VARIANTS; v < ENS_PAIR_VARIANTS && rc == LBRB_OK; v++) {
-    const int tx = ens_pair_tile_cols(v), ty = ens_pair_rows(v);
-    it.clear();
+  int rc = LBRB_OK;
+  for (int v = 0; v < ENS_PAIR_VARIANTS && rc == LBRB_OK; v++) {
+    if (e->d_pitems[v]) continue;
+    int x0, dx, dy;
+    ens_pair_item(v, &x0, &dx, &dy);
+    std::vector<int4> it;
     for (size_t i = 0; i < e->m.size(); i++) {
       const lbrb_t* h = e->m[i];
-      for (int y = 0; y < h->p.ny; y += ty)
-        for (int x = 0; x < h->p.nx; x += tx) it.push_back(make_int4((int)i, x, y, 0));
+      for (int y = 0; y < h->p.ny; y += dy)
+        for (int x = 0; x < h->p.nx; x += dx) it.push_back(make_int4((int)i, x0 + x, y, std::min(dy, h->p.ny - y)));
     }
-    rc = upload_items(e, it, &e->d_titems[v - ENS_MARCH_VARIANTS], &e->ntitems[v - ENS_MARCH_VARIANTS]);
+    rc = upload_items(e, it, &e->d_pitems[v], &e->npitems[v]);
   }
   return rc;
 }
@@ -624,9 +612,9 @@ int lbrb_ensemble_destroy(lbrb_ensemble_t* e) {
   if (e->pgexec) cudaGraphExecDestroy(e->pgexec);
   if (e->pgraph) cudaGraphDestroy(e->pgraph);
   for (void* p : {(void*)e->d_views, (void*)e->d_aux, (void*)e->d_items, (void*)e->d_pch, (void*)e->d_och,
-                  (void*)e->d_ctr, (void*)e->d_pviews, (void*)e->d_paux, (void*)e->d_pitems})
+                  (void*)e->d_ctr, (void*)e->d_pviews, (void*)e->d_paux})
     if (p) cudaFree(p);
-  for (int4* p : e->d_titems)
+  for (int4* p : e->d_pitems)
     if (p) cudaFree(p);
   for (cudaEvent_t ev : e->evpool) cudaEventDestroy(ev);
   if (e->ev) cudaEventDestroy(e->ev);

@@ -114,30 +114,56 @@ __global__ void __launch_bounds__(512)
 }
 
 // ------------------------------------------------- two steps per launch
-// The member's two step views are copied into shared memory; the ring of
-// march_block follows them (dynamic shared memory).  Block 0 counts the two
-// steps in ctr[0] (the later phases pick observation rows from it).
-template <typename Real, int R, int MINB, bool PRE, typename Off>
-__global__ void __launch_bounds__(32 * (R + 1), MINB)
-    ens_march_kernel(const LBView<Real>* __restrict__ views1, const LBView<Real>* __restrict__ views2,
-                     const int4* __restrict__ items, int* __restrict__ ctr) {
-  __shared__ LBView<Real> sV[2];
-  extern __shared__ __align__(16) unsigned char ens_march_smem[];
+// One warp per work item (member, first column, first row, rows), the
+// strip and chunk of wave_march; the warp's copy of the member's two step
+// views precedes its rows in shared memory.  Block 0 counts the two steps in
+// ctr[0] (the later phases pick observation rows from it).
+template <typename Real>
+constexpr int ENS_WAVE_STAGES = std::is_same<Real, float>::value ? 2 : 1;
+template <typename Real>
+constexpr size_t ens_wave_smem() {
+  return wave_smem_bytes<Real, 2, ENS_WAVE_STAGES<Real>>() + (2 * sizeof(LBView<Real>) + 15) / 16 * 16;
+}
+template <typename Real, int NW>
+__global__ void __launch_bounds__(32 * NW, 1)
+    ens_wave_kernel(const LBView<Real>* __restrict__ views1, const LBView<Real>* __restrict__ views2,
+                    const int4* __restrict__ items, int nitems, int* __restrict__ ctr) {
+  extern __shared__ __align__(16) unsigned char ens_wave_mem[];
   pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr[0], 2);
-  const int4 w = items[blockIdx.x];  // (member, first column, first row, rows)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int it = blockIdx.x * NW + warp;
+  if (it >= nitems) return;
+  const int4 w = items[it];
   constexpr int WORDS = (int)(sizeof(LBView<Real>) / sizeof(int));
   static_assert(sizeof(LBView<Real>) % sizeof(int) == 0, "view size");
+  unsigned char* mine = ens_wave_mem + warp * ens_wave_smem<Real>();
+  int* d = reinterpret_cast<int*>(mine + wave_smem_bytes<Real, 2, ENS_WAVE_STAGES<Real>>());
   const int* s1 = reinterpret_cast<const int*>(views1 + w.x);
   const int* s2 = reinterpret_cast<const int*>(views2 + w.x);
-  int* d = reinterpret_cast<int*>(sV);
-  for (int i = threadIdx.x; i < 2 * WORDS; i += blockDim.x) d[i] = i < WORDS ? s1[i] : s2[i - WORDS];
-  __syncthreads();
-  march_block<Real, R, PRE, Off>(sV[0], sV[1], w.y, w.z, w.w, ens_march_smem);
+  for (int i = lane; i < 2 * WORDS; i += 32) d[i] = i < WORDS ? s1[i] : s2[i - WORDS];
+  __syncwarp();
+  const LBView<Real>* V = reinterpret_cast<const LBView<Real>*>(d);
+  const int ncols = min(WAVE_COLS<2>, V[0].nx - (w.y - WAVE_X0<2>));
+  if constexpr (std::is_same<Real, float>::value) {
+    // local copies: what the march uses of the views stays in registers
+    // (676 against 694 us per launch; in FP64 they would spill)
+    const LBView<Real> V1 = V[0], V2 = V[1];
+    wave_march<Real, 2, ENS_WAVE_STAGES<Real>, true>(
+        [&](auto s) -> const LBView<Real>& {
+          if constexpr (decltype(s)::value == 0) return V1;
+          else return V2;
+        },
+        w.y, ncols, w.z, w.w, reinterpret_cast<Real*>(mine));
+  } else {
+    wave_march<Real, 2, ENS_WAVE_STAGES<Real>, true>(
+        [&](auto s) -> const LBView<Real>& { return V[decltype(s)::value]; }, w.y, ncols, w.z, w.w,
+        reinterpret_cast<Real*>(mine));
+  }
 }
 
 // The tile variant: work items (member, x0, y0, 0), one TX x TY tile each
-// (tile_block), the views as in ens_march_kernel
+// (tile_block), the views in shared memory
 template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
 __global__ void __launch_bounds__(NT, MINB)
     ens_tile_kernel(const LBView<Real>* __restrict__ views1, const LBView<Real>* __restrict__ views2,
@@ -220,30 +246,38 @@ __global__ void __launch_bounds__(512)
   obs_clear_one(A1.nx, A1.ny, A1.pitch, o1[o], o1[A1.nobs + o], threadIdx.x & 3, A1.acc2, A1.nmask);
 }
 
-// pair variants 0-2, marching: (rows per group, min blocks per SM, software
-// pipelining); 3-4, tiles: (tile columns, tile rows, threads, min blocks per
-// SM), as the single runs' pair shapes 6 and 5
-constexpr int3 ENS_PAIR_TABLE[ENS_MARCH_VARIANTS] = {{8, 3, 0}, {8, 3, 1}, {6, 4, 1}};
+// pair variants 0-2, strips (chunk heights, ens_pair_chunk); 3-4, tiles: (tile
+// columns, tile rows, threads, min blocks per SM), as the single runs' pair
+// shapes 6 and 5
+constexpr int ENS_WAVE_WARPS = 8;  // per block and SM, as the single runs' FP64 and most FP32 strip shapes
+constexpr int ENS_CHUNK_TABLE[ENS_MARCH_VARIANTS] = {64, 32, 16};
 constexpr int4 ENS_TILE_TABLE[ENS_PAIR_VARIANTS - ENS_MARCH_VARIANTS] = {{32, 8, 256, 5}, {30, 8, 320, 3}};
 int ens_pair_rows(int variant) {
-  return variant < ENS_MARCH_VARIANTS ? ENS_PAIR_TABLE[variant].x : ENS_TILE_TABLE[variant - ENS_MARCH_VARIANTS].y;
+  return variant < ENS_MARCH_VARIANTS ? ENS_WAVE_WARPS : ENS_TILE_TABLE[variant - ENS_MARCH_VARIANTS].y;
 }
 int ens_pair_tile_cols(int variant) {
   return variant < ENS_MARCH_VARIANTS ? 0 : ENS_TILE_TABLE[variant - ENS_MARCH_VARIANTS].x;
 }
+void ens_pair_item(int variant, int* x0, int* dx, int* dy) {
+  if (variant < ENS_MARCH_VARIANTS) {
+    *x0 = WAVE_X0<2>, *dx = WAVE_COLS<2>, *dy = ENS_CHUNK_TABLE[variant];
+  } else {
+    const int4 t = ENS_TILE_TABLE[variant - ENS_MARCH_VARIANTS];
+    *x0 = 0, *dx = t.x, *dy = t.y;
+  }
+}
 
-template <typename Real, int R, int MINB, bool PRE, typename Off>
-static cudaError_t ens_march_launch(const void* v1, const void* v2, const int4* items, int nitems, int* ctr,
-                                    cudaStream_t s) {
-  constexpr int MB = std::is_same<Real, double>::value ? (MINB + 1) / 2 : MINB;
-  auto k = ens_march_kernel<Real, R, MB, PRE, Off>;
-  constexpr size_t smem = march_smem_bytes<Real, R>();
+template <typename Real>
+static cudaError_t ens_wave_launch(const void* v1, const void* v2, const int4* items, int nitems, int* ctr,
+                                   cudaStream_t s) {
+  constexpr auto k = ens_wave_kernel<Real, ENS_WAVE_WARPS>;
+  constexpr size_t smem = ENS_WAVE_WARPS * ens_wave_smem<Real>();
   static std::atomic<unsigned long long> attr_set{0};
   const cudaError_t e = smem_limit_once((const void*)k, smem, attr_set);
   if (e != cudaSuccess) return e;
   if (nitems <= 0) return cudaSuccess;
-  return launch_k(k, nitems, 32 * (R + 1), smem, s, true, (const LBView<Real>*)v1, (const LBView<Real>*)v2,
-                  items, ctr);
+  return launch_k(k, (nitems + ENS_WAVE_WARPS - 1) / ENS_WAVE_WARPS, 32 * ENS_WAVE_WARPS, smem, s, true,
+                  (const LBView<Real>*)v1, (const LBView<Real>*)v2, items, nitems, ctr);
 }
 
 template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
@@ -260,25 +294,23 @@ static cudaError_t ens_tile_launch(const void* v1, const void* v2, const int4* i
 }
 
 template <typename Real, typename Off>
-static cudaError_t ens_march_dispatch(int variant, const void* v1, const void* v2, const int4* items, int nitems,
-                                      int* ctr, cudaStream_t s) {
+static cudaError_t ens_pair_dispatch(int variant, const void* v1, const void* v2, const int4* items, int nitems,
+                                     int* ctr, cudaStream_t s) {
   static_assert(ENS_PAIR_VARIANTS == 5, "pair variants");
   switch (variant) {
-    case 1: return ens_march_launch<Real, 8, 3, true, Off>(v1, v2, items, nitems, ctr, s);
-    case 2: return ens_march_launch<Real, 6, 4, true, Off>(v1, v2, items, nitems, ctr, s);
     case 3: return ens_tile_launch<Real, 32, 8, 256, 5, Off>(v1, v2, items, nitems, ctr, s);
     case 4: return ens_tile_launch<Real, 30, 8, 320, 3, Off>(v1, v2, items, nitems, ctr, s);
-    default: return ens_march_launch<Real, 8, 3, false, Off>(v1, v2, items, nitems, ctr, s);
+    default: return ens_wave_launch<Real>(v1, v2, items, nitems, ctr, s);
   }
 }
 
-cudaError_t launch_ens_march(bool f32, bool off32, int variant, const void* views1, const void* views2,
-                             const int4* items, int nitems, int* ctr, cudaStream_t s) {
+cudaError_t launch_ens_pair(bool f32, bool off32, int variant, const void* views1, const void* views2,
+                            const int4* items, int nitems, int* ctr, cudaStream_t s) {
   if (f32)
-    return off32 ? ens_march_dispatch<float, uint32_t>(variant, views1, views2, items, nitems, ctr, s)
-                 : ens_march_dispatch<float, size_t>(variant, views1, views2, items, nitems, ctr, s);
-  return off32 ? ens_march_dispatch<double, uint32_t>(variant, views1, views2, items, nitems, ctr, s)
-               : ens_march_dispatch<double, size_t>(variant, views1, views2, items, nitems, ctr, s);
+    return off32 ? ens_pair_dispatch<float, uint32_t>(variant, views1, views2, items, nitems, ctr, s)
+                 : ens_pair_dispatch<float, size_t>(variant, views1, views2, items, nitems, ctr, s);
+  return off32 ? ens_pair_dispatch<double, uint32_t>(variant, views1, views2, items, nitems, ctr, s)
+               : ens_pair_dispatch<double, size_t>(variant, views1, views2, items, nitems, ctr, s);
 }
 
 cudaError_t launch_ens_pre(bool f32, const void* views1, const void* aux1, const int2* ochunks, int nochunks,

@@ -76,51 +76,42 @@ __global__ void __launch_bounds__(NT, MINB) lb_pair_kernel(const LBView<Real> V1
   tile_block<Real, TX, TY, NT, Off>(V1, V2, blockIdx.x * TX, blockIdx.y * TY, pair_smem);
 }
 
-template <typename Real, int R, int MINB, bool PRE, typename Off>
-__global__ void __launch_bounds__(32 * (R + 1), MINB)
-    lb_march_kernel(const LBView<Real> V1, const LBView<Real> V2, int H) {
-  pdl_wait();
-  extern __shared__ __align__(16) unsigned char march_smem[];
-  const int nstrips = (V1.nx + 31) >> 5;
-  const int strip = blockIdx.x % nstrips, chunk = blockIdx.x / nstrips;
-  const int ya = chunk * H;
-  march_block<Real, R, PRE, Off>(V1, V2, strip * 32, ya, min(H, V1.ny - ya), march_smem);
-}
-
-template <int NW, int MINB, int D, bool NUD>
+// marching (lb_pair.cuh: wave_march): item = strip + chunk * nstrips, one per warp
+template <typename Real, int NW, int MINB, int D, bool NUD>
 __global__ void __launch_bounds__(32 * NW, MINB)
-    lb_wave2_kernel(const LBView<float> V1, const LBView<float> V2, int H, int nitems) {
+    lb_wave2_kernel(const LBView<Real> V1, const LBView<Real> V2, int H, int nitems) {
   pdl_wait();
-  extern __shared__ __align__(16) float wave_smem[];
+  extern __shared__ __align__(16) unsigned char wave_smem[];
   const int w = threadIdx.x >> 5, item = blockIdx.x * NW + w;
   if (item >= nitems) return;
   const int nstrips = (V1.nx + WAVE_COLS<2> - 1) / WAVE_COLS<2>;
   const int strip = item % nstrips, ya = item / nstrips * H;
-  wave_march<2, D, NUD>([&](auto s) -> const LBView<float>& { return decltype(s)::value == 0 ? V1 : V2; },
-                        strip * WAVE_COLS<2> + WAVE_X0<2>, min(WAVE_COLS<2>, V1.nx - strip * WAVE_COLS<2>), ya,
-                        min(H, V1.ny - ya), wave_smem + w * wave_smem_floats<2, D>());
+  wave_march<Real, 2, D, NUD>([&](auto s) -> const LBView<Real>& { return decltype(s)::value == 0 ? V1 : V2; },
+                              strip * WAVE_COLS<2> + WAVE_X0<2>, min(WAVE_COLS<2>, V1.nx - strip * WAVE_COLS<2>), ya,
+                              min(H, V1.ny - ya),
+                              reinterpret_cast<Real*>(wave_smem + w * wave_smem_bytes<Real, 2, D>()));
 }
 
 // four steps per launch: the populations and F cross HBM once per four steps
-template <int NW, int MINB, int D>
+template <typename Real, int NW, int MINB, int D>
 __global__ void __launch_bounds__(32 * NW, MINB)
-    lb_wave4_kernel(const LBView<float> V1, const LBView<float> V2, const LBView<float> V3, const LBView<float> V4,
+    lb_wave4_kernel(const LBView<Real> V1, const LBView<Real> V2, const LBView<Real> V3, const LBView<Real> V4,
                     int H, int nitems) {
   pdl_wait();
-  extern __shared__ __align__(16) float wave_smem[];
+  extern __shared__ __align__(16) unsigned char wave_smem[];
   const int w = threadIdx.x >> 5, item = blockIdx.x * NW + w;
   if (item >= nitems) return;
   const int nstrips = (V1.nx + WAVE_COLS<4> - 1) / WAVE_COLS<4>;
   const int strip = item % nstrips, ya = item / nstrips * H;
-  wave_march<4, D, false>(
-      [&](auto s) -> const LBView<float>& {
+  wave_march<Real, 4, D, false>(
+      [&](auto s) -> const LBView<Real>& {
         if constexpr (decltype(s)::value == 0) return V1;
         else if constexpr (decltype(s)::value == 1) return V2;
         else if constexpr (decltype(s)::value == 2) return V3;
         else return V4;
       },
       strip * WAVE_COLS<4> + WAVE_X0<4>, min(WAVE_COLS<4>, V1.nx - strip * WAVE_COLS<4>), ya, min(H, V1.ny - ya),
-      wave_smem + w * wave_smem_floats<4, D>());
+      reinterpret_cast<Real*>(wave_smem + w * wave_smem_bytes<Real, 4, D>()));
 }
 
 // pair launch shapes: (tile columns, tile rows, threads, min blocks per SM)
@@ -149,123 +140,90 @@ static cudaError_t launch_pair_t(const LBView<Real>& V1, const LBView<Real>& V2,
   return go(lb_pair_kernel<Real, TX, TY, NT, MB, size_t>);
 }
 
-// FP64 marching launch shapes: (rows per group R, min blocks per SM, waves): the
-// chunk height H = kR - 2 (whole groups) is chosen so that the grid of
-// strips x chunks holds about `waves` waves of resident blocks
-struct MarchShape { int r, minb, waves, pre; };
-constexpr MarchShape MARCH_SHAPES[] = {{8, 3, 8, 0}, {8, 3, 8, 1}, {8, 2, 8, 1},
-                                       {6, 4, 8, 1}, {4, 6, 8, 1}, {6, 3, 8, 1}};
-constexpr int NMARCH = sizeof(MARCH_SHAPES) / sizeof(MARCH_SHAPES[0]);
-static_assert(NPAIR + NMARCH == NUM_PAIR_SHAPES, "pair shape table");
-
-template <typename Real, int R, int MINB, bool PRE>
-static cudaError_t launch_march_t(const LBView<Real>& V1, const LBView<Real>& V2, int waves, cudaStream_t s,
-                                  bool pdl) {
-  constexpr int NT = 32 * (R + 1);
-  constexpr size_t smem = march_smem_bytes<Real, R>();
-  // (FP64 holds twice the registers and shared memory per value: half the blocks per SM)
-  constexpr int MB = std::is_same<Real, double>::value ? (MINB + 1) / 2 : MINB;
-  auto go = [&](auto kernel) -> cudaError_t {
-    static std::atomic<unsigned long long> attr_set{0};
-    static std::atomic<int> occ_cache[MAX_DEVICES] = {};
-    cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
-    if (e != cudaSuccess) return e;
-    int occ = 0, dev = 0, nsm = 0;
-    e = occupancy_once((const void*)kernel, NT, smem, occ_cache, &occ);
-    if (e == cudaSuccess) e = current_device(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    const int nx = V1.nx, ny = V1.ny;
-    const long nstrips = (nx + 31) / 32;
-    const long target = std::max(1L, ((long)waves * occ * nsm + nstrips / 2) / nstrips);  // chunks
-    const int h0 = (int)((ny + target - 1) / target);
-    const int H = ((h0 + 2 + R - 1) / R) * R - 2;  // whole groups of R rows
-    const long nchunks = (ny + H - 1) / H;
-    return launch_k(kernel, dim3((unsigned)(nstrips * nchunks)), NT, smem, s, pdl, V1, V2, H);
-  };
-  if (off32_ok(V1.plane)) return go(lb_march_kernel<Real, R, MB, PRE, uint32_t>);
-  return go(lb_march_kernel<Real, R, MB, PRE, size_t>);
-}
-
-// The FP32 marching shapes: wave_march, one warp per strip and chunk, (warps
-// per block, min blocks per SM, waves).  The chunk height is chosen so that
-// the items (strips x chunks) fill at most `waves` waves of resident warps:
-// few waves recompute fewer rows (two per chunk), many keep the warps of a
-// row band together, which the DRAM pages reward.  8 or 12 warps per SM: 15
-// of them (128 registers) ran 10% slower (128 against 118 us per step at
-// 4096x2048), their copies queueing behind one another.
+// The marching shapes: wave_march, one warp per strip and chunk, (warps per
+// block, min blocks per SM, waves) in FP32; in FP64 8 warps per SM and the
+// waves.  The chunk height is chosen so that the items (strips x chunks) fill
+// at most `waves` waves of resident warps: few waves recompute fewer rows
+// (two per chunk), many keep the warps of a row band together, which the DRAM
+// pages reward.  FP32, 4096x2048: 118 us per step with 8 warps per SM (6
+// waves) and with 12 (9 waves); with 15 (128 registers) 128 us, their copies
+// queueing behind one another.  FP64 (about 240 registers): 231 us with 8
+// warps, 345 with 11 (168 registers, spilling); the 32x6 tile takes 282.
 struct WaveShape { int nw, minb, waves; };
+constexpr int NMARCH = NUM_PAIR_SHAPES - NPAIR;
 constexpr WaveShape WAVE_SHAPES[NMARCH] = {{8, 1, 1}, {8, 1, 2}, {8, 1, 3}, {8, 1, 6}, {4, 3, 4}, {4, 3, 9}};
-constexpr int WAVE2_STAGES = 2;  // rows of inputs in flight per warp
+constexpr int WAVE_SHAPES_FP64[NMARCH] = {1, 2, 3, 4, 6, 9};
+// rows of inputs in flight per warp
+constexpr int WAVE2_STAGES = 2, WAVE2_STAGES_FP64 = 1;
 
-template <int NW, int MINB, bool NUD>
-static cudaError_t launch_wave2_t(const LBView<float>& V1, const LBView<float>& V2, int waves, cudaStream_t s,
-                                  bool pdl) {
-  constexpr auto kernel = lb_wave2_kernel<NW, MINB, WAVE2_STAGES, NUD>;
-  constexpr size_t smem = NW * wave_smem_floats<2, WAVE2_STAGES>() * sizeof(float);
-  static std::atomic<unsigned long long> attr_set{0};
-  static std::atomic<int> occ_cache[MAX_DEVICES] = {};
-  cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
-  if (e != cudaSuccess) return e;
+// the chunk height for `waves` waves of resident warps, and the items
+template <typename Kernel>
+static cudaError_t wave_grid(Kernel kernel, int nw, size_t smem, std::atomic<int>* occ_cache, int waves, int cols,
+                             int nx, int ny, int* H, long* nitems) {
   int occ = 0, dev = 0, nsm = 0;
-  e = occupancy_once((const void*)kernel, 32 * NW, smem, occ_cache, &occ);
+  cudaError_t e = occupancy_once((const void*)kernel, 32 * nw, smem, occ_cache, &occ);
   if (e == cudaSuccess) e = current_device(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  const int ny = V1.ny;
-  const long nstrips = (V1.nx + WAVE_COLS<2> - 1) / WAVE_COLS<2>;
-  const long chunks = std::min((long)ny, std::max(1L, (long)waves * occ * nsm * NW / nstrips));
-  const int H = (int)((ny + chunks - 1) / chunks);
-  const long nitems = nstrips * ((ny + H - 1) / H);
+  const long nstrips = (nx + cols - 1) / cols;
+  const long chunks = std::min((long)ny, std::max(1L, (long)waves * occ * nsm * nw / nstrips));
+  *H = (int)((ny + chunks - 1) / chunks);
+  *nitems = nstrips * ((ny + *H - 1) / *H);
+  return cudaSuccess;
+}
+
+template <typename Real, int NW, int MINB, int D, bool NUD>
+static cudaError_t launch_wave2_t(const LBView<Real>& V1, const LBView<Real>& V2, int waves, cudaStream_t s,
+                                  bool pdl) {
+  constexpr auto kernel = lb_wave2_kernel<Real, NW, MINB, D, NUD>;
+  constexpr size_t smem = NW * wave_smem_bytes<Real, 2, D>();
+  static std::atomic<unsigned long long> attr_set{0};
+  static std::atomic<int> occ_cache[MAX_DEVICES] = {};
+  cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
+  int H = 0;
+  long nitems = 0;
+  if (e == cudaSuccess) e = wave_grid(kernel, NW, smem, occ_cache, waves, WAVE_COLS<2>, V1.nx, V1.ny, &H, &nitems);
+  if (e != cudaSuccess) return e;
   return launch_k(kernel, dim3((unsigned)((nitems + NW - 1) / NW)), 32 * NW, smem, s, pdl, V1, V2, H, (int)nitems);
+}
+static cudaError_t launch_march(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
+  const WaveShape w = WAVE_SHAPES[m];
+  if (w.nw == 8)
+    return V1.nmask ? launch_wave2_t<float, 8, 1, WAVE2_STAGES, true>(V1, V2, w.waves, s, pdl)
+                    : launch_wave2_t<float, 8, 1, WAVE2_STAGES, false>(V1, V2, w.waves, s, pdl);
+  return V1.nmask ? launch_wave2_t<float, 4, 3, WAVE2_STAGES, true>(V1, V2, w.waves, s, pdl)
+                  : launch_wave2_t<float, 4, 3, WAVE2_STAGES, false>(V1, V2, w.waves, s, pdl);
+}
+static cudaError_t launch_march(const LBView<double>& V1, const LBView<double>& V2, int m, cudaStream_t s, bool pdl) {
+  return V1.nmask ? launch_wave2_t<double, 8, 1, WAVE2_STAGES_FP64, true>(V1, V2, WAVE_SHAPES_FP64[m], s, pdl)
+                  : launch_wave2_t<double, 8, 1, WAVE2_STAGES_FP64, false>(V1, V2, WAVE_SHAPES_FP64[m], s, pdl);
 }
 
 // four-step launch shapes: waves of resident warps the chunk height aims at
 constexpr int QUAD_WAVES[NUM_QUAD_SHAPES] = {1, 2, 4};
-cudaError_t launch_quad_fp32(const LBView<float> (&V)[4], int shape, cudaStream_t s, bool pdl) {
-  constexpr int NW = 4, MINB = 3, D = 1;
-  constexpr auto kernel = lb_wave4_kernel<NW, MINB, D>;
-  constexpr size_t smem = NW * wave_smem_floats<4, D>() * sizeof(float);
+template <typename Real>
+static cudaError_t launch_quad(const LBView<Real> (&V)[4], int shape, cudaStream_t s, bool pdl) {
+  // 12 warps per SM in FP32, 6 in FP64 (shared memory)
+  constexpr bool F32 = std::is_same<Real, float>::value;
+  constexpr int NW = F32 ? 4 : 6, MINB = F32 ? 3 : 1, D = 1;
+  constexpr auto kernel = lb_wave4_kernel<Real, NW, MINB, D>;
+  constexpr size_t smem = NW * wave_smem_bytes<Real, 4, D>();
   static std::atomic<unsigned long long> attr_set{0};
   static std::atomic<int> occ_cache[MAX_DEVICES] = {};
   cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
+  int H = 0;
+  long nitems = 0;
+  if (e == cudaSuccess)
+    e = wave_grid(kernel, NW, smem, occ_cache, QUAD_WAVES[shape], WAVE_COLS<4>, V[0].nx, V[0].ny, &H, &nitems);
   if (e != cudaSuccess) return e;
-  int occ = 0, dev = 0, nsm = 0;
-  e = occupancy_once((const void*)kernel, 32 * NW, smem, occ_cache, &occ);
-  if (e == cudaSuccess) e = current_device(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  const int ny = V[0].ny;
-  const long nstrips = (V[0].nx + WAVE_COLS<4> - 1) / WAVE_COLS<4>;
-  const long chunks = std::min((long)ny, std::max(1L, (long)QUAD_WAVES[shape] * occ * nsm * NW / nstrips));
-  const int H = (int)((ny + chunks - 1) / chunks);
-  const long nitems = nstrips * ((ny + H - 1) / H);
   return launch_k(kernel, dim3((unsigned)((nitems + NW - 1) / NW)), 32 * NW, smem, s, pdl, V[0], V[1], V[2], V[3], H,
                   (int)nitems);
 }
-
-static cudaError_t launch_wave2(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
-  const WaveShape w = WAVE_SHAPES[m];
-  if (w.nw == 8)
-    return V1.nmask ? launch_wave2_t<8, 1, true>(V1, V2, w.waves, s, pdl)
-                    : launch_wave2_t<8, 1, false>(V1, V2, w.waves, s, pdl);
-  return V1.nmask ? launch_wave2_t<4, 3, true>(V1, V2, w.waves, s, pdl)
-                  : launch_wave2_t<4, 3, false>(V1, V2, w.waves, s, pdl);
+cudaError_t launch_quad_fp32(const LBView<float> (&V)[4], int shape, cudaStream_t s, bool pdl) {
+  return launch_quad<float>(V, shape, s, pdl);
 }
-
-static cudaError_t launch_march(const LBView<double>& V1, const LBView<double>& V2, int m, cudaStream_t s, bool pdl) {
-  const int waves = MARCH_SHAPES[m].waves;
-  switch (m) {
-    case 1: return launch_march_t<double, 8, 3, true>(V1, V2, waves, s, pdl);
-    case 2: return launch_march_t<double, 8, 2, true>(V1, V2, waves, s, pdl);
-    case 3: return launch_march_t<double, 6, 4, true>(V1, V2, waves, s, pdl);
-    case 4: return launch_march_t<double, 4, 6, true>(V1, V2, waves, s, pdl);
-    case 5: return launch_march_t<double, 6, 3, true>(V1, V2, waves, s, pdl);
-    default: return launch_march_t<double, 8, 3, false>(V1, V2, waves, s, pdl);
-  }
-}
-static cudaError_t launch_march(const LBView<float>& V1, const LBView<float>& V2, int m, cudaStream_t s, bool pdl) {
-  return launch_wave2(V1, V2, m, s, pdl);
+cudaError_t launch_quad_fp64(const LBView<double> (&V)[4], int shape, cudaStream_t s, bool pdl) {
+  return launch_quad<double>(V, shape, s, pdl);
 }
 
 template <typename Real>
@@ -332,7 +290,8 @@ cudaError_t launch_lb_fp32(const LBView<float>& V, int twall, int shape, cudaStr
 }
 
 // Autotuner: time every launch shape on this run's grid (CUDA events, `reps`
-// launches after one warm-up launch each) and return the fastest.  A trial
+// launches after one warm-up launch each, with programmatic dependent launch
+// as the steps use) and return the fastest.  A trial
 // launch reads the current state and writes only buffers the real step
 // overwrites: the other population buffer, the other F buffer and, when the
 // caller's view stores u, v (runs with particles), the u, v slot of the next
@@ -353,8 +312,8 @@ static int tune(const LBView<Real>& Vin, int twall, bool refnudge, cudaStream_t 
   for (int round = 0; round < 2; round++) {
     for (int sh = 0; sh < NSHAPES; sh++) {
       auto go = [&]() {
-        if constexpr (std::is_same<Real, double>::value) return launch_lb_fp64(V, twall, refnudge, sh, s, false);
-        else return launch_lb_fp32(V, twall, sh, s, false);
+        if constexpr (std::is_same<Real, double>::value) return launch_lb_fp64(V, twall, refnudge, sh, s, true);
+        else return launch_lb_fp32(V, twall, sh, s, true);
       };
       if (go() != cudaSuccess) { cudaGetLastError(); continue; }
       cudaEventRecord(a, s);
@@ -429,12 +388,12 @@ static int tune_pair(const LBView<Real>& A, const LBView<Real>& B, cudaStream_t 
   for (float& m : shape_ms) m = 1e30f;
   for (int round = 0; round < 2; round++) {  // (as tune(): each shape's faster round)
     for (int sh = 0; sh < NUM_PAIR_SHAPES; sh++) {
-      if (launch_pair<Real>(V1, V2, sh, s, false) != cudaSuccess) {
+      if (launch_pair<Real>(V1, V2, sh, s, true) != cudaSuccess) {
         cudaGetLastError();
         continue;
       }
       cudaEventRecord(a, s);
-      for (int r = 0; r < reps; r++) launch_pair<Real>(V1, V2, sh, s, false);
+      for (int r = 0; r < reps; r++) launch_pair<Real>(V1, V2, sh, s, true);
       cudaEventRecord(b, s);
       cudaEventSynchronize(b);
       float ms = 0.f;
@@ -452,8 +411,9 @@ static int tune_pair(const LBView<Real>& A, const LBView<Real>& B, cudaStream_t 
   return best;
 }
 // the four-step launch shapes, timed as tune_pair's (no T or rho stored)
-int tune_quad_fp32(const LBView<float> (&Vin)[4], cudaStream_t s, float* best_ms) {
-  LBView<float> V[4] = {Vin[0], Vin[1], Vin[2], Vin[3]};
+template <typename Real>
+static int tune_quad(const LBView<Real> (&Vin)[4], cudaStream_t s, float* best_ms) {
+  LBView<Real> V[4] = {Vin[0], Vin[1], Vin[2], Vin[3]};
   for (auto& v : V) v.write_rt = 0;
   cudaEvent_t a, b;
   cudaEventCreate(&a);
@@ -463,12 +423,12 @@ int tune_quad_fp32(const LBView<float> (&Vin)[4], cudaStream_t s, float* best_ms
   float bt = 1e30f;
   for (int round = 0; round < 2; round++) {
     for (int sh = 0; sh < NUM_QUAD_SHAPES; sh++) {
-      if (launch_quad_fp32(V, sh, s, false) != cudaSuccess) {
+      if (launch_quad<Real>(V, sh, s, true) != cudaSuccess) {
         cudaGetLastError();
         continue;
       }
       cudaEventRecord(a, s);
-      for (int r = 0; r < reps; r++) launch_quad_fp32(V, sh, s, false);
+      for (int r = 0; r < reps; r++) launch_quad<Real>(V, sh, s, true);
       cudaEventRecord(b, s);
       cudaEventSynchronize(b);
       float ms = 1e30f;
@@ -480,6 +440,12 @@ int tune_quad_fp32(const LBView<float> (&Vin)[4], cudaStream_t s, float* best_ms
   cudaEventDestroy(b);
   if (best_ms) *best_ms = bt / reps;
   return best;
+}
+int tune_quad_fp32(const LBView<float> (&V)[4], cudaStream_t s, float* best_ms) {
+  return tune_quad<float>(V, s, best_ms);
+}
+int tune_quad_fp64(const LBView<double> (&V)[4], cudaStream_t s, float* best_ms) {
+  return tune_quad<double>(V, s, best_ms);
 }
 int tune_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, cudaStream_t s, float* best_ms) {
   return tune_pair<float>(V1, V2, s, best_ms);

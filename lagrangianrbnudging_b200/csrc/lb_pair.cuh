@@ -1,5 +1,5 @@
 // lb_pair.cuh -- device code of the two-step launches shared by the
-// single-run kernels (lb_kernels.cu: lb_pair_kernel, lb_march_kernel) and
+// single-run kernels (lb_kernels.cu: lb_pair_kernel, lb_wave2_kernel, lb_wave4_kernel) and
 // the ensemble's two-step kernels (ensemble_kernels.cu): the ghost rows of a
 // y-slab, the nudging sums of a nudged run, one tile block and one marching
 // block.
@@ -204,150 +204,7 @@ __device__ __forceinline__ void tile_block(const LBView<Real>& V1, const LBView<
   lb_finish_node<Real, false, Off>(V2, (Off)j * pitch + (Off)x, fs, gs, SF[ty * TX + tx]);
 }
 
-// ------------------------------------------- two steps per launch, marching
-// The same two steps as tile_block, with far less recomputation: a block
-// owns a strip of 32 columns [x0, x0 + 32) and a chunk of rows [ya, ya + Hc)
-// and walks down it in groups of R rows.  With ly = y - ya + 1 (ring row
-// index; ly = 0 is the row below the chunk), group q does
-//   phase 1: step n at rows ly in [qR, qR + R) for the 34 region columns
-//            x0-1 .. x0+32 (R warps take the strip's columns of one row
-//            each; one more warp takes the two halo columns of all R rows),
-//            pulled from HBM exactly as lb_update_node pulls, into a ring of
-//            RING = 2R + 2 rows in shared memory; the chunk's own rows also
-//            store u^n, v^n (T^n on a record step) and keep F^{n+1};
-//   one barrier;
-//   phase 2: step n+1 at output rows ly in [qR - 1, qR + R - 1) within
-//            [1, Hc], pulled from the ring with pull_node's wall rules.
-// Phase 2 of group q reads ring rows [qR - 2, qR + R - 1]; phase 1 of group
-// q + 1 overwrites rows [qR - R - 2, qR - 3], which only phase 2 of group
-// q - 1 read, before the barrier of group q: one barrier per group orders
-// the ring.  Recomputed per strip and chunk: the two halo columns and the two
-// rows beyond the chunk (34/32 x (Hc + 2)/Hc node updates in phase 1,
-// against 34 x 10 / (32 x 8) for the 32 x 8 tile).  The per-node arithmetic
-// is lb_update_node's, so the result equals two single steps bit for bit.
-// Slabs: as in tile_block, rows -1 and ny come from the ghost blocks.
-// shared memory of march_block: the ring of step-n populations, then F^{n+1}
-template <typename Real, int R>
-constexpr size_t march_smem_bytes() {
-  return ((size_t)2 * NPOP * (2 * R + 2) * 34 + (size_t)(2 * R + 2) * 32) * sizeof(Real);
-}
-
-// One block's strip [x0, x0 + 32) and chunk of rows [ya, ya + Hc); smem:
-// march_smem_bytes<Real, R>() of shared memory; 32 (R + 1) threads
-// PRE: software pipelining -- a thread pulls its phase-1 inputs of group
-// q + 1 right after the barrier of group q, so the loads are in flight while
-// it computes phase 2 of group q (the inputs live in registers meanwhile)
-template <typename Real, int R, bool PRE, typename Off>
-__device__ __forceinline__ void march_block(const LBView<Real>& V1, const LBView<Real>& V2, int x0, int ya, int Hc,
-                                            unsigned char* smem) {
-  static_assert(2 * R <= 32, "the halo warp takes 2R nodes");
-  constexpr int RING = 2 * R + 2, CW = 34, PL = RING * CW;
-  Real* S = reinterpret_cast<Real*>(smem);  // [2 * NPOP][RING][CW]: f then g of step n
-  Real* SF = S + 2 * NPOP * PL;             // [RING][32]: F^{n+1} at the strip's columns
-  const int nx = V1.nx, ny = V1.ny;
-  const int ncols = min(32, nx - x0);
-  const Off pitch = (Off)V1.pitch;
-  const bool glo = V1.gh2_lo != nullptr, ghi = V1.gh2_hi != nullptr;
-  const int ylo = glo ? -1 : 0, yhi = ghi ? ny : ny - 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // this thread's phase-1 node: row w of the group, column x, ring column c
-  int w, x, c;
-  bool col_ok;
-  if (warp < R) {
-    w = warp;
-    x = x0 + lane;
-    c = lane + 1;
-    col_ok = lane < ncols;
-  } else {
-    const bool right = lane >= R;  // lanes [0, R): column x0 - 1; [R, 2R): x0 + ncols
-    w = right ? lane - R : lane;
-    c = right ? ncols + 1 : 0;
-    x = right ? x0 + ncols : x0 - 1;
-    if (x < 0) x += nx;
-    else if (x >= nx) x -= nx;
-    col_ok = lane < 2 * R;
-  }
-  // phase-1 inputs of this thread's node in group q: the pulled populations
-  // (walls applied), the step's buoyancy, the nudging sum of a nudged run
-  Real fs[NPOP], gs[NPOP], Fy = Real(0);
-  long long nsum = 0;
-  bool on = false;
-  int y1 = 0, slot = 0;
-  Off o1 = 0;
-  auto fetch = [&](int q) {
-    const int ly = q * R + w;
-    y1 = ya - 1 + ly;
-    on = col_ok && ly <= Hc + 1 && y1 >= ylo && y1 <= yhi;
-    if (!on) return;
-    slot = ly % RING;
-    o1 = (Off)(y1 < 0 ? 0 : (y1 >= ny ? ny - 1 : y1)) * pitch + (Off)x;  // (ghost rows: no stores)
-    if (y1 < 0 || y1 >= ny) {
-      pull_ghost_row<Real, Off>(V1, y1 < 0, x, fs, gs, Fy);
-    } else {
-      pull_node<Real, LBRB_TWALL_DIRICHLET, Off, true>(V1, y1, x, fs, gs);
-      dirichlet_walls(V1, y1, gs);
-      Fy = V1.Fin[o1];
-    }
-    if (V1.nmask) nsum = pair_nudge_sum(V1, y1, x, (size_t)o1);
-  };
-  // phase 1 from the fetched inputs: collide into the ring; the chunk's own
-  // nodes of the strip also store their moments and keep F^{n+1}
-  auto collide = [&]() {
-    if (!on) return;
-    Real r, u, v, t;
-    Real* Sc = S + slot * CW + c;
-    double nsv = 0.0;
-    if (V1.nmask && nsum != 0) nsv = (double)nsum * (1.0 / FIX_SCALE);
-    lb_collide<Real, false>(
-        V1, (size_t)o1, fs, gs, Fy, r, u, v, t, [&](int k, Real val) { Sc[k * PL] = val; },
-        [&](int k, Real val) {
-          if (nsum != 0) val = val + nudge_increment<Real>(k, nsv);
-          Sc[(NPOP + k) * PL] = val;
-        });
-    if (warp < R && y1 >= ya && y1 < ya + Hc) {  // a node of this block's strip and chunk
-      SF[slot * 32 + lane] = Fy;
-      if (V1.write_F) V1.Fout[o1] = Fy;
-      if (V1.write_uv) {
-        V1.u[o1] = u;
-        V1.v[o1] = v;
-      }
-      if (V1.write_rt & 1) V1.T[o1] = t;
-      if (V1.write_rt & 2) V1.rho[o1] = r;
-    }
-  };
-  const int Q = (Hc + 2 + R - 1) / R;
-  if (PRE) fetch(0);
-  for (int q = 0; q < Q; q++) {
-    if (!PRE) fetch(q);
-    collide();
-    __syncthreads();
-    if (PRE && q + 1 < Q) fetch(q + 1);
-    if (warp < R) {
-      const int ly = q * R - 1 + w, y = ya - 1 + ly;
-      if (lane < ncols && ly >= 1 && ly <= Hc) {
-        const int s0 = ly % RING, sm = (ly - 1) % RING, sp = (ly + 1) % RING;
-        Real f2[NPOP], g2[NPOP];
-        static_for<NPOP>([&](auto kc) {
-          constexpr int k = decltype(kc)::value;
-          const int js = y - icy(k);
-          if ((js < 0 && !glo) || (js >= ny && !ghi)) {
-            f2[k] = S[opp(k) * PL + s0 * CW + lane + 1];
-            g2[k] = Real(0);
-          } else {
-            const int sl = icy(k) == 1 ? sm : (icy(k) == -1 ? sp : s0);
-            const int cc = lane + 1 - icx(k);
-            f2[k] = S[k * PL + sl * CW + cc];
-            g2[k] = S[(NPOP + k) * PL + sl * CW + cc];
-          }
-        });
-        dirichlet_walls(V2, y, g2);
-        lb_finish_node<Real, false, Off>(V2, (Off)y * pitch + (Off)(x0 + lane), f2, g2, SF[s0 * 32 + lane]);
-      }
-    }
-  }
-}
-
-// -------------------- S steps per launch, one warp per strip, two FP32 nodes per thread
+// -------------------------- S steps per launch, one warp per strip, two nodes per thread
 // A warp owns a strip of up to WAVE_COLS<S> columns [x0, x0 + ncols) and a
 // chunk of rows [ya, ya + Hc), and walks up it one row per iteration: level 1
 // computes step n at row y, level 2 step n+1 at row y - 1, ..., level S step
@@ -364,9 +221,11 @@ __device__ __forceinline__ void march_block(const LBView<Real>& V1, const LBView
 // 2 (32 - S) columns, and recomputes S - s rows beyond each end of its chunk.
 // Level 1's inputs come through D stages of shared memory filled by 16-byte
 // asynchronous copies: a row's 64 columns from x0 - S (a multiple of 4, so x0
-// is 2 mod 4 for S = 2 and 0 mod 4 for S = 4) of one population of f (lanes
-// 0-15) and of g (lanes 16-31), each from the row it streams out of, per
-// instruction.  Strips wrap around in x, pair by pair.
+// is 2 mod 4 for S = 2 and 0 mod 4 for S = 4), each population from the row
+// it streams out of; in FP32 one instruction copies a population of f (lanes
+// 0-15) and of g (lanes 16-31).  Strips wrap around in x, pair by pair.
+// FP32 collides the pair in two-lane arithmetic (node_shift2), FP64 one node
+// after the other in the reference's order (node_ref).
 // Wall rows bounce back from the node's own populations: at row 0 the slot
 // of row -1 takes the level's f4, f7, f8 instead (read at the node's own
 // columns); at the top the c_y = +1 populations of the row itself are there.
@@ -384,13 +243,44 @@ constexpr int WAVE_X0 = S % 4;  // first strip's x0
 constexpr int WAVE_SLOTS = 7 + 2 * 6, WAVE_STAGE = 2 * NPOP + 1;
 constexpr int wave_cols(int level) { return 2 * (32 - level); }
 constexpr int wave_lag(int level) { return level == 0 ? 0 : wave_lag(level - 1) + WAVE_SLOTS * wave_cols(level); }
-template <int S, int D>
-constexpr size_t wave_smem_floats() {
-  return ((size_t)D * WAVE_STAGE * 64 + wave_lag(S - 1) + 8 + 3) / 4 * 4;
+template <typename Real, int S, int D>
+constexpr size_t wave_smem_bytes() {
+  return ((size_t)D * WAVE_STAGE * 64 + wave_lag(S - 1) + 8 + 3) / 4 * 4 * sizeof(Real);
 }
 
-__device__ __forceinline__ void stcs2(char* p, unsigned o, float2 a) { __stcs(reinterpret_cast<float2*>(p + o), a); }
-__device__ __forceinline__ void cp16(unsigned dst, const float* src) {
+template <typename Real>
+struct PairOf { using type = float2; };
+template <>
+struct PairOf<double> { using type = double2; };
+template <typename Real>
+using Pair = typename PairOf<Real>::type;
+__device__ __forceinline__ float2 pair_of(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 pair_of(double a, double b) { return make_double2(a, b); }
+// the collision of a pair of nodes
+__device__ __forceinline__ void collide_pair(const LBView<float>& V, float2* f, float2* g, float2& F, float2& r,
+                                             float2& u, float2& v, float2& t) {
+  node_shift2(V, f, g, F, r, u, v, t);
+}
+__device__ __forceinline__ void collide_pair(const LBView<double>& V, double2* f, double2* g, double2& F, double2& r,
+                                             double2& u, double2& v, double2& t) {
+  double fa[NPOP], ga[NPOP];
+  auto none = [](int, double) {};
+#pragma unroll
+  for (int k = 0; k < NPOP; k++) fa[k] = f[k].x, ga[k] = g[k].x;
+  node_ref<false>(V, 0, fa, ga, F.x, r.x, u.x, v.x, t.x, none, none);
+#pragma unroll
+  for (int k = 0; k < NPOP; k++) {
+    f[k].x = fa[k], g[k].x = ga[k];
+    fa[k] = f[k].y, ga[k] = g[k].y;
+  }
+  node_ref<false>(V, 0, fa, ga, F.y, r.y, u.y, v.y, t.y, none, none);
+#pragma unroll
+  for (int k = 0; k < NPOP; k++) f[k].y = fa[k], g[k].y = ga[k];
+}
+
+template <typename P>
+__device__ __forceinline__ void stcs2(char* p, unsigned o, P a) { __stcs(reinterpret_cast<P*>(p + o), a); }
+__device__ __forceinline__ void cp16(unsigned dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -399,16 +289,19 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 
 // a level's moments at its strip's aligned pairs (ODD: the lane's second
 // column with its right neighbour's first)
-template <bool ODD>
-__device__ __forceinline__ void wave_put(float* p, float2 a, bool ok) {
-  const float2 b = ODD ? make_float2(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)) : a;
-  if (ok) *reinterpret_cast<float2*>(p) = b;
+template <bool ODD, typename Real>
+__device__ __forceinline__ void wave_put(Real* p, Pair<Real> a, bool ok) {
+  const Pair<Real> b = ODD ? pair_of(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)) : a;
+  if (ok) *reinterpret_cast<Pair<Real>*>(p) = b;
 }
 
-template <int S, int D, bool NUD, typename GetV>
-__device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int ya, int Hc, float* sm) {
+template <typename Real, int S, int D, bool NUD, typename GetV>
+__device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int ya, int Hc, Real* sm) {
+  using P2 = Pair<Real>;
+  constexpr bool F32 = std::is_same<Real, float>::value;
+  constexpr int ES = sizeof(Real), ROW = 64 * ES;  // bytes of a value, of a staged row
   static_assert(S == 2 || S == 4, "x0 - S a multiple of 4 and aligned pairs");
-  const LBView<float>& V1 = view(std::integral_constant<int, 0>{});
+  const LBView<Real>& V1 = view(std::integral_constant<int, 0>{});
   const int nx = V1.nx, ny = V1.ny;
   const unsigned pitch = (unsigned)V1.pitch;
   const size_t plane = V1.plane;
@@ -416,24 +309,29 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   const int ylo = glo ? -1 : 0, yhi = ghi ? ny : ny - 1;
   const int lane = threadIdx.x & 31;
   const int l1 = min(lane + 1, 31);
-  float* const lag = sm + D * WAVE_STAGE * 64;
+  Real* const lag = sm + D * WAVE_STAGE * 64;
   const unsigned sm_addr = (unsigned)__cvta_generic_to_shared(sm);
 
-  // this lane's 4 columns of a staged row
-  const int cq = 4 * (lane & 15);
+  // this lane's 16 bytes of a staged row: of f or g by half-warp in FP32, of
+  // one plane per instruction in FP64
+  constexpr int VEC = 16 / ES;
+  const int cq = VEC * (F32 ? (lane & 15) : lane);
   const bool cp_ok = cq < ncols + 2 * S;
   const unsigned cp_col = (unsigned)((x0 - S + cq + 16 * nx) % nx);
-  const float* const cp_base = (lane < 16 ? V1.fsrc : V1.gsrc) + cp_col;
-  const unsigned cp_dst = sm_addr + (lane < 16 ? 0 : NPOP * 256) + cq * 4;
+  const Real* const cp_base = (!F32 || lane < 16 ? V1.fsrc : V1.gsrc) + cp_col;
+  const unsigned cp_dst = sm_addr + (!F32 || lane < 16 ? 0 : NPOP * ROW) + cq * ES;
+  const ptrdiff_t g_off = F32 ? 0 : V1.gsrc - V1.fsrc;
   auto issue = [&](int y, int stage) {
     if (y > 0 && y < ny - 1 && cp_ok) {
-      const float* p = cp_base + (size_t)((unsigned)y * pitch);
-      const unsigned d = cp_dst + stage * (WAVE_STAGE * 256);
+      const Real* p = cp_base + (size_t)((unsigned)y * pitch);
+      const unsigned d = cp_dst + stage * (WAVE_STAGE * ROW);
       static_for<NPOP>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
-        cp16(d + k * 256, p + ((ptrdiff_t)(k * plane) - (ptrdiff_t)icy(k) * (ptrdiff_t)pitch));
+        const Real* q = p + ((ptrdiff_t)(k * plane) - (ptrdiff_t)icy(k) * (ptrdiff_t)pitch);
+        cp16(d + k * ROW, q);
+        if constexpr (!F32) cp16(d + (NPOP + k) * ROW, q + g_off);
       });
-      if (lane < 16) cp16(d + 2 * NPOP * 256, V1.Fin + ((unsigned)y * pitch + cp_col));
+      if (!F32 || lane < 16) cp16(d + 2 * NPOP * ROW, V1.Fin + ((unsigned)y * pitch + cp_col));
     }
     cp_commit();
   };
@@ -444,7 +342,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   // a row are loaded two iterations ahead, its sums (where a bit is set) one
   const int nxa = (x0 - (S - 1) + 2 * lane + 16 * nx) % nx, nxb = nxa + 1 == nx ? 0 : nxa + 1;
   auto mask_bits = [&](int yy) -> unsigned {
-    if (yy < 0 || yy >= ny) return 0;
+    if (!V1.nmask || yy < 0 || yy >= ny) return 0;  // (an ensemble's members may have none)
     const unsigned* m = V1.nmask + (size_t)yy * (pitch >> 5);
     return ((m[nxa >> 5] >> (nxa & 31)) & 1u) | (((m[nxb >> 5] >> (nxb & 31)) & 1u) << 1);
   };
@@ -463,15 +361,15 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   int stage = 0;
   int p0 = 0, p1 = 6;  // c_y = +1 slots of this iteration's row (and of the row two before it), and of the row before
   for (int it = 0; it < nit; it++, y++) {
-    float2 f[NPOP], g[NPOP], F, r, u, v, t;
+    P2 f[NPOP], g[NPOP], F, r, u, v, t;
     const bool on1 = y >= ylo && y <= yhi;
     cp_wait<D - 1>();
     __syncwarp();
-    const float* st = sm + stage * WAVE_STAGE * 64;
+    const Real* st = sm + stage * WAVE_STAGE * 64;
     // a staged plane at the lane's pair, its right neighbour's, and one column right of its own
-    auto sown = [&](int i) { return reinterpret_cast<const float2*>(st + i * 64)[lane]; };
-    auto snxt = [&](int i) { return reinterpret_cast<const float2*>(st + i * 64)[l1]; };
-    auto smid = [&](int i) { return make_float2(st[i * 64 + 2 * lane + 1], st[i * 64 + 2 * l1]); };
+    auto sown = [&](int i) { return reinterpret_cast<const P2*>(st + i * 64)[lane]; };
+    auto snxt = [&](int i) { return reinterpret_cast<const P2*>(st + i * 64)[l1]; };
+    auto smid = [&](int i) { return pair_of(st[i * 64 + 2 * lane + 1], st[i * 64 + 2 * l1]); };
     if (y > 0 && y < ny - 1) {
       static_for<NPOP>([&](auto kc) {
         constexpr int k = decltype(kc)::value;
@@ -480,13 +378,13 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
       });
       F = smid(2 * NPOP);
     } else if (on1) {
-      float a[2 * NPOP], b[2 * NPOP];
-      auto one = [&](int x, float* p, float& Fx) {
+      Real a[2 * NPOP], b[2 * NPOP];
+      auto one = [&](int x, Real* p, Real& Fx) {
         x = (x + 16 * nx) % nx;
         if (S == 2 && (y < 0 || y >= ny)) {
-          pull_ghost_row<float, size_t>(V1, y < 0, x, p, p + NPOP, Fx);
+          pull_ghost_row<Real, size_t>(V1, y < 0, x, p, p + NPOP, Fx);
         } else {
-          pull_node<float, LBRB_TWALL_DIRICHLET, size_t, false>(V1, y, x, p, p + NPOP);
+          pull_node<Real, LBRB_TWALL_DIRICHLET, size_t, false>(V1, y, x, p, p + NPOP);
           dirichlet_walls(V1, y, p + NPOP);
           Fx = V1.Fin[(unsigned)y * pitch + x];
         }
@@ -495,25 +393,25 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
       one(x0 - (S - 1) + 2 * lane + 1, b, F.y);
 #pragma unroll
       for (int k = 0; k < NPOP; k++) {
-        f[k] = make_float2(a[k], b[k]);
-        g[k] = make_float2(a[NPOP + k], b[NPOP + k]);
+        f[k] = pair_of(a[k], b[k]);
+        g[k] = pair_of(a[NPOP + k], b[NPOP + k]);
       }
     }
     __syncwarp();
     issue(it + D < nit ? y + D : -1, stage);
     stage = stage + 1 == D ? 0 : stage + 1;
     if (on1) {
-      node_shift2(V1, f, g, F, r, u, v, t);
+      collide_pair(V1, f, g, F, r, u, v, t);
       if constexpr (NUD) {
         if (na != 0) {
           const double sv = (double)na * (1.0 / FIX_SCALE);
 #pragma unroll
-          for (int k = 0; k < NPOP; k++) g[k].x = g[k].x + nudge_increment<float>(k, sv);
+          for (int k = 0; k < NPOP; k++) g[k].x = g[k].x + nudge_increment<Real>(k, sv);
         }
         if (nb != 0) {
           const double sv = (double)nb * (1.0 / FIX_SCALE);
 #pragma unroll
-          for (int k = 0; k < NPOP; k++) g[k].y = g[k].y + nudge_increment<float>(k, sv);
+          for (int k = 0; k < NPOP; k++) g[k].y = g[k].y + nudge_increment<Real>(k, sv);
         }
       }
     }
@@ -524,7 +422,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
     static_for<S>([&](auto sc) {
       constexpr int s = decltype(sc)::value + 1;  // level, whose row yr is now in f, g, F and r, u, v, t
       constexpr int off = S - s;
-      const LBView<float>& V = view(std::integral_constant<int, s - 1>{});
+      const LBView<Real>& V = view(std::integral_constant<int, s - 1>{});
       const int yr = y - (s - 1);
       const bool on = s == 1 ? on1 : (yr >= max(ya - off, 0) && yr <= min(ya + Hc - 1 + off, ny - 1));
       // the level's moments (and the last level's state) in its strip and chunk
@@ -533,45 +431,45 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         const bool ok = c >= 0 && c < ncols;
         const int xc = x0 + c;
         const unsigned o = (unsigned)yr * pitch + (unsigned)(xc >= nx ? xc - nx : xc);
-        const unsigned ob = o * 4u;  // (bytes within a plane)
+        const unsigned ob = o * (unsigned)ES;  // (bytes within a plane)
         constexpr bool ODD = (off & 1) != 0;
         if constexpr (s == S) {
           if (ok) {
 #pragma unroll
             for (int k = 0; k < NPOP; k++) {
-              stcs2(reinterpret_cast<char*>(V.fdst) + k * plane * 4, ob, f[k]);
-              stcs2(reinterpret_cast<char*>(V.gdst) + k * plane * 4, ob, g[k]);
+              stcs2(reinterpret_cast<char*>(V.fdst) + k * plane * ES, ob, f[k]);
+              stcs2(reinterpret_cast<char*>(V.gdst) + k * plane * ES, ob, g[k]);
             }
           }
         }
-        if (s == S || V.write_F) wave_put<ODD>(V.Fout + o, F, ok);
+        if (s == S || V.write_F) wave_put<ODD, Real>(V.Fout + o, F, ok);
         if (V.write_uv) {
-          wave_put<ODD>(V.u + o, u, ok);
-          wave_put<ODD>(V.v + o, v, ok);
+          wave_put<ODD, Real>(V.u + o, u, ok);
+          wave_put<ODD, Real>(V.v + o, v, ok);
         }
-        if (V.write_rt & 1) wave_put<ODD>(V.T + o, t, ok);
-        if (V.write_rt & 2) wave_put<ODD>(V.rho + o, r, ok);
+        if (V.write_rt & 1) wave_put<ODD, Real>(V.T + o, t, ok);
+        if (V.write_rt & 2) wave_put<ODD, Real>(V.rho + o, r, ok);
       }
       if constexpr (s < S) {
         // the next level's inputs at row yn; this level's row takes their place
         const int yn = yr - 1;
         const bool lo = yn == 0 && !glo, hi = yn == ny - 1 && !ghi;
         constexpr int CW = wave_cols(s);
-        float* w0 = lag + wave_lag(s - 1);
-        float* w1 = w0 + (7 + p0) * CW;
-        float* wp = w0 + (7 + p1) * CW;
-        auto own = [&](const float* q, int i) { return reinterpret_cast<const float2*>(q + i * CW)[lane]; };
-        auto nxt = [&](const float* q, int i) { return reinterpret_cast<const float2*>(q + i * CW)[l1]; };
-        auto mid = [&](const float* q, int i) { return make_float2(q[i * CW + 2 * lane + 1], q[i * CW + 2 * l1]); };
-        const float2 a0 = mid(w0, 0), a1 = own(w0, 1), a3 = nxt(w0, 2);
-        const float2 b0 = mid(w0, 3), b1 = own(w0, 4), b3 = nxt(w0, 5);
-        const float2 Fn = mid(w0, 6);
-        float2 a2 = mid(w1, 0), a5 = own(w1, 1), a6 = nxt(w1, 2);
+        Real* w0 = lag + wave_lag(s - 1);
+        Real* w1 = w0 + (7 + p0) * CW;
+        Real* wp = w0 + (7 + p1) * CW;
+        auto own = [&](const Real* q, int i) { return reinterpret_cast<const P2*>(q + i * CW)[lane]; };
+        auto nxt = [&](const Real* q, int i) { return reinterpret_cast<const P2*>(q + i * CW)[l1]; };
+        auto mid = [&](const Real* q, int i) { return pair_of(q[i * CW + 2 * lane + 1], q[i * CW + 2 * l1]); };
+        const P2 a0 = mid(w0, 0), a1 = own(w0, 1), a3 = nxt(w0, 2);
+        const P2 b0 = mid(w0, 3), b1 = own(w0, 4), b3 = nxt(w0, 5);
+        const P2 Fn = mid(w0, 6);
+        P2 a2 = mid(w1, 0), a5 = own(w1, 1), a6 = nxt(w1, 2);
         if (lo) a5 = mid(w1, 1), a6 = mid(w1, 2);
-        float2 b2 = mid(w1, 3), b5 = own(w1, 4), b6 = nxt(w1, 5);
+        P2 b2 = mid(w1, 3), b5 = own(w1, 4), b6 = nxt(w1, 5);
         __syncwarp();
         if (on && 2 * lane < CW) {
-          auto put = [&](float* q, int i, float2 a) { reinterpret_cast<float2*>(q + i * CW)[lane] = a; };
+          auto put = [&](Real* q, int i, P2 a) { reinterpret_cast<P2*>(q + i * CW)[lane] = a; };
           put(w0, 0, f[0]), put(w0, 1, f[1]), put(w0, 2, f[3]);
           put(w0, 3, g[0]), put(w0, 4, g[1]), put(w0, 5, g[3]);
           put(w0, 6, F);
@@ -579,33 +477,33 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
           put(w1, 3, g[2]), put(w1, 4, g[5]), put(w1, 5, g[6]);
           if (yr == 0 && !glo) put(wp, 0, f[4]), put(wp, 1, f[7]), put(wp, 2, f[8]);
         }
-        auto shm = [&](float2 a) { return make_float2(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)); };
-        auto shn = [&](float2 a) {
-          return make_float2(__shfl_down_sync(0xffffffffu, a.x, 1), __shfl_down_sync(0xffffffffu, a.y, 1));
+        auto shm = [&](P2 a) { return pair_of(a.y, __shfl_down_sync(0xffffffffu, a.x, 1)); };
+        auto shn = [&](P2 a) {
+          return pair_of(__shfl_down_sync(0xffffffffu, a.x, 1), __shfl_down_sync(0xffffffffu, a.y, 1));
         };
         f[4] = shm(f[4]), f[7] = shn(f[7]);  // (f[8]: the lane's own)
         g[4] = shm(g[4]), g[7] = shn(g[7]);
         f[0] = a0, f[1] = a1, f[3] = a3, f[2] = a2, f[5] = a5, f[6] = a6;
         g[0] = b0, g[1] = b1, g[3] = b3, g[2] = b2, g[5] = b5, g[6] = b6;
         F = Fn;
-        const LBView<float>& VN = view(std::integral_constant<int, s>{});
+        const LBView<Real>& VN = view(std::integral_constant<int, s>{});
         if (lo || hi) {
           if (lo) {
-            g[2] = g[5] = g[6] = make_float2(0.f, 0.f);
+            g[2] = g[5] = g[6] = pair_of(Real(0), Real(0));
           } else {
             f[4] = mid(wp, 0), f[7] = mid(wp, 1), f[8] = mid(wp, 2);
-            g[4] = g[7] = g[8] = make_float2(0.f, 0.f);
+            g[4] = g[7] = g[8] = pair_of(Real(0), Real(0));
           }
-          float ga[NPOP], gb[NPOP];
+          Real ga[NPOP], gb[NPOP];
 #pragma unroll
           for (int k = 0; k < NPOP; k++) ga[k] = g[k].x, gb[k] = g[k].y;
           dirichlet_walls(VN, yn, ga);
           dirichlet_walls(VN, yn, gb);
 #pragma unroll
-          for (int k = 0; k < NPOP; k++) g[k] = make_float2(ga[k], gb[k]);
+          for (int k = 0; k < NPOP; k++) g[k] = pair_of(ga[k], gb[k]);
         }
         __syncwarp();
-        if (yn >= max(ya - off + 1, 0) && yn <= min(ya + Hc - 2 + off, ny - 1)) node_shift2(VN, f, g, F, r, u, v, t);
+        if (yn >= max(ya - off + 1, 0) && yn <= min(ya + Hc - 2 + off, ny - 1)) collide_pair(VN, f, g, F, r, u, v, t);
       }
     });
     const int pt = p0;

@@ -48,11 +48,11 @@ constexpr double CS2 = 1.0 / 3.0;
 inline bool off32_ok(size_t plane) { return plane * 2 * NPOP < (size_t(1) << 32); }
 
 // launch shapes of the two-step kernels (lb_kernels.cu): the tiles of
-// lb_pair_kernel (PAIR_SHAPES), then the marching lb_march_kernel
-// (MARCH_SHAPES)
+// lb_pair_kernel (PAIR_SHAPES), then the marching lb_wave2_kernel
+// (WAVE_SHAPES)
 constexpr int NUM_PAIR_TILES = 9;
 constexpr int NUM_PAIR_SHAPES = NUM_PAIR_TILES + 6;
-// launch shapes of the FP32 four-step kernel (QUAD_WAVES)
+// launch shapes of the four-step kernel (QUAD_WAVES)
 constexpr int NUM_QUAD_SHAPES = 3;
 // planes (of nx values) of a y-slab's ghost block for two steps per launch
 // (aux_kernels.cu: slab_pack2_kernel)
