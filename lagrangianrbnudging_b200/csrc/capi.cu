@@ -249,7 +249,7 @@ static void free_all(lbrb_t* h) {
   auto F = [](void* q) { if (q) cudaFree(q); };
   F(h->pops[0]); F(h->pops[1]); F(h->F[0]); F(h->F[1]);
   F(h->rho[0]); F(h->rho[1]); F(h->T[0]); F(h->T[1]);
-  for (int a = 0; a < 3; a++) for (int b = 0; b < 2; b++) F(h->uv[a][b]);
+  for (int a = 0; a < 3; a++) for (int b = 0; b < 2; b++) F(h->uv_own[a][b]);
   F(h->uv_extra);
   F(h->px); F(h->pid); F(h->ptype); F(h->d_ring);
   if (h->h_ring) cudaFreeHost(h->h_ring);
@@ -335,9 +335,13 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
   void** scal[] = {&h->F[0], &h->F[1], &h->rho[0], &h->rho[1], &h->T[0], &h->T[1],
                    &h->uv[0][0], &h->uv[0][1], &h->uv[1][0], &h->uv[1][1], &h->uv[2][0], &h->uv[2][1]};
   for (void** s : scal) {
-    if (cudaMalloc(s, h->plane * h->esize) != cudaSuccess) return done(LBRB_ERR_NOMEM);
+    if (cudaMalloc(s, h->plane * h->esize) != cudaSuccess) {
+      std::memcpy(h->uv_own, h->uv, sizeof h->uv_own);
+      return done(LBRB_ERR_NOMEM);
+    }
     cudaMemset(*s, 0, h->plane * h->esize);
   }
+  std::memcpy(h->uv_own, h->uv, sizeof h->uv_own);
   h->np = p.nprtcl;
   if (h->np > 0) {
     if (dalloc(&h->px, (size_t)9 * h->np) || dalloc(&h->pid, h->np) || dalloc(&h->ptype, h->np))
@@ -354,20 +358,18 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
           return done(LBRB_ERR_CUDA);
     }
   }
-  // the two extra u, v slots of four-step launches with particles, unless an
-  // earlier handle of this kind timed pairs as faster (lbrb_step); a run
-  // without memory for them steps in pairs
-  if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge == LBRB_NUDGE_NONE) {
-    int sh = 0;
-    float ms = 0.f;
+  // the extra u, v slots (lbrb_step: particles inside the next launch, and
+  // four-step launches); a run without memory for them steps in pairs, each
+  // followed by its particles
+  if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge != LBRB_NUDGE_REFBOX) {
+    constexpr int extra = UV_SLOTS - 3;
     const size_t pb1 = h->plane * h->esize;
-    if (!tuned_get(g_tuned_quad, h, &sh, &ms) || sh >= 0) {
-      if (cudaMalloc(&h->uv_extra, 4 * pb1) != cudaSuccess) {
-        cudaGetLastError();
-        h->uv_extra = nullptr;
-      } else {
-        for (int q = 0; q < 4; q++) h->uv[3 + q / 2][q % 2] = (char*)h->uv_extra + q * pb1;
-      }
+    if (cudaMalloc(&h->uv_extra, 2 * extra * pb1) != cudaSuccess) {
+      cudaGetLastError();
+      h->uv_extra = nullptr;
+    } else {
+      for (int q = 0; q < 2 * extra; q++) h->uv[3 + q / 2][q % 2] = (char*)h->uv_extra + q * pb1;
+      h->nuv = UV_SLOTS;
     }
   }
   h->nobs = p.nobs;
@@ -911,7 +913,115 @@ int lbrb_step(lbrb_t* h, int n) {
     if (h->p.obs_cycle) row %= h->obs_nsteps;
     return h->obs + (size_t)row * 3 * h->nobs;
   };
+  // ---- particles of the steps of a two- or four-step launch: `Group`, the
+  // steps istep0 .. istep0 + n - 1 with the u, v slots of each (and of the step
+  // before), the T of its record steps and their ring slots (-1: no record).
+  // With slots to spare (nuv) a pair's group waits (`pend`) and rides in the
+  // next tile launch of this call; `flush` gives it a launch of its own.
+  // Nothing is left pending when the call returns.
+  struct Group {
+    int n = 0, istep0 = 0, prev = 0;
+    int slot[4] = {}, rec[4] = {-1, -1, -1, -1};
+    const void* T[4] = {};
+  };
+  Group pend;
+  auto ride = [&]() {
+    return !h->timing && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES && h->quad_shape < 0;
+  };
+  auto rec_ptr = [&](int slot) -> double* {
+    return slot < 0 ? nullptr : h->d_ring + (size_t)slot * h->nrec_fields * h->np;
+  };
+  auto pend_recs = [&]() {
+    int k = 0;
+    for (int q = 0; q < pend.n; q++) k += pend.rec[q] >= 0;
+    return k;
+  };
+  auto group_copies = [&](const Group& g) -> int {
+    for (int q = 0; q < g.n; q++)
+      if (g.rec[q] >= 0) {
+        const int rc = record_copy(g.istep0 + q, g.rec[q], rec_ptr(g.rec[q]), h->stream);
+        if (rc) return rc;
+      }
+    return LBRB_OK;
+  };
+  auto group_fields = [&](const Group& g, const void* (&f)[4][5]) {
+    for (int q = 0; q < g.n; q++) {
+      const int b = q ? g.slot[q - 1] : g.prev;
+      for (int c = 0; c < 2; c++) f[q][c] = h->uv[g.slot[q]][c], f[q][2 + c] = h->uv[b][c];
+      f[q][4] = g.T[q];
+    }
+  };
+  auto group_launch = [&](const Group& g) -> int {
+    const void* f[4][5];
+    group_fields(g, f);
+    double* r[4] = {rec_ptr(g.rec[0]), rec_ptr(g.rec[1]), rec_ptr(g.rec[2]), rec_ptr(g.rec[3])};
+    const int tm = tmark_begin(h, 1, h->stream);
+    if (g.n == 4)
+      CK(h, launch_particles_quad(f, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full, r,
+                                  h->dflags, h->stream, pdl_ok));
+    else
+      CK(h, launch_particles_pair(f[0], f[1], f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta,
+                                  h->p.record_full, r[0], r[1], h->dflags, h->stream, pdl_ok));
+    tmark_end(h, tm, h->stream);
+    return group_copies(g);
+  };
+  auto flush = [&]() -> int {
+    if (!pend.n) return LBRB_OK;
+    const Group g = pend;
+    pend = Group{};
+    return group_launch(g);
+  };
+  auto group_job = [&](auto zero, const Group& g) {
+    using Real = decltype(zero);
+    PJob<Real> J{};
+    const void* f[4][5];
+    group_fields(g, f);
+    for (int q = 0; q < g.n; q++) {
+      double* r = rec_ptr(g.rec[q]);
+      J.V[q] = PView<Real>{(const Real*)f[q][0], (const Real*)f[q][1], (const Real*)f[q][2], (const Real*)f[q][3],
+                           (const Real*)f[q][4], nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, r ? 1 : 0,
+                           h->p.record_full, r, h->dflags};
+    }
+    J.nsteps = g.n;
+    return J;
+  };
+  // k slots for the steps of the next launch, none that the pending group
+  // reads; a pending group that leaves too few, or whose record T the launch
+  // would overwrite (t0, t1: the T buffers it stores to), goes first
+  auto take_slots = [&](int k, const void* t0, const void* t1, int* out) -> int {
+    bool hit = false;
+    for (int q = 0; q < pend.n; q++) hit = hit || (pend.rec[q] >= 0 && (pend.T[q] == t0 || pend.T[q] == t1));
+    if (pend.n && (hit || pend.n + 1 + k > h->nuv)) {
+      const int rc = flush();
+      if (rc) return rc;
+    }
+    unsigned busy = 1u << h->uvcur;
+    if (pend.n) busy |= 1u << pend.prev;
+    for (int q = 0; q < pend.n; q++) busy |= 1u << pend.slot[q];
+    for (int q = 0, at = 0; q < k; at++)
+      if (!(busy >> at & 1u)) out[q++] = at;
+    return LBRB_OK;
+  };
+  // uvcur and uvprev back among slots 0-2 (graphs of single steps hold slot
+  // pointers: captured again)
+  auto settle_slots = [&]() {
+    bool moved = false;
+    for (int* s : {&h->uvcur, &h->uvprev}) {
+      if (*s < 3) continue;
+      const int other = s == &h->uvcur ? h->uvprev : h->uvcur;
+      const int j = other == 0 ? 1 : 0;
+      std::swap(h->uv[*s][0], h->uv[j][0]);
+      std::swap(h->uv[*s][1], h->uv[j][1]);
+      *s = j;
+      moved = true;
+    }
+    if (!moved) return;
+    for (cudaGraphExec_t& g : h->graph_exec)
+      if (g) cudaGraphExecDestroy(g), g = nullptr;
+  };
   auto one = [&](bool last) -> int {
+    if (const int rc = flush()) return rc;
+    settle_slots();
     const int istep = h->istep + 1;
     const bool rec = h->np > 0 && h->p.noutconfig > 0 && istep % h->p.noutconfig == 0;
     if (rec && !h->slab && (h->rec_head - h->rec_tail) >= h->p.record_slots)
@@ -1006,14 +1116,18 @@ int lbrb_step(lbrb_t* h, int n) {
     const bool rec1 = parts && h->p.noutconfig > 0 && i1 % h->p.noutconfig == 0;
     const bool rec2 = parts && h->p.noutconfig > 0 && i2 % h->p.noutconfig == 0;
     const int src = h->cur, dst = h->cur ^ 1;
-    const int A = parts ? 3 - h->uvcur - h->uvprev : h->uvcur;  // u^n
-    // u^{n+1}: the slot of u^{n-2}; without particles only the call's last
-    // step stores u, v, in the free slot as one(true) would
-    const int B = parts ? h->uvprev : (last ? 3 - h->uvcur - h->uvprev : h->uvcur);
+    const bool nud = h->p.nudge == LBRB_NUDGE_BILINEAR;
+    // slots of u^n and u^{n+1}; without particles only the call's last step
+    // stores u, v, in the free slot as one(true) would
+    int ab[2] = {h->uvcur, last ? 3 - h->uvcur - h->uvprev : h->uvcur};
+    if (parts) {
+      const int rc = take_slots(2, rec1 || last ? h->T[src] : nullptr, rec2 || last || nud ? h->T[dst] : nullptr, ab);
+      if (rc) return rc;
+    }
+    const int A = ab[0], B = ab[1];
     const int wuv = parts ? 1 : 0;
     // bilinear nudging: step n's innovations before the launch (into acc2 and
     // the node mask, read inside it), step n+1's after it (T^{n+1} stored)
-    const bool nud = h->p.nudge == LBRB_NUDGE_BILINEAR;
     const double* o1 = nud ? obs_row(i1) : nullptr;
     const double* o2 = nud ? obs_row(i2) : nullptr;
     const size_t no = (size_t)h->nobs;
@@ -1035,15 +1149,17 @@ int lbrb_step(lbrb_t* h, int n) {
         V1.T = (float*)h->T[src];
         V1.rho = (float*)h->rho[src];
         with_sums(V1);
+        const PJob<float> J = group_job(0.f, pend);
         CK(h, launch_pair_fp32(V1, make_view<float>(h, dst, dst, B, wuv || last, rt2), h->pair_shape, h->stream,
-                               pdl_ok));
+                               pdl_ok, &J));
       } else {
         LBView<double> V1 = make_view<double>(h, src, dst, A, wuv, rec1 ? 1 : 0);
         V1.T = (double*)h->T[src];
         V1.rho = (double*)h->rho[src];
         with_sums(V1);
+        const PJob<double> J = group_job(0.0, pend);
         CK(h, launch_pair_fp64(V1, make_view<double>(h, dst, dst, B, wuv || last, rt2), h->pair_shape, h->stream,
-                               pdl_ok));
+                               pdl_ok, &J));
       }
       tmark_end(h, tm, h->stream);
     }
@@ -1057,27 +1173,22 @@ int lbrb_step(lbrb_t* h, int n) {
       tmark_end(h, tm, h->stream);
     }
     if (parts) {
-      // both steps of every particle in one launch; the ring slots in step order
+      // the pending group rode in the launch; this one's turn is next
+      const Group done = pend;
+      pend = Group{};
+      int rc = group_copies(done);
+      if (rc) return rc;
+      Group g;
+      g.n = 2;
+      g.istep0 = i1;
+      g.prev = h->uvcur;
+      g.slot[0] = A, g.slot[1] = B;
+      g.T[0] = h->T[src], g.T[1] = h->T[dst];
       long head = h->rec_head;
-      const int slot1 = rec1 ? (int)(head++ % h->p.record_slots) : 0;
-      const int slot2 = rec2 ? (int)(head % h->p.record_slots) : 0;
-      const size_t per = (size_t)h->nrec_fields * h->np;
-      double* r1 = rec1 ? h->d_ring + (size_t)slot1 * per : nullptr;
-      double* r2 = rec2 ? h->d_ring + (size_t)slot2 * per : nullptr;
-      const void* fa[5] = {h->uv[A][0], h->uv[A][1], h->uv[h->uvcur][0], h->uv[h->uvcur][1], h->T[src]};
-      const void* fb[5] = {h->uv[B][0], h->uv[B][1], h->uv[A][0], h->uv[A][1], h->T[dst]};
-      const int tm = tmark_begin(h, 1, h->stream);
-      CK(h, launch_particles_pair(fa, fb, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta,
-                                  h->p.record_full, r1, r2, h->dflags, h->stream, pdl_ok));
-      tmark_end(h, tm, h->stream);
-      if (rec1) {
-        const int rc = record_copy(i1, slot1, r1, h->stream);
-        if (rc) return rc;
-      }
-      if (rec2) {
-        const int rc = record_copy(i2, slot2, r2, h->stream);
-        if (rc) return rc;
-      }
+      if (rec1) g.rec[0] = (int)(head++ % h->p.record_slots);
+      if (rec2) g.rec[1] = (int)(head % h->p.record_slots);
+      if (ride()) pend = g;
+      else if ((rc = group_launch(g))) return rc;
       h->uvprev = A;
       h->uvcur = B;
     } else if (last) {
@@ -1119,16 +1230,13 @@ int lbrb_step(lbrb_t* h, int n) {
     }
     return LBRB_OK;
   };
-  // Four plain steps n .. n+3 in one launch (lb_wave4_kernel), then the
-  // particles of all four.  As `two`: u, v of n+2 and n+3 go to the slots two
-  // pairs would leave them in, those of n and n+1 to the extra slots; at most
-  // one of the steps is a record step, whose T goes to the source buffer, or
-  // for step n+3 to the destination's.  Never the call's last step.
-  auto quad_views = [&](auto zero, const bool* rec, auto& V) {
+  // Four plain steps n .. n+3 in one launch (lb_wave4_kernel).  At most one of
+  // the steps is a record step, whose T goes to the source buffer, or for step
+  // n+3 to the destination's.  Never the call's last step.
+  auto quad_views = [&](auto zero, const bool* rec, const int* slot, auto& V) {
     using Real = decltype(zero);
     const int src = h->cur, dst = h->cur ^ 1;
     const bool parts = h->np > 0;
-    const int slot[4] = {3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
     for (int q = 0; q < 4; q++) {
       V[q] = make_view<Real>(h, src, dst, parts ? slot[q] : h->uvcur, parts ? 1 : 0, rec[q] ? 1 : 0);
       if (q < 3) V[q].T = (Real*)h->T[src];
@@ -1136,40 +1244,38 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   auto four = [&]() -> int {
     const bool parts = h->np > 0;
+    const int src = h->cur, dst = h->cur ^ 1;
     bool rec[4];
     for (int q = 0; q < 4; q++) rec[q] = parts && h->p.noutconfig > 0 && (h->istep + 1 + q) % h->p.noutconfig == 0;
+    Group g;
+    if (parts) {
+      if (const int rc = flush()) return rc;
+      const int rc = take_slots(4, rec[0] || rec[1] || rec[2] ? h->T[src] : nullptr, rec[3] ? h->T[dst] : nullptr, g.slot);
+      if (rc) return rc;
+    }
     const int tm = tmark_begin(h, 0, h->stream);
     if (f32) {
       LBView<float> V[4];
-      quad_views(0.f, rec, V);
+      quad_views(0.f, rec, g.slot, V);
       CK(h, launch_quad_fp32(V, h->quad_shape, h->stream, pdl_ok));
     } else {
       LBView<double> V[4];
-      quad_views(0.0, rec, V);
+      quad_views(0.0, rec, g.slot, V);
       CK(h, launch_quad_fp64(V, h->quad_shape, h->stream, pdl_ok));
     }
     tmark_end(h, tm, h->stream);
     if (parts) {
-      const int slot[5] = {h->uvcur, 3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
-      const void* fields[4][5];
-      double* r[4] = {};
-      const int rslot = (int)(h->rec_head % h->p.record_slots);
+      int rc;
+      g.n = 4;
+      g.istep0 = h->istep + 1;
+      g.prev = h->uvcur;
       for (int q = 0; q < 4; q++) {
-        for (int c = 0; c < 2; c++) fields[q][c] = h->uv[slot[q + 1]][c], fields[q][2 + c] = h->uv[slot[q]][c];
-        fields[q][4] = h->T[q < 3 ? h->cur : h->cur ^ 1];
-        if (rec[q]) r[q] = h->d_ring + (size_t)rslot * h->nrec_fields * h->np;
+        g.T[q] = h->T[q < 3 ? src : dst];
+        if (rec[q]) g.rec[q] = (int)(h->rec_head % h->p.record_slots);
       }
-      const int tp = tmark_begin(h, 1, h->stream);
-      CK(h, launch_particles_quad(fields, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full,
-                                  r, h->dflags, h->stream, pdl_ok));
-      tmark_end(h, tp, h->stream);
-      for (int q = 0; q < 4; q++)
-        if (rec[q]) {
-          const int rc = record_copy(h->istep + 1 + q, rslot, r[q], h->stream);
-          if (rc) return rc;
-        }
-      h->uvprev = slot[3];
-      h->uvcur = slot[4];
+      if ((rc = group_launch(g))) return rc;
+      h->uvprev = g.slot[2];
+      h->uvcur = g.slot[3];
     }
     h->cur ^= 1;
     h->prev_valid = false;
@@ -1183,18 +1289,19 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   auto tune_quads = [&]() -> int {
     h->quad_shape = -1;
-    if (h->np > 0 && !h->uv_extra) return LBRB_OK;  // (no memory for the slots: pairs)
+    if (h->np > 0 && h->nuv < UV_SLOTS) return LBRB_OK;  // (no memory for the slots: pairs)
     float ms = 0.f;
     int sh = 0;
     if (!tuned_get(g_tuned_quad, h, &sh, &ms)) {
       const bool none[4] = {};
+      const int slot[4] = {3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
       if (f32) {
         LBView<float> V[4];
-        quad_views(0.f, none, V);
+        quad_views(0.f, none, slot, V);
         sh = tune_quad_fp32(V, h->stream, &ms);
       } else {
         LBView<double> V[4];
-        quad_views(0.0, none, V);
+        quad_views(0.0, none, slot, V);
         sh = tune_quad_fp64(V, h->stream, &ms);
       }
       CK(h, cudaGetLastError());
@@ -1285,7 +1392,7 @@ int lbrb_step(lbrb_t* h, int n) {
       int need = 0;
       for (int q = 1; q <= 4; q++)
         need += h->np > 0 && h->p.noutconfig > 0 && (h->istep + q) % h->p.noutconfig == 0;
-      if (need <= 1 && h->rec_head - h->rec_tail + need <= h->p.record_slots) {
+      if (need <= 1 && h->rec_head - h->rec_tail + pend_recs() + need <= h->p.record_slots) {
         const int rc = four();
         if (rc) return rc;
         s += 4;
@@ -1304,7 +1411,7 @@ int lbrb_step(lbrb_t* h, int n) {
       for (int q = 1; q <= 2; q++)
         need += h->np > 0 && h->p.noutconfig > 0 && (h->istep + q) % h->p.noutconfig == 0;
       const bool obs_ok = h->p.nudge != LBRB_NUDGE_BILINEAR || (obs_row(h->istep + 1) && obs_row(h->istep + 2));
-      if (h->rec_head - h->rec_tail + need <= h->p.record_slots && obs_ok) {
+      if (h->rec_head - h->rec_tail + pend_recs() + need <= h->p.record_slots && obs_ok) {
         const int rc = two(n - s == 2);
         if (rc) return rc;
         s += 2;
@@ -1315,6 +1422,8 @@ int lbrb_step(lbrb_t* h, int n) {
     if (rc) return rc;
     s++;
   }
+  if (const int rc = flush()) return rc;
+  settle_slots();
   // the caller's stream sees the record copies as part of the steps
   if (h->join_pending) {
     CK(h, cudaEventRecord(h->join_ev, h->copy_stream));

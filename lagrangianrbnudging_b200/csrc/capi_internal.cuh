@@ -9,6 +9,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "lbrb_internal.cuh"
+#include "particle_dev.cuh"
 #include "slab_parts.cuh"
 
 namespace lbrb {
@@ -27,9 +28,13 @@ int tune_lb_fp64(const LBView<double>& V, int twall, cudaStream_t s, float* best
 cudaError_t launch_pull_fp64(const LBView<double>& V, int twall, void* outf, void* outg, cudaStream_t s);
 cudaError_t launch_pull_fp32(const LBView<float>& V, int twall, void* outf, void* outg, cudaStream_t s);
 int tune_lb_fp32(const LBView<float>& V, int twall, cudaStream_t s, float* best_ms);
-// two steps per launch (Dirichlet walls, no ghost rows): V1 = step n, V2 = step n+1
-cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, int shape, cudaStream_t s, bool pdl);
-cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s, bool pdl);
+// two steps per launch (Dirichlet walls, no ghost rows): V1 = step n, V2 =
+// step n+1; job: particles of earlier steps advanced by the launch (tile
+// shapes only), or null
+cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, int shape, cudaStream_t s, bool pdl,
+                             const PJob<float>* job = nullptr);
+cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s, bool pdl,
+                             const PJob<double>* job = nullptr);
 int tune_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, cudaStream_t s, float* best_ms);
 int tune_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, cudaStream_t s, float* best_ms);
 // four steps per launch (as pairs; no nudging, no y-slab): one view per step

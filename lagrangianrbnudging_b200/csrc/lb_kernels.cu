@@ -36,6 +36,7 @@
 #include <type_traits>
 
 #include "lb_pair.cuh"
+#include "particle_dev.cuh"
 
 namespace lbrb {
 
@@ -69,11 +70,20 @@ __global__ void __launch_bounds__(BS, MINB) lb_node_kernel(const LBView<Real> V)
 // ------------------------------------------------------- two steps per launch
 // Temporal blocking of two steps n, n+1 in TX x TY tiles, one per block
 // (lb_pair.cuh: tile_block, the per-block work).
+// The first J.nblocks blocks advance particles (PJob; FP32 at 512x256 with 4096
+// tracers: 7.1 us per step with its records, 8.2 with particle launches of
+// their own).
 template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
-__global__ void __launch_bounds__(NT, MINB) lb_pair_kernel(const LBView<Real> V1, const LBView<Real> V2) {
+__global__ void __launch_bounds__(NT, MINB)
+    lb_pair_kernel(const LBView<Real> V1, const LBView<Real> V2, const __grid_constant__ PJob<Real> J, int tiles_x) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char pair_smem[];
-  tile_block<Real, TX, TY, NT, Off>(V1, V2, blockIdx.x * TX, blockIdx.y * TY, pair_smem);
+  const int b = blockIdx.x - J.nblocks;
+  if (b < 0) {
+    particle_job(J, blockIdx.x);
+    return;
+  }
+  tile_block<Real, TX, TY, NT, Off>(V1, V2, b % tiles_x * TX, b / tiles_x * TY, pair_smem);
 }
 
 // marching (lb_pair.cuh: wave_march): item = strip + chunk * nstrips, one per warp
@@ -122,17 +132,31 @@ constexpr PairShape PAIR_SHAPES[] = {{32, 8, 256, 4}, {32, 4, 128, 6}, {32, 16, 
 constexpr int NPAIR = sizeof(PAIR_SHAPES) / sizeof(PAIR_SHAPES[0]);
 static_assert(NPAIR <= NUM_PAIR_SHAPES, "pair shape table");
 
+// the caller's particles (or none) for blocks of nt threads
+template <typename Real>
+static PJob<Real> job_for(const PJob<Real>* job, int nt) {
+  PJob<Real> J{};
+  if (job && job->nsteps > 0) {
+    J = *job;
+    J.nblocks = (J.V[0].np + nt - 1) / nt;
+  }
+  return J;
+}
+
 template <typename Real, int TX, int TY, int NT, int MINB>
-static cudaError_t launch_pair_t(const LBView<Real>& V1, const LBView<Real>& V2, cudaStream_t s, bool pdl) {
+static cudaError_t launch_pair_t(const LBView<Real>& V1, const LBView<Real>& V2, cudaStream_t s, bool pdl,
+                                 const PJob<Real>* job) {
   constexpr size_t smem = tile_smem_bytes<Real, TX, TY>();
-  dim3 grid((V1.nx + TX - 1) / TX, (V1.ny + TY - 1) / TY);
+  const PJob<Real> J = job_for(job, NT);
+  const int tiles_x = (V1.nx + TX - 1) / TX;
+  const unsigned grid = (unsigned)(J.nblocks + (long)tiles_x * ((V1.ny + TY - 1) / TY));
   auto go = [&](auto kernel) -> cudaError_t {
     // the shared-memory limit is a per-device attribute of the kernel: set
     // once per device (one bit per device ordinal, per instantiation)
     static std::atomic<unsigned long long> attr_set{0};
     const cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
     if (e != cudaSuccess) return e;
-    return launch_k(kernel, grid, NT, smem, s, pdl, V1, V2);
+    return launch_k(kernel, grid, NT, smem, s, pdl, V1, V2, J, tiles_x);
   };
   // (FP64 holds twice the registers per value: half the blocks per SM)
   constexpr int MB = std::is_same<Real, double>::value ? (MINB + 1) / 2 : MINB;
@@ -227,18 +251,22 @@ cudaError_t launch_quad_fp64(const LBView<double> (&V)[4], int shape, cudaStream
 }
 
 template <typename Real>
-static cudaError_t launch_pair(const LBView<Real>& V1, const LBView<Real>& V2, int shape, cudaStream_t s, bool pdl) {
+static cudaError_t launch_pair(const LBView<Real>& V1, const LBView<Real>& V2, int shape, cudaStream_t s, bool pdl,
+                               const PJob<Real>* job = nullptr) {
+  // (no particles in the strips' launches: a strip's warps run for the whole
+  // launch, and particle blocks in their places cost more than they hide --
+  // 1500x701 with 20,000 inertial particles 12.7 against 11.9 ms per 301 steps)
   if (shape >= NPAIR) return launch_march(V1, V2, shape - NPAIR, s, pdl);
   switch (shape) {
-    case 1: return launch_pair_t<Real, 32, 4, 128, 6>(V1, V2, s, pdl);
-    case 2: return launch_pair_t<Real, 32, 16, 512, 2>(V1, V2, s, pdl);
-    case 3: return launch_pair_t<Real, 64, 4, 256, 3>(V1, V2, s, pdl);
-    case 4: return launch_pair_t<Real, 32, 8, 352, 2>(V1, V2, s, pdl);
-    case 5: return launch_pair_t<Real, 30, 8, 320, 3>(V1, V2, s, pdl);
-    case 6: return launch_pair_t<Real, 32, 8, 256, 5>(V1, V2, s, pdl);
-    case 7: return launch_pair_t<Real, 32, 6, 192, 5>(V1, V2, s, pdl);
-    case 8: return launch_pair_t<Real, 64, 8, 512, 2>(V1, V2, s, pdl);
-    default: return launch_pair_t<Real, 32, 8, 256, 4>(V1, V2, s, pdl);
+    case 1: return launch_pair_t<Real, 32, 4, 128, 6>(V1, V2, s, pdl, job);
+    case 2: return launch_pair_t<Real, 32, 16, 512, 2>(V1, V2, s, pdl, job);
+    case 3: return launch_pair_t<Real, 64, 4, 256, 3>(V1, V2, s, pdl, job);
+    case 4: return launch_pair_t<Real, 32, 8, 352, 2>(V1, V2, s, pdl, job);
+    case 5: return launch_pair_t<Real, 30, 8, 320, 3>(V1, V2, s, pdl, job);
+    case 6: return launch_pair_t<Real, 32, 8, 256, 5>(V1, V2, s, pdl, job);
+    case 7: return launch_pair_t<Real, 32, 6, 192, 5>(V1, V2, s, pdl, job);
+    case 8: return launch_pair_t<Real, 64, 8, 512, 2>(V1, V2, s, pdl, job);
+    default: return launch_pair_t<Real, 32, 8, 256, 4>(V1, V2, s, pdl, job);
   }
 }
 
@@ -366,12 +394,13 @@ int tune_lb_fp32(const LBView<float>& V, int twall, cudaStream_t s, float* best_
 
 // two steps per launch: V1 is step n (its pops and F outputs unused), V2 step
 // n+1 (its pop and F inputs unused)
-cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, int shape, cudaStream_t s, bool pdl) {
-  return launch_pair<float>(V1, V2, shape, s, pdl);
+cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, int shape, cudaStream_t s, bool pdl,
+                             const PJob<float>* job) {
+  return launch_pair<float>(V1, V2, shape, s, pdl, job);
 }
-cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s,
-                             bool pdl) {
-  return launch_pair<double>(V1, V2, shape, s, pdl);
+cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2, int shape, cudaStream_t s, bool pdl,
+                             const PJob<double>* job) {
+  return launch_pair<double>(V1, V2, shape, s, pdl, job);
 }
 
 // pair shape autotuner: as tune(), the trial launches write only buffers the

@@ -276,6 +276,11 @@ __device__ __forceinline__ Real nudge_increment(int k, double sv) {
   else return (float)(w_of(k) * sv);
 }
 
+// u, v slots of a run with particles: the three steps whose u, v the particles
+// of a pair read and the two that the launch beside them writes; or the step
+// before a four-step launch and its four
+constexpr int UV_SLOTS = 5;
+
 struct SlabParts;  // particles of a y-slab held by their owner slab (slab_parts.cuh)
 
 // --------------------------------------------------------------- handle
@@ -358,9 +363,14 @@ struct Handle {
   // particle kernel of step n can run beside the fused kernel of step n+1
   void* rho[2] = {nullptr, nullptr};
   void* T[2] = {nullptr, nullptr};
-  // (slots 3 and 4, in uv_extra: u^n, u^{n+1} inside a four-step launch with particles)
-  void* uv[5][2] = {};
+  // nuv slots in all: three between calls (uvcur, uvprev and a free one are
+  // slots 0-2); the others, in uv_extra, hold steps of a four-step launch and
+  // steps whose particles the next launch advances.  lbrb_step may exchange
+  // slots' pointers; uv_own are those that free_all releases.
+  void* uv[UV_SLOTS][2] = {};
+  void* uv_own[3][2] = {};
   void* uv_extra = nullptr;
+  int nuv = 3;
   int uvcur = 0, uvprev = 1;
   // second stream: the adjoint window's segment recompute (events order it
   // against `stream`)

@@ -209,5 +209,22 @@ __device__ __forceinline__ void particle_update(const PView<Real>& V, int p) {
   X[7 * n + p] = vold;
 }
 
+// Particles of the steps before, advanced inside a fused launch by its first
+// nblocks blocks: nsteps (2 or 4) steps whose u, v (and T) are complete, in
+// slots that the launch does not write.  A particle launch of its own is a
+// chain of dependent gathers (6-7 us for two steps however few the
+// particles); beside the fused step it costs almost nothing.
+template <typename Real>
+struct PJob {
+  PView<Real> V[4];
+  int nsteps, nblocks;
+};
+template <typename Real>
+__device__ __noinline__ void particle_job(const PJob<Real>& J, int block) {
+  const int p = block * blockDim.x + threadIdx.x;
+  if (p >= J.V[0].np) return;
+#pragma unroll 1
+  for (int q = 0; q < J.nsteps; q++) particle_update<Real, true>(J.V[q], p);
+}
 
 }  // namespace lbrb
