@@ -11,6 +11,8 @@
 //  * a NaN/Inf scan of the populations.
 #include <type_traits>
 
+#include <algorithm>
+
 #include "lbrb_internal.cuh"
 
 namespace lbrb {
@@ -276,6 +278,41 @@ struct KSum {
 constexpr int RED_BLOCKS = 1184;  // 8 per SM on 148 SMs
 constexpr int RED_Q = 3;          // ke, T, vT
 
+// compensated sums over a block, by halving: warps by shuffles, then the warps'
+// results in the first warp; thread 0 has the block's sums.  (Three threads
+// folding 512 values one after another took 12 us of a 17 us launch.)
+__device__ __forceinline__ void ksum_merge(KSum& a, double s, double c) {
+  a.add(s);
+  a.add(c);
+}
+__device__ __forceinline__ void ksum_block(KSum (&a)[RED_Q]) {
+  __shared__ double sh[RED_Q][2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int q = 0; q < RED_Q; q++) {
+      const double s = __shfl_down_sync(0xffffffffu, a[q].s, off), c = __shfl_down_sync(0xffffffffu, a[q].c, off);
+      ksum_merge(a[q], s, c);
+    }
+  if (lane == 0)
+    for (int q = 0; q < RED_Q; q++) sh[q][0][warp] = a[q].s, sh[q][1][warp] = a[q].c;
+  __syncthreads();
+  if (warp == 0) {
+    for (int q = 0; q < RED_Q; q++) {
+      a[q].s = lane < 8 ? sh[q][0][lane] : 0.0;
+      a[q].c = lane < 8 ? sh[q][1][lane] : 0.0;
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+      for (int q = 0; q < RED_Q; q++) {
+        const double s = __shfl_down_sync(0xffffffffu, a[q].s, off), c = __shfl_down_sync(0xffffffffu, a[q].c, off);
+        ksum_merge(a[q], s, c);
+      }
+  }
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(256) stats_partial_kernel(const Real* __restrict__ rho,
                                                             const Real* __restrict__ u,
@@ -283,57 +320,38 @@ __global__ void __launch_bounds__(256) stats_partial_kernel(const Real* __restri
                                                             const Real* __restrict__ T, int nx,
                                                             int ny, int pitch,
                                                             double* __restrict__ part) {
+  pdl_wait();
   KSum a[RED_Q];
-  const long n = (long)nx * ny;
-  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(q % nx), j = (int)(q / nx);
+  // a warp takes 32-column pieces of rows, in order
+  const int ncx = (nx + 31) / 32;
+  const long pieces = (long)ncx * ny;
+  for (long w = blockIdx.x * 8L + (threadIdx.x >> 5); w < pieces; w += 8L * gridDim.x) {
+    const int i = (int)(w % ncx) * 32 + (threadIdx.x & 31), j = (int)(w / ncx);
+    if (i >= nx) continue;
     const size_t o = (size_t)j * pitch + i;
     const double r = rho[o], uu = u[o], vv = v[o], t = T[o];
     a[0].add(0.5 * r * (uu * uu + vv * vv));
     a[1].add(t);
     a[2].add(vv * t);
   }
-  __shared__ double sh[RED_Q][2][256];
-  for (int w = 0; w < RED_Q; w++) {
-    sh[w][0][threadIdx.x] = a[w].s;
-    sh[w][1][threadIdx.x] = a[w].c;
-  }
-  __syncthreads();
-  if (threadIdx.x < RED_Q) {
-    KSum b;
-    for (int t = 0; t < 256; t++) {
-      b.add(sh[threadIdx.x][0][t]);
-      b.add(sh[threadIdx.x][1][t]);
+  ksum_block(a);
+  if (threadIdx.x == 0)
+    for (int q = 0; q < RED_Q; q++) {
+      part[(size_t)blockIdx.x * 2 * RED_Q + 2 * q] = a[q].s;
+      part[(size_t)blockIdx.x * 2 * RED_Q + 2 * q + 1] = a[q].c;
     }
-    part[(size_t)blockIdx.x * 2 * RED_Q + 2 * threadIdx.x] = b.s;
-    part[(size_t)blockIdx.x * 2 * RED_Q + 2 * threadIdx.x + 1] = b.c;
-  }
 }
 
-// one block: every thread folds a strided share of the block partials, then
-// thread 0 folds the per-thread results (all compensated)
+// one block folds the blocks' partials (out: device or pinned host memory)
 __global__ void __launch_bounds__(256) stats_final_kernel(const double* __restrict__ part,
                                                           int nblocks, double* __restrict__ out) {
-  __shared__ double sh[RED_Q][2][256];
+  pdl_wait();
   KSum a[RED_Q];
   for (int k = threadIdx.x; k < nblocks; k += blockDim.x)
-    for (int q = 0; q < RED_Q; q++) {
-      a[q].add(part[(size_t)k * 2 * RED_Q + 2 * q]);
-      a[q].add(part[(size_t)k * 2 * RED_Q + 2 * q + 1]);
-    }
-  for (int q = 0; q < RED_Q; q++) {
-    sh[q][0][threadIdx.x] = a[q].s;
-    sh[q][1][threadIdx.x] = a[q].c;
-  }
-  __syncthreads();
-  if (threadIdx.x < RED_Q) {
-    KSum b;
-    for (int t = 0; t < (int)blockDim.x; t++) {
-      b.add(sh[threadIdx.x][0][t]);
-      b.add(sh[threadIdx.x][1][t]);
-    }
-    out[threadIdx.x] = b.val();
-  }
+    for (int q = 0; q < RED_Q; q++) ksum_merge(a[q], part[(size_t)k * 2 * RED_Q + 2 * q], part[(size_t)k * 2 * RED_Q + 2 * q + 1]);
+  ksum_block(a);
+  if (threadIdx.x == 0)
+    for (int q = 0; q < RED_Q; q++) out[q] = a[q].val();
 }
 
 // per-row sums, one block per row
@@ -553,16 +571,18 @@ int red_blocks() { return RED_BLOCKS; }
 
 cudaError_t launch_stats(const void* rho, const void* u, const void* v, const void* T, bool fp32,
                          int nx, int ny, int pitch, double* part, double* out, cudaStream_t s) {
+  // (a warp takes at least one 32-column piece of a row)
+  const long pieces = (long)((nx + 31) / 32) * ny;
+  const int blocks = (int)std::min((long)RED_BLOCKS, (pieces + 7) / 8);
+  cudaError_t e;
   if (fp32)
-    stats_partial_kernel<float><<<RED_BLOCKS, 256, 0, s>>>((const float*)rho, (const float*)u,
-                                                           (const float*)v, (const float*)T, nx, ny,
-                                                           pitch, part);
+    e = launch_k(stats_partial_kernel<float>, blocks, 256, 0, s, true, (const float*)rho, (const float*)u,
+                 (const float*)v, (const float*)T, nx, ny, pitch, part);
   else
-    stats_partial_kernel<double><<<RED_BLOCKS, 256, 0, s>>>((const double*)rho, (const double*)u,
-                                                            (const double*)v, (const double*)T, nx,
-                                                            ny, pitch, part);
-  stats_final_kernel<<<1, 256, 0, s>>>(part, RED_BLOCKS, out);
-  return cudaGetLastError();
+    e = launch_k(stats_partial_kernel<double>, blocks, 256, 0, s, true, (const double*)rho, (const double*)u,
+                 (const double*)v, (const double*)T, nx, ny, pitch, part);
+  if (e != cudaSuccess) return e;
+  return launch_k(stats_final_kernel, 1, 256, 0, s, true, (const double*)part, blocks, out);
 }
 
 cudaError_t launch_profile(const void* rho, const void* u, const void* v, const void* T, bool fp32,

@@ -446,7 +446,7 @@ struct Handle {
   double* red = nullptr;    // reduction partials
   unsigned* dflags = nullptr;
   unsigned* h_flags = nullptr;
-  double* h_scalar = nullptr;  // pinned: one device scalar read back (the misfit)
+  double* h_scalar = nullptr;  // pinned: device scalars read back (the misfit; the three diagnostics sums)
 };
 
 }  // namespace lbrb
