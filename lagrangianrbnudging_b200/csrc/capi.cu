@@ -260,7 +260,7 @@ static void free_all(lbrb_t* h) {
     delete[] h->ring_ev;
   }
   F(h->nb); F(h->nbi); F(h->nudge_vol); F(h->tempreadint); F(h->nud_term); F(h->tsum0);
-  F(h->cell_count); F(h->cell_start); F(h->cell_fill); F(h->cell_dirty); F(h->cell_items);
+  F(h->box_work);
   delete[] h->h_chk; delete[] h->h_oid;
   F(h->obs); F(h->acc); F(h->acc2); F(h->nmask); F(h->staging); F(h->big); F(h->red); F(h->dflags);
   F(h->adj_obs); F(h->adj_res); F(h->adj_chk); F(h->adj_seg); F(h->adj_lam); F(h->adj_lT); F(h->adj_T0);
@@ -381,9 +381,8 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
     const size_t nc = (size_t)h->ncx * h->ncy;
     if (dalloc(&h->nb, (size_t)NB_COUNT * n) || dalloc(&h->nbi, (size_t)NBI_COUNT * n) ||
         dalloc(&h->nudge_vol, h->plane) || dalloc(&h->tempreadint, h->plane) ||
-        dalloc(&h->nud_term, h->plane) || dalloc(&h->tsum0, (size_t)h->pitch) || dalloc(&h->cell_count, nc) ||
-        dalloc(&h->cell_start, nc) || dalloc(&h->cell_fill, nc) || dalloc(&h->cell_dirty, nc) ||
-        dalloc(&h->cell_items, (size_t)2 * 12 * n))
+        dalloc(&h->nud_term, h->plane) || dalloc(&h->tsum0, (size_t)h->pitch) ||
+        dalloc(&h->box_work, box_cell_ints(n, (int)nc)))
       return done(LBRB_ERR_NOMEM);
     h->h_chk = new int[n]();
     h->h_oid = new int[n]();
@@ -872,7 +871,10 @@ int lbrb_step(lbrb_t* h, int n) {
   if (h->lb_shape < 0) {
     // autotune the fused kernel's launch shape on this grid (trial launches
     // write only the buffers the real step overwrites)
-    int sh = h->p.launch_shape;
+    // (box-nudged steps update nud_term in place and are not tuned: 128
+    // threads, 4 blocks per SM was the fastest on 1680x840 -- 9.4 ms per 100
+    // steps, 10.2 with 256 threads -- and ties on 512x256)
+    int sh = refbox && h->p.autotune ? 3 : h->p.launch_shape;
     float ms = 0.f;
     if (h->p.autotune && !refbox && !tuned_get(g_tuned_single, h, &sh, &ms)) {
       // trials store u, v as the steps will (particles need them every step),
@@ -1038,10 +1040,8 @@ int lbrb_step(lbrb_t* h, int n) {
         return fail(h, LBRB_ERR_STATE, "step: observation file for this interval not loaded");
       const int tm = tmark_begin(h, 2, h->stream);
       CK(h, launch_box_nudge(h->nb, h->nbi, h->nobs, nx, ny, h->slab ? h->slab_ny_total : ny, h->slab ? h->slab_j0 : 0,
-                             nt, istep, h->ncx, h->ncy,
-                             h->cell_count, h->cell_start, h->cell_fill, h->cell_dirty,
-                             h->cell_items, h->nudge_vol, h->tempreadint, h->pitch, h->dflags,
-                             h->stream));
+                             nt, istep, h->ncx, h->ncy, h->box_work, ++h->box_seq, h->nudge_vol, h->tempreadint,
+                             h->pitch, h->stream, pdl_ok));
       tmark_end(h, tm, h->stream);
       if (istep % nt == 1) h->nudge_file_loaded = false;
     }

@@ -13,12 +13,19 @@
 //   contributions are binned into 8x8-node cells, each cell sorts its
 //   contribution keys (3k + image), and each node walks its cell's sorted
 //   list.  Only cells that hold contributions, or held some the step before,
-//   touch memory.
+//   touch memory: two launches a step, one that advances the observations and
+//   bins them into a few places per cell (and lists the cells it touches),
+//   one over the listed cells of this step and the last.  (1680x840, 1600
+//   observations: the box launches take 14 us of a step; with a count, a
+//   one-block scan of all cells, a fill and a block for every cell they took
+//   45, the scan alone 17.)
 // Bilinear mode (no reference counterpart): innovation
 //   d = alpha (T_obs - T(x_obs)) spread to the 4 cell corners with bilinear
 //   weights; contributions are summed in 2^-40 fixed point with integer
 //   atomics, so the result does not depend on their order, then added to the
 //   post-collision g as w_k * S.
+#include <algorithm>
+
 #include "lbrb_internal.cuh"
 #include "nudge_dev.cuh"
 
@@ -32,6 +39,13 @@ enum { NB_OX = 0, NB_OY, NB_OT, NB_FX, NB_FY, NB_FT, NB_XINT, NB_YINT, NB_TINT, 
 // per-observation int arrays in Handle::nbi
 enum { NBI_CHK = 0, NBI_BC, NBI_XIDX, NBI_YIDX, NBI_COUNT };
 
+// Contributions of a cell: the first BOX_SLOTS in the cell's own slots, the
+// rest in one list of (cell, key) for all cells.  A step's lists and counters
+// are one of three sets, by `seq` (a count of steps, from 1): this step's, the
+// last one's, and the one that this step leaves cleared for the next.
+constexpr int BOX_SLOTS = 8;
+enum { BOX_NCELLS = 0, BOX_NOVER, BOX_NSORT, BOX_NCOUNT };
+
 struct BoxView {
   double* nb;
   int* nbi;
@@ -39,26 +53,25 @@ struct BoxView {
   // the whole domain's rows (positions and boxes); j0: the handle's first
   // row in the domain (0 unless a y-slab)
   int n, nx, ny, nt, istep, nyT, j0;
-  int ncx, ncy;
-  int* cell_count;
-  int* cell_start;
-  int* cell_fill;
-  int* cell_dirty;
-  int* items;
-  int* sorted;
+  int ncx, ncell, seq;
+  int* cnt;      // [3][BOX_NCOUNT]
+  int* count;    // [ncell] contributions of a cell this step (0 between steps)
+  int* stamp;    // [ncell] the last step that touched a cell
+  int* slots;    // [ncell][BOX_SLOTS]
+  int* cells;    // [3][lcap] cells touched
+  int2* over;    // [12 n] (cell, key)
+  int* scratch;  // [2][12 n]
+  int lcap;
   int* nudge_vol;
   double* tempreadint;
   int pitch;
-  unsigned* dflags;
 };
 
 __device__ __forceinline__ double* NB(const BoxView& B, int a) { return B.nb + (size_t)a * B.n; }
 __device__ __forceinline__ int* NBI(const BoxView& B, int a) { return B.nbi + (size_t)a * B.n; }
 
-// time interpolation, one thread per observation (read_prtcl's three branches)
-__global__ void box_interp_kernel(const BoxView B) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B.n) return;
+// time interpolation of observation i (read_prtcl's three branches)
+__device__ __forceinline__ void box_interp(const BoxView& B, int i) {
   const int nx = B.nx, ny = B.nyT, nt = B.nt;
   double *ox = NB(B, NB_OX), *oy = NB(B, NB_OY), *oT = NB(B, NB_OT);
   double *fx = NB(B, NB_FX), *fy = NB(B, NB_FY), *fT = NB(B, NB_FT);
@@ -109,6 +122,10 @@ __global__ void box_interp_kernel(const BoxView B) {
     if (bci == 2) { Tnow = fT[c]; bci = 1; }
     Tint[i] = Tnow;
     bc[i] = bci;
+    // the loaded file becomes the "last file" (read by the other branches only)
+    ox[i] = fx[i];
+    oy[i] = fy[i];
+    oT[i] = fT[i];
   } else if (ph == 0) {
     const int c = chk[i];
     xint[i] = ox[c];
@@ -136,15 +153,6 @@ __global__ void box_interp_kernel(const BoxView B) {
   }
 }
 
-// after the file branch: the loaded file becomes the "last file"
-__global__ void box_commit_file_kernel(const BoxView B) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B.n) return;
-  NB(B, NB_OX)[i] = NB(B, NB_FX)[i];
-  NB(B, NB_OY)[i] = NB(B, NB_FY)[i];
-  NB(B, NB_OT)[i] = NB(B, NB_FT)[i];
-}
-
 // node box of contribution (k, img), reference 1-based node coordinates of
 // the whole domain, clipped to its interior; false when empty.  img 0: main 7x7 box; img 1:
 // left periodic image (xidx < 4); img 2: right periodic image (xidx > nx-2).
@@ -168,113 +176,146 @@ __device__ __forceinline__ bool contrib_box(const BoxView& B, int k, int img, in
   return xa <= xb && ya <= yb;
 }
 
-template <bool FILL>
-__global__ void box_bin_kernel(const BoxView B) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * B.n) return;
-  const int k = t / 3, img = t - 3 * k;
-  int xa, xb, ya, yb;
-  if (!contrib_box(B, k, img, xa, xb, ya, yb)) return;
-  // the rows of this handle (a y-slab bins only what reaches its rows)
-  ya = max(ya, B.j0 + 1);
-  yb = min(yb, B.j0 + B.ny);
-  if (ya > yb) return;
-  const int ca = (xa - 1) / CELL, cb = (xb - 1) / CELL;
-  const int ra = (ya - 1 - B.j0) / CELL, rb = (yb - 1 - B.j0) / CELL;
-  for (int cy = ra; cy <= rb; cy++)
-    for (int cx = ca; cx <= cb; cx++) {
-      const int c = cy * B.ncx + cx;
-      if (FILL) {
-        const int slot = atomicAdd(&B.cell_fill[c], 1);
-        B.items[B.cell_start[c] + slot] = t;
-      } else {
-        atomicAdd(&B.cell_count[c], 1);
-      }
-    }
-}
-
-// exclusive scan of cell_count into cell_start: one block
-__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ in, int* __restrict__ out,
-                                                    int n) {
-  __shared__ int part[1024];
-  const int tid = threadIdx.x;
-  const int per = (n + 1023) / 1024;
-  const int a = tid * per, b = min(n, a + per);
-  int s = 0;
-  for (int q = a; q < b; q++) s += in[q];
-  part[tid] = s;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    int v = tid >= off ? part[tid - off] : 0;
-    __syncthreads();
-    part[tid] += v;
-    __syncthreads();
-  }
-  int run = part[tid] - s;
-  for (int q = a; q < b; q++) {
-    out[q] = run;
-    run += in[q];
-  }
-}
-
-// one block of CELL*CELL threads per cell: sort the cell's keys, then every
-// node applies the running mean in key order
-__global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B) {
-  const int c = blockIdx.x;
-  const int cnt = B.cell_count[c];
-  const int dirty = B.cell_dirty[c];
-  if (cnt == 0 && !dirty) return;
-  const int cx = c % B.ncx, cy = c / B.ncx;
-  const int tid = threadIdx.x;
-  const int i = cx * CELL + (tid % CELL) + 1;  // reference node coordinates (of the domain)
-  const int j = B.j0 + cy * CELL + (tid / CELL) + 1;
-  const int st = B.cell_start[c];
-  // rank sort (keys are unique)
-  for (int a = tid; a < cnt; a += blockDim.x) {
-    const int key = B.items[st + a];
-    int rank = 0;
-    for (int b = 0; b < cnt; b++) rank += (B.items[st + b] < key);
-    B.sorted[st + rank] = key;
-  }
-  __syncthreads();
-  int nv = 0;
-  double tri = 0.0;
-  const double* Tint = NB(B, NB_TINT);
-  for (int a = 0; a < cnt; a++) {
-    const int key = B.sorted[st + a];
-    const int k = key / 3, img = key - 3 * k;
+// one thread per observation: its new position and temperature, then its
+// contributions into the cells they reach
+__global__ void __launch_bounds__(32) box_bin_kernel(const BoxView B) {
+  pdl_wait();
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= B.n) return;
+  box_interp(B, k);
+  const int set = B.seq % 3;
+  int* cnt = B.cnt + set * BOX_NCOUNT;
+  for (int img = 0; img < 3; img++) {
     int xa, xb, ya, yb;
     if (!contrib_box(B, k, img, xa, xb, ya, yb)) continue;
-    if (i >= xa && i <= xb && j >= ya && j <= yb) {
-      tri = (tri * (double)nv + Tint[k]) / ((double)nv + 1.0);
-      nv = nv + 1;
-    }
+    // the rows of this handle (a y-slab bins only what reaches its rows)
+    ya = max(ya, B.j0 + 1);
+    yb = min(yb, B.j0 + B.ny);
+    if (ya > yb) continue;
+    const int ca = (xa - 1) / CELL, cb = (xb - 1) / CELL;
+    const int ra = (ya - 1 - B.j0) / CELL, rb = (yb - 1 - B.j0) / CELL;
+    for (int cy = ra; cy <= rb; cy++)
+      for (int cx = ca; cx <= cb; cx++) {
+        const int c = cy * B.ncx + cx, key = 3 * k + img;
+        const int at = atomicAdd(&B.count[c], 1);
+        if (at == 0) {
+          B.stamp[c] = B.seq;
+          B.cells[(size_t)set * B.lcap + atomicAdd(&cnt[BOX_NCELLS], 1)] = c;
+        }
+        if (at < BOX_SLOTS) B.slots[(size_t)c * BOX_SLOTS + at] = key;
+        else B.over[atomicAdd(&cnt[BOX_NOVER], 1)] = make_int2(c, key);
+      }
   }
-  if (i <= B.nx && j <= B.j0 + B.ny) {
-    const size_t q = (size_t)(j - 1 - B.j0) * B.pitch + (i - 1);
-    B.nudge_vol[q] = nv;
-    B.tempreadint[q] = tri;
-  }
-  if (tid == 0) B.cell_dirty[c] = cnt > 0;
 }
 
+// one block of CELL*CELL threads per listed cell: sort the cell's keys, then
+// every node applies the running mean in key order; cells of the last step
+// that this one did not touch are cleared
+__global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B) {
+  pdl_wait();
+  constexpr int NT = CELL * CELL;
+  __shared__ int keys[BOX_SLOTS];
+  __shared__ int sh[2];
+  const int tid = threadIdx.x;
+  const int set = B.seq % 3, last = (B.seq + 2) % 3, next = (B.seq + 1) % 3;
+  const int ncur = B.cnt[set * BOX_NCOUNT + BOX_NCELLS], nlast = B.cnt[last * BOX_NCOUNT + BOX_NCELLS];
+  if (blockIdx.x == 0 && tid < BOX_NCOUNT) B.cnt[next * BOX_NCOUNT + tid] = 0;
+  const double* Tint = NB(B, NB_TINT);
+  for (int it = blockIdx.x; it < ncur + nlast; it += gridDim.x) {
+    const bool now = it < ncur;
+    const int c = now ? B.cells[(size_t)set * B.lcap + it] : B.cells[(size_t)last * B.lcap + it - ncur];
+    if (!now && B.stamp[c] == B.seq) continue;  // (listed in this step too)
+    const int cx = c % B.ncx, cy = c / B.ncx;
+    const int i = cx * CELL + (tid % CELL) + 1;  // reference node coordinates (of the domain)
+    const int j = B.j0 + cy * CELL + (tid / CELL) + 1;
+    int nv = 0;
+    double tri = 0.0;
+    if (now) {
+      const int cnt = B.count[c];
+      const int* list = keys;
+      if (cnt <= BOX_SLOTS) {
+        // rank sort (keys are unique)
+        if (tid < cnt) {
+          const int key = B.slots[(size_t)c * BOX_SLOTS + tid];
+          int rank = 0;
+          for (int b = 0; b < cnt; b++) rank += (B.slots[(size_t)c * BOX_SLOTS + b] < key);
+          keys[rank] = key;
+        }
+        __syncthreads();
+      } else {
+        // more than the slots hold: the cell's keys into scratch, then ranked there
+        if (tid == 0) {
+          sh[0] = atomicAdd(&B.cnt[set * BOX_NCOUNT + BOX_NSORT], cnt);
+          sh[1] = BOX_SLOTS;
+        }
+        __syncthreads();
+        int* raw = B.scratch + sh[0];
+        int* sorted = raw + (size_t)12 * B.n;
+        for (int a = tid; a < BOX_SLOTS; a += NT) raw[a] = B.slots[(size_t)c * BOX_SLOTS + a];
+        const int nover = B.cnt[set * BOX_NCOUNT + BOX_NOVER];
+        for (int a = tid; a < nover; a += NT)
+          if (B.over[a].x == c) raw[atomicAdd(&sh[1], 1)] = B.over[a].y;
+        __syncthreads();
+        for (int a = tid; a < cnt; a += NT) {
+          const int key = raw[a];
+          int rank = 0;
+          for (int b = 0; b < cnt; b++) rank += (raw[b] < key);
+          sorted[rank] = key;
+        }
+        __syncthreads();
+        list = sorted;
+      }
+      for (int a = 0; a < cnt; a++) {
+        const int key = list[a];
+        const int k = key / 3, img = key - 3 * k;
+        int xa, xb, ya, yb;
+        if (!contrib_box(B, k, img, xa, xb, ya, yb)) continue;
+        if (i >= xa && i <= xb && j >= ya && j <= yb) {
+          tri = (tri * (double)nv + Tint[k]) / ((double)nv + 1.0);
+          nv = nv + 1;
+        }
+      }
+      __syncthreads();  // (every thread has the count and the keys)
+      if (tid == 0) B.count[c] = 0;
+    }
+    if (i <= B.nx && j <= B.j0 + B.ny) {
+      const size_t q = (size_t)(j - 1 - B.j0) * B.pitch + (i - 1);
+      B.nudge_vol[q] = nv;
+      B.tempreadint[q] = tri;
+    }
+  }
+}
+
+// ints of the cell lists for n observations over ncell cells: counters,
+// counts, stamps, slots, three lists, the overflow list, scratch
+static size_t box_lcap(int n, int ncell) { return std::min((size_t)ncell, (size_t)12 * n); }
+size_t box_cell_ints(int n, int ncell) {
+  return 16 + (size_t)ncell * (2 + BOX_SLOTS) + 3 * box_lcap(n, ncell) + (size_t)4 * 12 * n;
+}
+
+// `work`: box_cell_ints ints, zero at the start of the run; seq: 1, 2, ... from call to call
 cudaError_t launch_box_nudge(double* nb, int* nbi, int n, int nx, int ny, int ny_total, int j0, int nt, int istep,
-                             int ncx, int ncy, int* cell_count, int* cell_start, int* cell_fill,
-                             int* cell_dirty, int* items, int* nudge_vol, double* tempreadint,
-                             int pitch, unsigned* dflags, cudaStream_t s) {
+                             int ncx, int ncy, int* work, int seq, int* nudge_vol, double* tempreadint, int pitch,
+                             cudaStream_t s, bool pdl) {
   const int ncell = ncx * ncy;
-  BoxView B{nb, nbi, n, nx, ny, nt, istep, ny_total, j0, ncx, ncy, cell_count, cell_start, cell_fill,
-            cell_dirty, items, items + (size_t)n * 3 * 4, nudge_vol, tempreadint, pitch, dflags};
-  const int tb = 128;
-  box_interp_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(B);
-  if (istep % nt == 1) box_commit_file_kernel<<<(n + tb - 1) / tb, tb, 0, s>>>(B);
-  cudaMemsetAsync(cell_count, 0, sizeof(int) * ncell, s);
-  cudaMemsetAsync(cell_fill, 0, sizeof(int) * ncell, s);
-  box_bin_kernel<false><<<(3 * n + tb - 1) / tb, tb, 0, s>>>(B);
-  scan_kernel<<<1, 1024, 0, s>>>(cell_count, cell_start, ncell);
-  box_bin_kernel<true><<<(3 * n + tb - 1) / tb, tb, 0, s>>>(B);
-  box_cells_kernel<<<ncell, CELL * CELL, 0, s>>>(B);
-  return cudaGetLastError();
+  const size_t lcap = box_lcap(n, ncell);
+  BoxView B{nb, nbi, n, nx, ny, nt, istep, ny_total, j0, ncx, ncell, seq};
+  B.cnt = work;
+  B.over = reinterpret_cast<int2*>(work + 16);
+  B.scratch = work + 16 + (size_t)2 * 12 * n;
+  B.count = B.scratch + (size_t)2 * 12 * n;
+  B.stamp = B.count + ncell;
+  B.slots = B.stamp + ncell;
+  B.cells = B.slots + (size_t)ncell * BOX_SLOTS;
+  B.lcap = (int)lcap;
+  B.nudge_vol = nudge_vol;
+  B.tempreadint = tempreadint;
+  B.pitch = pitch;
+  // (32 threads a block: a few thousand observations still reach most SMs)
+  const cudaError_t e = launch_k(box_bin_kernel, (n + 31) / 32, 32, 0, s, pdl, B);
+  if (e != cudaSuccess) return e;
+  const int blocks = (int)std::min((size_t)2 * lcap, (size_t)148 * 16);
+  return launch_k(box_cells_kernel, blocks, CELL * CELL, 0, s, pdl, B);
 }
 
 // ------------------------------------------------------------ bilinear mode
