@@ -928,8 +928,16 @@ int lbrb_step(lbrb_t* h, int n) {
     const void* T[4] = {};
   };
   Group pend;
+  // Riding pays while the particles are few beside the nodes: FP32 at 864x372,
+  // per step, 8.6 us against 9.3 with launches of their own for one particle
+  // per 8 nodes, 11.1 against 10.3 for one per 4 (512x256, one per 32: 3.9
+  // against 5.4).  With the Maxey-Riley stencil it pays in FP64 (512x256: 9.1
+  // against 10.8) but not in FP32 (9.9 against 8.7), whose tile launches
+  // leave too few registers for it.
+  const bool stencil = h->p.beta != 0.0 || h->p.record_full;
+  const bool few = 8L * h->np <= (long)nx * ny && !(f32 && stencil);
   auto ride = [&]() {
-    return !h->timing && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES && h->quad_shape < 0;
+    return few && !h->timing && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES && h->quad_shape < 0;
   };
   auto rec_ptr = [&](int slot) -> double* {
     return slot < 0 ? nullptr : h->d_ring + (size_t)slot * h->nrec_fields * h->np;
@@ -979,12 +987,11 @@ int lbrb_step(lbrb_t* h, int n) {
     PJob<Real> J{};
     const void* f[4][5];
     group_fields(g, f);
-    for (int q = 0; q < g.n; q++) {
-      double* r = rec_ptr(g.rec[q]);
-      J.V[q] = PView<Real>{(const Real*)f[q][0], (const Real*)f[q][1], (const Real*)f[q][2], (const Real*)f[q][3],
-                           (const Real*)f[q][4], nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, r ? 1 : 0,
-                           h->p.record_full, r, h->dflags};
-    }
+    for (int q = 0; q < g.n; q++)
+      J.step[q] = {(const Real*)f[q][0], (const Real*)f[q][1], (const Real*)f[q][2], (const Real*)f[q][3],
+                   (const Real*)f[q][4], rec_ptr(g.rec[q])};
+    J.P = h->px, J.ptype = h->ptype, J.dflags = h->dflags, J.beta = h->p.beta;
+    J.np = h->np, J.nx = nx, J.ny = ny, J.pitch = h->pitch, J.full = h->p.record_full;
     J.nsteps = g.n;
     return J;
   };
@@ -1602,8 +1609,10 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
     // launches write two slots that the forward pass overwrites)
     float ms = 0.f;
     int sh = 0;
-    if (f32) sh = tune_pair_fp32(seg_view<float>(h, chk, trial1, 0), seg_view<float>(h, chk, trial2, 0), h->stream, &ms);
-    else sh = tune_pair_fp64(seg_view<double>(h, chk, trial1, 0), seg_view<double>(h, chk, trial2, 0), h->stream, &ms);
+    // (storing the moments, as the launches of a gradient window mostly do)
+    const int mom = dJdT0 ? 1 : 0;
+    if (f32) sh = tune_pair_fp32(seg_view<float>(h, chk, trial1, mom), seg_view<float>(h, chk, trial2, mom), h->stream, &ms);
+    else sh = tune_pair_fp64(seg_view<double>(h, chk, trial1, mom), seg_view<double>(h, chk, trial2, mom), h->stream, &ms);
     CK(h, cudaGetLastError());
     h->pair_shape = sh;
     h->pair_ms = ms;

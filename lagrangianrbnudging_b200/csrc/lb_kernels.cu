@@ -70,12 +70,20 @@ __global__ void __launch_bounds__(BS, MINB) lb_node_kernel(const LBView<Real> V)
 // ------------------------------------------------------- two steps per launch
 // Temporal blocking of two steps n, n+1 in TX x TY tiles, one per block
 // (lb_pair.cuh: tile_block, the per-block work).
-// The first J.nblocks blocks advance particles (PJob; FP32 at 512x256 with 4096
-// tracers: 7.1 us per step with its records, 8.2 with particle launches of
-// their own).
+template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
+__global__ void __launch_bounds__(NT, MINB) lb_pair_kernel(const LBView<Real> V1, const LBView<Real> V2) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char pair_smem[];
+  tile_block<Real, TX, TY, NT, Off>(V1, V2, blockIdx.x * TX, blockIdx.y * TY, pair_smem);
+}
+// the same tiles after blocks that advance particles (PJob: the first
+// J.nblocks; FP32 at 512x256 with 4096 tracers 3.9 us per step, 5.4 with
+// particle launches of their own).  A kernel of its own: launches without
+// particles keep the smaller parameter block and the plain grid.
 template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
 __global__ void __launch_bounds__(NT, MINB)
-    lb_pair_kernel(const LBView<Real> V1, const LBView<Real> V2, const __grid_constant__ PJob<Real> J, int tiles_x) {
+    lb_pair_job_kernel(const LBView<Real> V1, const LBView<Real> V2, const __grid_constant__ PJob<Real> J,
+                       int tiles_x) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char pair_smem[];
   const int b = blockIdx.x - J.nblocks;
@@ -132,36 +140,38 @@ constexpr PairShape PAIR_SHAPES[] = {{32, 8, 256, 4}, {32, 4, 128, 6}, {32, 16, 
 constexpr int NPAIR = sizeof(PAIR_SHAPES) / sizeof(PAIR_SHAPES[0]);
 static_assert(NPAIR <= NUM_PAIR_SHAPES, "pair shape table");
 
-// the caller's particles (or none) for blocks of nt threads
-template <typename Real>
-static PJob<Real> job_for(const PJob<Real>* job, int nt) {
-  PJob<Real> J{};
-  if (job && job->nsteps > 0) {
-    J = *job;
-    J.nblocks = (J.V[0].np + nt - 1) / nt;
-  }
-  return J;
+template <auto kernel, size_t smem>
+static cudaError_t tile_limit() {
+  // the shared-memory limit is a per-device attribute of the kernel: set
+  // once per device (one bit per device ordinal, per kernel)
+  static std::atomic<unsigned long long> attr_set{0};
+  return smem_limit_once((const void*)kernel, smem, attr_set);
 }
-
+template <typename Real, int TX, int TY, int NT, int MINB, typename Off>
+static cudaError_t launch_tile(const LBView<Real>& V1, const LBView<Real>& V2, cudaStream_t s, bool pdl,
+                               const PJob<Real>* job) {
+  constexpr size_t smem = tile_smem_bytes<Real, TX, TY>();
+  const int tiles_x = (V1.nx + TX - 1) / TX, tiles_y = (V1.ny + TY - 1) / TY;
+  if (job && job->nsteps > 0) {
+    constexpr auto kernel = lb_pair_job_kernel<Real, TX, TY, NT, MINB, Off>;
+    const cudaError_t e = tile_limit<kernel, smem>();
+    if (e != cudaSuccess) return e;
+    PJob<Real> J = *job;
+    J.nblocks = (J.np + NT - 1) / NT;
+    return launch_k(kernel, dim3((unsigned)(J.nblocks + (long)tiles_x * tiles_y)), NT, smem, s, pdl, V1, V2, J, tiles_x);
+  }
+  constexpr auto kernel = lb_pair_kernel<Real, TX, TY, NT, MINB, Off>;
+  const cudaError_t e = tile_limit<kernel, smem>();
+  if (e != cudaSuccess) return e;
+  return launch_k(kernel, dim3(tiles_x, tiles_y), NT, smem, s, pdl, V1, V2);
+}
 template <typename Real, int TX, int TY, int NT, int MINB>
 static cudaError_t launch_pair_t(const LBView<Real>& V1, const LBView<Real>& V2, cudaStream_t s, bool pdl,
                                  const PJob<Real>* job) {
-  constexpr size_t smem = tile_smem_bytes<Real, TX, TY>();
-  const PJob<Real> J = job_for(job, NT);
-  const int tiles_x = (V1.nx + TX - 1) / TX;
-  const unsigned grid = (unsigned)(J.nblocks + (long)tiles_x * ((V1.ny + TY - 1) / TY));
-  auto go = [&](auto kernel) -> cudaError_t {
-    // the shared-memory limit is a per-device attribute of the kernel: set
-    // once per device (one bit per device ordinal, per instantiation)
-    static std::atomic<unsigned long long> attr_set{0};
-    const cudaError_t e = smem_limit_once((const void*)kernel, smem, attr_set);
-    if (e != cudaSuccess) return e;
-    return launch_k(kernel, grid, NT, smem, s, pdl, V1, V2, J, tiles_x);
-  };
   // (FP64 holds twice the registers per value: half the blocks per SM)
   constexpr int MB = std::is_same<Real, double>::value ? (MINB + 1) / 2 : MINB;
-  if (off32_ok(V1.plane)) return go(lb_pair_kernel<Real, TX, TY, NT, MB, uint32_t>);
-  return go(lb_pair_kernel<Real, TX, TY, NT, MB, size_t>);
+  if (off32_ok(V1.plane)) return launch_tile<Real, TX, TY, NT, MB, uint32_t>(V1, V2, s, pdl, job);
+  return launch_tile<Real, TX, TY, NT, MB, size_t>(V1, V2, s, pdl, job);
 }
 
 // The marching shapes: wave_march, one warp per strip and chunk, (warps per
@@ -403,12 +413,11 @@ cudaError_t launch_pair_fp64(const LBView<double>& V1, const LBView<double>& V2,
   return launch_pair<double>(V1, V2, shape, s, pdl, job);
 }
 
-// pair shape autotuner: as tune(), the trial launches write only buffers the
-// real steps overwrite (the views' destinations; no rho or T)
+// pair shape autotuner: as tune(), the trial launches write only what the
+// views store, buffers the real steps overwrite
 template <typename Real>
 static int tune_pair(const LBView<Real>& A, const LBView<Real>& B, cudaStream_t s, float* best_ms) {
-  LBView<Real> V1 = A, V2 = B;
-  V1.write_rt = V2.write_rt = 0;
+  const LBView<Real>&V1 = A, &V2 = B;
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
@@ -439,11 +448,9 @@ static int tune_pair(const LBView<Real>& A, const LBView<Real>& B, cudaStream_t 
   if (best_ms) *best_ms = bt / reps;
   return best;
 }
-// the four-step launch shapes, timed as tune_pair's (no T or rho stored)
+// the four-step launch shapes, timed as tune_pair's
 template <typename Real>
-static int tune_quad(const LBView<Real> (&Vin)[4], cudaStream_t s, float* best_ms) {
-  LBView<Real> V[4] = {Vin[0], Vin[1], Vin[2], Vin[3]};
-  for (auto& v : V) v.write_rt = 0;
+static int tune_quad(const LBView<Real> (&V)[4], cudaStream_t s, float* best_ms) {
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);

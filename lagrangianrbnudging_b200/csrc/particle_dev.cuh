@@ -209,22 +209,37 @@ __device__ __forceinline__ void particle_update(const PView<Real>& V, int p) {
   X[7 * n + p] = vold;
 }
 
-// Particles of the steps before, advanced inside a fused launch by its first
-// nblocks blocks: nsteps (2 or 4) steps whose u, v (and T) are complete, in
-// slots that the launch does not write.  A particle launch of its own is a
-// chain of dependent gathers (6-7 us for two steps however few the
-// particles); beside the fused step it costs almost nothing.
+// Particles of the two steps before, advanced inside a fused launch by its
+// first nblocks blocks: steps whose u, v (and T) are complete, in slots that
+// the launch does not write.  A particle launch of its own is a chain of
+// dependent gathers (6-7 us for two steps however few the particles); beside
+// the fused step it costs little while the particles are few beside the
+// nodes.  nsteps 0: none.
 template <typename Real>
 struct PJob {
-  PView<Real> V[4];
+  struct Step {
+    const Real *u, *v, *ub, *vb, *T;
+    double* rec;  // ring slot of a record step, else null
+  } step[2];
+  double* P;
+  const int* ptype;
+  unsigned* dflags;
+  double beta;
+  int np, nx, ny, pitch, full;
   int nsteps, nblocks;
 };
+// (FP32: runs without the derivative stencil only)
 template <typename Real>
 __device__ __noinline__ void particle_job(const PJob<Real>& J, int block) {
   const int p = block * blockDim.x + threadIdx.x;
-  if (p >= J.V[0].np) return;
+  if (p >= J.np) return;
 #pragma unroll 1
-  for (int q = 0; q < J.nsteps; q++) particle_update<Real, true>(J.V[q], p);
+  for (int q = 0; q < J.nsteps; q++) {
+    const typename PJob<Real>::Step& S = J.step[q];
+    const PView<Real> V{S.u, S.v, S.ub, S.vb, S.T, J.nx, J.ny, J.pitch, J.P, J.ptype, J.np, J.beta, S.rec ? 1 : 0,
+                        J.full, S.rec, J.dflags};
+    particle_update<Real, sizeof(Real) == 8>(V, p);
+  }
 }
 
 }  // namespace lbrb
