@@ -229,6 +229,9 @@ __device__ __forceinline__ void tile_block(const LBView<Real>& V1, const LBView<
 // Wall rows bounce back from the node's own populations: at row 0 the slot
 // of row -1 takes the level's f4, f7, f8 instead (read at the node's own
 // columns); at the top the c_y = +1 populations of the row itself are there.
+// Rows outside the domain, and a level's iterations before its first inputs,
+// run on whatever is in their places: nothing of them is stored, and no row of
+// the domain reads them (a level skips the arithmetic of the latter).
 // Level 1 takes the domain's first and last row, and the ghost rows of a
 // y-slab (S = 2), by pull_node / pull_ghost_row instead of a stage.
 template <int S>
@@ -362,7 +365,6 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   int p0 = 0, p1 = 6;  // c_y = +1 slots of this iteration's row (and of the row two before it), and of the row before
   for (int it = 0; it < nit; it++, y++) {
     P2 f[NPOP], g[NPOP], F, r, u, v, t;
-    const bool on1 = y >= ylo && y <= yhi;
     cp_wait<D - 1>();
     __syncwarp();
     const Real* st = sm + stage * WAVE_STAGE * 64;
@@ -377,7 +379,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         g[k] = icx(k) == 1 ? sown(NPOP + k) : (icx(k) == -1 ? snxt(NPOP + k) : smid(NPOP + k));
       });
       F = smid(2 * NPOP);
-    } else if (on1) {
+    } else if (y >= ylo && y <= yhi) {
       Real a[2 * NPOP], b[2 * NPOP];
       auto one = [&](int x, Real* p, Real& Fx) {
         x = (x + 16 * nx) % nx;
@@ -400,19 +402,17 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
     __syncwarp();
     issue(it + D < nit ? y + D : -1, stage);
     stage = stage + 1 == D ? 0 : stage + 1;
-    if (on1) {
-      collide_pair(V1, f, g, F, r, u, v, t);
-      if constexpr (NUD) {
-        if (na != 0) {
-          const double sv = (double)na * (1.0 / FIX_SCALE);
+    collide_pair(V1, f, g, F, r, u, v, t);
+    if constexpr (NUD) {
+      if (na != 0) {
+        const double sv = (double)na * (1.0 / FIX_SCALE);
 #pragma unroll
-          for (int k = 0; k < NPOP; k++) g[k].x = g[k].x + nudge_increment<Real>(k, sv);
-        }
-        if (nb != 0) {
-          const double sv = (double)nb * (1.0 / FIX_SCALE);
+        for (int k = 0; k < NPOP; k++) g[k].x = g[k].x + nudge_increment<Real>(k, sv);
+      }
+      if (nb != 0) {
+        const double sv = (double)nb * (1.0 / FIX_SCALE);
 #pragma unroll
-          for (int k = 0; k < NPOP; k++) g[k].y = g[k].y + nudge_increment<Real>(k, sv);
-        }
+        for (int k = 0; k < NPOP; k++) g[k].y = g[k].y + nudge_increment<Real>(k, sv);
       }
     }
     if constexpr (NUD) {
@@ -424,9 +424,8 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
       constexpr int off = S - s;
       const LBView<Real>& V = view(std::integral_constant<int, s - 1>{});
       const int yr = y - (s - 1);
-      const bool on = s == 1 ? on1 : (yr >= max(ya - off, 0) && yr <= min(ya + Hc - 1 + off, ny - 1));
       // the level's moments (and the last level's state) in its strip and chunk
-      if (on && yr >= ya && yr < ya + Hc) {
+      if ((unsigned)(yr - ya) < (unsigned)Hc) {
         const int c = 2 * lane - off + (off & 1);  // column in the strip of the aligned pair
         const bool ok = c >= 0 && c < ncols;
         const int xc = x0 + c;
@@ -468,7 +467,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         if (lo) a5 = mid(w1, 1), a6 = mid(w1, 2);
         P2 b2 = mid(w1, 3), b5 = own(w1, 4), b6 = nxt(w1, 5);
         __syncwarp();
-        if (on && 2 * lane < CW) {
+        if (2 * lane < CW) {
           auto put = [&](Real* q, int i, P2 a) { reinterpret_cast<P2*>(q + i * CW)[lane] = a; };
           put(w0, 0, f[0]), put(w0, 1, f[1]), put(w0, 2, f[3]);
           put(w0, 3, g[0]), put(w0, 4, g[1]), put(w0, 5, g[3]);
@@ -503,7 +502,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
           for (int k = 0; k < NPOP; k++) g[k] = pair_of(ga[k], gb[k]);
         }
         __syncwarp();
-        if (yn >= max(ya - off + 1, 0) && yn <= min(ya + Hc - 2 + off, ny - 1)) collide_pair(VN, f, g, F, r, u, v, t);
+        if (it >= 2 * s) collide_pair(VN, f, g, F, r, u, v, t);  // (before that its inputs are not there yet)
       }
     });
     const int pt = p0;
