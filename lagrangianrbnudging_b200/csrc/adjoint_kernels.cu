@@ -87,10 +87,11 @@ struct AdjMom {
 template <typename LX>
 __device__ __forceinline__ AdjMom adj_moments(LX&& X) {
   constexpr double w0 = w_of(0), w1 = w_of(1), w5 = w_of(5);
-  const double s13 = X(1) + X(3), d13 = X(1) - X(3);
-  const double s24 = X(2) + X(4), d24 = X(2) - X(4);
-  const double c57 = X(5) + X(7), c68 = X(6) + X(8);
-  const double e57 = X(5) - X(7), e68 = X(6) - X(8);
+  const double x1 = X(1), x2 = X(2), x3 = X(3), x4 = X(4), x5 = X(5), x6 = X(6), x7 = X(7), x8 = X(8);
+  const double s13 = x1 + x3, d13 = x1 - x3;
+  const double s24 = x2 + x4, d24 = x2 - x4;
+  const double c57 = x5 + x7, c68 = x6 + x8;
+  const double e57 = x5 - x7, e68 = x6 - x8;
   const double cs = c57 + c68;
   AdjMom M;
   M.mxx = fma(w1, s13, w5 * cs);
@@ -237,55 +238,91 @@ struct AdjPairView {
 // TX x TY tile, NT threads; the ring of (TX+2)(TY+2) nodes takes a second,
 // partial round of phase 1 when it has more nodes than the block threads
 // (tiles with (TX+2)(TY+2) == NT, e.g. 30x6 on 256 threads, measured slower
-// on B200: unaligned rows and more blocks)
+// on B200: unaligned rows and more blocks).
+// Phase 1's lambda comes straight into the shared memory that its results
+// take: a thread starts the copies of all its ring nodes (both rounds) before
+// any arithmetic, and each result replaces the value it was made from.  The
+// launch is bound by latency and the L1 / shared-memory data path (78% busy):
+// 1024x512, window of 400 steps with FP32 forward, in ms: 13.4-13.7 on 32x8
+// tiles; 14.1 with the first round through registers; 14.0-14.4 with each
+// lambda read from shared memory twice (fewer registers, more blocks); 14.8
+// with both rounds through registers, one after the other.
+__device__ __forceinline__ void adj_cp8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 template <typename Real, int TX, int TY, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) adjoint_pair_kernel(const AdjPairView<Real> P) {
   pdl_wait();
   extern __shared__ double sm[];
-  constexpr int HX = TX + 2, HY = TY + 2, NH = HX * HY;
+  constexpr int HX = TX + 2, HY = TY + 2, NH = HX * HY, ROUNDS = (NH + NT - 1) / NT;
   static_assert(NT >= TX * TY, "one thread per tile node");
   const AdjView<Real>& V = P.a;
   const int nx = V.nx, ny = V.ny;
   const int x0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
-  // the forward quantities of this thread's phase-2 node do not depend on
-  // phase 1: their loads go out first and overlap it
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  const int x = x0 + tx, j = j0 + ty;
-  const bool mine = (int)threadIdx.x < TX * TY && x < nx && j < ny;
-  AdjLoc L2{};
-  double lt2 = 0.0;
-  if (mine) {
-    L2 = adj_locals(P.mom_b, P.Fin_b, V.plane, (size_t)j * V.pitch + x);
-    if (P.lT_b) lt2 = (double)P.lT_b[(size_t)j * V.pitch + x] * (1.0 / ADJ_FIX);
-  }
-  // phase 1: step n at the tile and its ring
-  for (int h = threadIdx.x; h < NH; h += blockDim.x) {
+  // phase 1's inputs: lambda^n and lambda F^{n+1} into shared memory, the
+  // step's moments, F and observation term into registers
+  Real m1[ROUNDS][5];
+  long long t1[ROUNDS];
+  int row[ROUNDS];  // -1: no node there
+#pragma unroll
+  for (int q = 0; q < ROUNDS; q++) {
+    const int h = threadIdx.x + q * NT;
+    row[q] = -1;
+    if (h >= NH) continue;
     const int hx = h % HX, hy = h / HX;
     int xh = x0 - 1 + hx;
     const int jh = j0 - 1 + hy;
     if (xh == -1) xh = nx - 1;
     else if (xh == nx) xh = 0;
-    if (jh < 0 || jh >= ny || xh >= nx) continue;  // no node there
+    if (jh < 0 || jh >= ny || xh >= nx) continue;
+    row[q] = jh;
     const size_t o = (size_t)jh * V.pitch + xh;
-    double lf[NPOP], lg[NPOP];
 #pragma unroll
     for (int k = 0; k < NPOP; k++) {
-      lf[k] = V.lf_out[(size_t)k * V.plane + o];
-      lg[k] = V.lg_out[(size_t)k * V.plane + o];
+      adj_cp8(sm + k * NH + h, V.lf_out + (size_t)k * V.plane + o);
+      adj_cp8(sm + (NPOP + k) * NH + h, V.lg_out + (size_t)k * V.plane + o);
     }
-    const double lFo = V.lF[o];
-    const double lt = V.lT ? (double)V.lT[o] * (1.0 / ADJ_FIX) : 0.0;
-    const AdjLoc L = adj_locals(V.mom, V.Fin, V.plane, o);
+    adj_cp8(sm + 2 * NPOP * NH + h, V.lF + o);
+#pragma unroll
+    for (int c = 0; c < 4; c++) m1[q][c] = V.mom[(size_t)c * V.plane + o];
+    m1[q][4] = V.Fin[o];
+    t1[q] = V.lT ? V.lT[o] : 0;
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  // the forward quantities of this thread's phase-2 node do not depend on
+  // phase 1: their loads go out too and overlap it
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  const int x = x0 + tx, j = j0 + ty;
+  const bool mine = (int)threadIdx.x < TX * TY && x < nx && j < ny;
+  Real m2[5] = {};
+  long long t2 = 0;
+  if (mine) {
+    const size_t o = (size_t)j * V.pitch + x;
+#pragma unroll
+    for (int c = 0; c < 4; c++) m2[c] = P.mom_b[(size_t)c * V.plane + o];
+    m2[4] = P.Fin_b[o];
+    if (P.lT_b) t2 = P.lT_b[o];
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // phase 1: step n at the tile and its ring (a thread reads only what it copied)
+#pragma unroll
+  for (int q = 0; q < ROUNDS; q++) {
+    if (row[q] < 0) continue;
+    double* S = sm + threadIdx.x + q * NT;
+    const AdjLoc L{(double)m1[q][0], (double)m1[q][3], (double)m1[q][1], (double)m1[q][2], (double)m1[q][4]};
     double lFin;
     adj_local(
-        V, L, jh, [&](int k) { return lf[k]; }, [&](int k) { return lg[k]; }, lFo, lt,
-        [&](int k, double val) { sm[k * NH + h] = val; },
-        [&](int k, double val) { sm[(NPOP + k) * NH + h] = val; }, lFin);
-    sm[2 * NPOP * NH + h] = lFin;
+        V, L, row[q], [&](int k) { return S[k * NH]; }, [&](int k) { return S[(NPOP + k) * NH]; }, S[2 * NPOP * NH],
+        (double)t1[q] * (1.0 / ADJ_FIX), [&](int k, double val) { S[k * NH] = val; },
+        [&](int k, double val) { S[(NPOP + k) * NH] = val; }, lFin);
+    S[2 * NPOP * NH] = lFin;
   }
   __syncthreads();
   // phase 2: step n-1 at the tile
   if (!mine) return;
+  const AdjLoc L2{(double)m2[0], (double)m2[3], (double)m2[1], (double)m2[2], (double)m2[4]};
+  const double lt2 = (double)t2 * (1.0 / ADJ_FIX);
   const int hs = (tx + 1) + (ty + 1) * HX;  // this node in the ring layout
   // output m of step n-1 at this node went to node (x, j) + c_m (pulled there
   // by step n); at a wall it was bounced back into opp(m) here (f) or left
@@ -736,9 +773,9 @@ cudaError_t launch_adjoint_pair(bool fp32, int variant, const void* after_a, con
     P.lg_in = lg_in;
     P.lF_out = lF_out;
     switch (variant) {
-      case 1: return launch_pair_t<Real, 32, 4, 128, 6>(P, s);
+      case 1: return launch_pair_t<Real, 32, 6, 192, 2>(P, s);
       case 2: return launch_pair_t<Real, 32, 8, 256, 2>(P, s);
-      case 3: return launch_pair_t<Real, 32, 8, 256, 3>(P, s);
+      case 3: return launch_pair_t<Real, 32, 16, 512, 1>(P, s);
       case 4: return launch_march_t<Real, 7, 1, 1>(P, 2, s);
       case 5: return launch_march_t<Real, 6, 1, 1>(P, 2, s);
       case 6: return launch_march_t<Real, 7, 1, 2>(P, 2, s);
