@@ -239,11 +239,11 @@ __global__ void __launch_bounds__(512)
   const EnsAux<Real>& A = aux2[c.x];
   const int o = c.y + (threadIdx.x >> 2);
   if (o >= A.nobs) return;
-  const double* ob = ens_obs_row(A, ctr[0] - 1);
-  obs_apply_one(A.g, A.plane, A.nx, A.ny, A.pitch, ob[o], ob[A.nobs + o], threadIdx.x & 3, A.acc);
   const EnsAux<Real>& A1 = aux1[c.x];
-  const double* o1 = ens_obs_row(A1, ctr[0] - 2);
-  obs_clear_one(A1.nx, A1.ny, A1.pitch, o1[o], o1[A1.nobs + o], threadIdx.x & 3, A1.acc2, A1.nmask);
+  const double *ob = ens_obs_row(A, ctr[0] - 1), *o1 = ens_obs_row(A1, ctr[0] - 2);
+  const double x1 = o1[o], y1 = o1[A1.nobs + o], x2 = ob[o], y2 = ob[A.nobs + o];
+  obs_clear_one(A1.nx, A1.ny, A1.pitch, x1, y1, threadIdx.x & 3, A1.acc2, A1.nmask);
+  obs_apply_one(A.g, A.plane, A.nx, A.ny, A.pitch, x2, y2, threadIdx.x & 3, A.acc);
 }
 
 // pair variants 0-2, strips (chunk heights, ens_pair_chunk); 3-4, tiles: (tile

@@ -88,14 +88,18 @@ __device__ __forceinline__ void obs_apply_one(Real* __restrict__ g, size_t plane
   int jy = (y1 - 1) % ny; if (jy < 0) jy += ny;
   if (nyl >= 0 && (unsigned)(jy - j0) >= (unsigned)nyl) return;
   const size_t q = (size_t)(jy - j0) * pitch + ix;
+  // the populations are loaded before their sum is known, all nine at once:
+  // loaded one after the other, each behind the store before it, they were a
+  // chain of nine trips to memory.  (Only the thread that takes the sum writes
+  // the node; what the others loaded is not used.)
+  Real v[NPOP];
+#pragma unroll
+  for (int k = 0; k < NPOP; k++) v[k] = g[(size_t)k * plane + q];
   const long long sfix = (long long)atomicExch(&acc[q], 0ull);
   if (sfix == 0) return;
   const double sv = (double)sfix * (1.0 / FIX_SCALE);
 #pragma unroll
-  for (int k = 0; k < NPOP; k++) {
-    Real* a = g + (size_t)k * plane + q;
-    *a = *a + nudge_increment<Real>(k, sv);
-  }
+  for (int k = 0; k < NPOP; k++) g[(size_t)k * plane + q] = v[k] + nudge_increment<Real>(k, sv);
 }
 
 // T^n at node (i, j) as the fused step forms it: the sum of the g streaming

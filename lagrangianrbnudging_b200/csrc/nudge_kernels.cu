@@ -370,8 +370,9 @@ __global__ void obs_apply_clear_kernel(Real* __restrict__ g, size_t plane, int n
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 4 * nobs) return;
   const int p = t >> 2;
-  obs_apply_one(g, plane, nx, ny, pitch, ox2[p], oy2[p], t & 3, acc);
-  obs_clear_one(nx, ny, pitch, ox1[p], oy1[p], t & 3, acc2, mask);
+  const double x1 = ox1[p], y1 = oy1[p], x2 = ox2[p], y2 = oy2[p];
+  obs_clear_one(nx, ny, pitch, x1, y1, t & 3, acc2, mask);
+  obs_apply_one(g, plane, nx, ny, pitch, x2, y2, t & 3, acc);
 }
 
 cudaError_t launch_obs_pre_fp32(const LBView<float>& V, const double* ox, const double* oy, const double* oT,
