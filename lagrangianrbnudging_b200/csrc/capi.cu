@@ -12,6 +12,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <thread>
@@ -189,7 +190,12 @@ static void parallel_copy(const std::vector<CopyJob>& jobs) {
       std::memcpy(pieces[i].dst, pieces[i].src, pieces[i].bytes);
   };
   std::vector<std::thread> pool;
-  for (unsigned t = 1; t < nt; t++) pool.emplace_back(work);
+  try {
+    pool.reserve(nt);
+    for (unsigned t = 1; t < nt; t++) pool.emplace_back(work);
+  } catch (const std::exception&) {
+    // no more threads to be had: those that started and this one share the pieces
+  }
   work();
   for (std::thread& t : pool) t.join();
 }
@@ -361,11 +367,14 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
   }
   // the extra u, v slots (lbrb_step: particles inside the next launch, and
   // four-step launches); a run without memory for them steps in pairs, each
-  // followed by its particles
+  // followed by its particles.  They take at most a quarter of what is free,
+  // so that they displace nothing that a run allocates later.
   if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge != LBRB_NUDGE_REFBOX) {
     constexpr int extra = UV_SLOTS - 3;
     const size_t pb1 = h->plane * h->esize;
-    if (cudaMalloc(&h->uv_extra, 2 * extra * pb1) != cudaSuccess) {
+    size_t avail = 0, total = 0;
+    const bool room = cudaMemGetInfo(&avail, &total) == cudaSuccess && 2 * extra * pb1 <= avail / 4;
+    if (!room || cudaMalloc(&h->uv_extra, 2 * extra * pb1) != cudaSuccess) {
       cudaGetLastError();
       h->uv_extra = nullptr;
     } else {

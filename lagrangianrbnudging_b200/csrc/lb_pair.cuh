@@ -320,7 +320,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   constexpr int VEC = 16 / ES;
   const int cq = VEC * (F32 ? (lane & 15) : lane);
   const bool cp_ok = cq < ncols + 2 * S;
-  const unsigned cp_col = (unsigned)((x0 - S + cq + 16 * nx) % nx);
+  const unsigned cp_col = (unsigned)((x0 - S + cq + nx) % nx);  // (x0 - S >= -4 >= -nx)
   const Real* const cp_base = (!F32 || lane < 16 ? V1.fsrc : V1.gsrc) + cp_col;
   const unsigned cp_dst = sm_addr + (!F32 || lane < 16 ? 0 : NPOP * ROW) + cq * ES;
   const ptrdiff_t g_off = F32 ? 0 : V1.gsrc - V1.fsrc;
@@ -349,7 +349,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
   // it do not count; predicated loads of the sums): guarded by branches they
   // cost 15 us of an 88 us launch at 2048x1024, with one observation.
   const bool nudged = NUD && V1.nmask != nullptr;  // (an ensemble's members may have none)
-  const int nxa = (x0 - (S - 1) + 2 * lane + 16 * nx) % nx, nxb = nxa + 1 == nx ? 0 : nxa + 1;
+  const int nxa = (x0 - (S - 1) + 2 * lane + nx) % nx, nxb = nxa + 1 == nx ? 0 : nxa + 1;
   const unsigned* const mw_a = V1.nmask + (nxa >> 5);
   const unsigned* const mw_b = V1.nmask + (nxb >> 5);
   unsigned ma = 0, mb = 0;
@@ -413,7 +413,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
     } else if (y >= ylo && y <= yhi) {
       Real a[2 * NPOP], b[2 * NPOP];
       auto one = [&](int x, Real* p, Real& Fx) {
-        x = (x + 16 * nx) % nx;
+        x = (x + nx) % nx;
         if (S == 2 && (y < 0 || y >= ny)) {
           pull_ghost_row<Real, size_t>(V1, y < 0, x, p, p + NPOP, Fx);
         } else {
@@ -458,7 +458,7 @@ __device__ __forceinline__ void wave_march(GetV&& view, int x0, int ncols, int y
         const bool ok = c >= 0 && c < ncols;
         const int xc = x0 + c;
         const unsigned o = (unsigned)yr * pitch + (unsigned)(xc >= nx ? xc - nx : xc);
-        const unsigned ob = o * (unsigned)ES;  // (bytes within a plane)
+        const unsigned ob = o * (unsigned)ES;  // (bytes within a plane: 2^32 of them would be a run of 200 GB)
         constexpr bool ODD = (off & 1) != 0;
         if constexpr (s == S) {
           if (ok) {
