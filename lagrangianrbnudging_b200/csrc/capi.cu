@@ -558,6 +558,7 @@ int lbrb_particles_set(lbrb_t* h, int n, const int* ids, const double* x, const 
   std::memcpy(&P[8 * (size_t)n], invtau, n * sizeof(double));
   CK(h, cudaMemcpyAsync(h->px, P.data(), P.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   CK(h, cudaMemcpyAsync(h->pid, ids, n * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  h->inertial = std::any_of(ptype, ptype + n, [](int t) { return t != LBRB_PTYPE_TRACER; });
   CK(h, cudaMemcpyAsync(h->ptype, ptype, n * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   CK(h, cudaStreamSynchronize(h->stream));
   h->h_ids.assign(ids, ids + n);
@@ -943,7 +944,18 @@ int lbrb_step(lbrb_t* h, int n) {
   // against 5.4).  With the Maxey-Riley stencil it pays in FP64 (512x256: 9.1
   // against 10.8) but not in FP32 (9.9 against 8.7), whose tile launches
   // leave too few registers for it.
-  const bool stencil = h->p.beta != 0.0 || h->p.record_full;
+  // Beta acts on inertial particles only: a run of tracers, at whatever beta,
+  // needs no stencil (FP32 at 512x256 with 4096 tracers and the default beta:
+  // 3.5 us per step, 5.1 with it).
+  // Single steps, and what a caller captures, keep beta: their graphs may be
+  // replayed with other particles.
+  double beta = h->p.beta;
+  if (!h->inertial && h->np > 0 && beta != 0.0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(h->stream, &cs));
+    if (cs == cudaStreamCaptureStatusNone) beta = 0.0;
+  }
+  const bool stencil = beta != 0.0 || h->p.record_full;
   const bool few = 8L * h->np <= (long)nx * ny && !(f32 && stencil);
   auto ride = [&]() {
     return few && !h->timing && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES && h->quad_shape < 0;
@@ -977,10 +989,10 @@ int lbrb_step(lbrb_t* h, int n) {
     double* r[4] = {rec_ptr(g.rec[0]), rec_ptr(g.rec[1]), rec_ptr(g.rec[2]), rec_ptr(g.rec[3])};
     const int tm = tmark_begin(h, 1, h->stream);
     if (g.n == 4)
-      CK(h, launch_particles_quad(f, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta, h->p.record_full, r,
+      CK(h, launch_particles_quad(f, f32, nx, ny, h->pitch, h->px, h->ptype, h->np, beta, h->p.record_full, r,
                                   h->dflags, h->stream, pdl_ok));
     else
-      CK(h, launch_particles_pair(f[0], f[1], f32, nx, ny, h->pitch, h->px, h->ptype, h->np, h->p.beta,
+      CK(h, launch_particles_pair(f[0], f[1], f32, nx, ny, h->pitch, h->px, h->ptype, h->np, beta,
                                   h->p.record_full, r[0], r[1], h->dflags, h->stream, pdl_ok));
     tmark_end(h, tm, h->stream);
     return group_copies(g);
@@ -999,7 +1011,7 @@ int lbrb_step(lbrb_t* h, int n) {
     for (int q = 0; q < g.n; q++)
       J.step[q] = {(const Real*)f[q][0], (const Real*)f[q][1], (const Real*)f[q][2], (const Real*)f[q][3],
                    (const Real*)f[q][4], rec_ptr(g.rec[q])};
-    J.P = h->px, J.ptype = h->ptype, J.dflags = h->dflags, J.beta = h->p.beta;
+    J.P = h->px, J.ptype = h->ptype, J.dflags = h->dflags, J.beta = beta;
     J.np = h->np, J.nx = nx, J.ny = ny, J.pitch = h->pitch, J.full = h->p.record_full;
     J.nsteps = g.n;
     return J;

@@ -381,6 +381,7 @@ struct Handle {
   double* px = nullptr;  // [9][np]: x y u v xo yo uo vo invtau
   int* pid = nullptr;
   int* ptype = nullptr;
+  bool inertial = true;  // some particle may not be a tracer (lbrb_particles_set)
   bool particles_set = false;
   // records
   int nrec_fields = LBRB_REC_NBASIC;
