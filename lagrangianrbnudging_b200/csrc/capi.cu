@@ -1068,7 +1068,7 @@ int lbrb_step(lbrb_t* h, int n) {
         return fail(h, LBRB_ERR_STATE, "step: observation file for this interval not loaded");
       const int tm = tmark_begin(h, 2, h->stream);
       CK(h, launch_box_nudge(h->nb, h->nbi, h->nobs, nx, ny, h->slab ? h->slab_ny_total : ny, h->slab ? h->slab_j0 : 0,
-                             nt, istep, h->ncx, h->ncy, h->box_work, ++h->box_seq, h->nudge_vol, h->tempreadint,
+                             nt, istep, h->ncx, h->ncy, h->box_work, h->nudge_vol, h->tempreadint,
                              h->pitch, h->stream, pdl_ok));
       tmark_end(h, tm, h->stream);
       if (istep % nt == 1) h->nudge_file_loaded = false;

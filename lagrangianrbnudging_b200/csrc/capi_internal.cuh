@@ -78,7 +78,7 @@ cudaError_t launch_bilinear_nudge_slab(const void* Trows, void* g, bool fp32, si
                                        cudaStream_t s);
 size_t box_cell_ints(int n, int ncell);
 cudaError_t launch_box_nudge(double* nb, int* nbi, int n, int nx, int ny, int ny_total, int j0, int nt, int istep,
-                             int ncx, int ncy, int* work, int seq, int* nudge_vol, double* tempreadint, int pitch,
+                             int ncx, int ncy, int* work, int* nudge_vol, double* tempreadint, int pitch,
                              cudaStream_t s, bool pdl);
 cudaError_t launch_bilinear_nudge(void* T, void* g, bool fp32, size_t plane, int nx, int ny,
                                   int pitch, const double* ox, const double* oy, const double* oT,

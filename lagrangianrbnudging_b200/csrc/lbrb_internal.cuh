@@ -399,7 +399,6 @@ struct Handle {
   double* nud_term = nullptr;
   double* tsum0 = nullptr;  // [pitch]: row 0's sum of g without the 1/2 nud_term (LBView::tsum0)
   int* box_work = nullptr;  // cell lists (nudge_kernels.cu: box_cell_ints)
-  int box_seq = 0;          // steps whose boxes were placed
   int ncx = 0, ncy = 0;
   bool nudge_init_done = false, nudge_file_loaded = false;
   int* h_chk = nullptr;     // host copy of chk_id (ids matched on the host)

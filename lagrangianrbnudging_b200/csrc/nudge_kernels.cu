@@ -42,9 +42,13 @@ enum { NBI_CHK = 0, NBI_BC, NBI_XIDX, NBI_YIDX, NBI_COUNT };
 // Contributions of a cell: the first BOX_SLOTS in the cell's own slots, the
 // rest in one list of (cell, key) for all cells.  A step's lists and counters
 // are one of three sets, by `seq` (a count of steps, from 1): this step's, the
-// last one's, and the one that this step leaves cleared for the next.
+// last one's, and the one that this step leaves cleared for the next.  The
+// count is in device memory, so that replays of a captured step go on from the
+// step before them, whichever it was.  Each of its two words is written by the
+// kernel that does not read it.
 constexpr int BOX_SLOTS = 8;
-enum { BOX_NCELLS = 0, BOX_NOVER, BOX_NSORT, BOX_NCOUNT };
+enum { BOX_NCELLS = 0, BOX_NOVER, BOX_NSORT, BOX_NCOUNT = 4 };
+enum { BOX_PLACED = 3 * BOX_NCOUNT, BOX_PLACING, BOX_HEAD = 16 };  // words after the counters: steps done, begun
 
 struct BoxView {
   double* nb;
@@ -53,8 +57,8 @@ struct BoxView {
   // the whole domain's rows (positions and boxes); j0: the handle's first
   // row in the domain (0 unless a y-slab)
   int n, nx, ny, nt, istep, nyT, j0;
-  int ncx, ncell, seq;
-  int* cnt;      // [3][BOX_NCOUNT]
+  int ncx, ncell;
+  int* cnt;      // [3][BOX_NCOUNT], BOX_PLACED, BOX_PLACING
   int* count;    // [ncell] contributions of a cell this step (0 between steps)
   int* stamp;    // [ncell] the last step that touched a cell
   int* slots;    // [ncell][BOX_SLOTS]
@@ -182,8 +186,10 @@ __global__ void __launch_bounds__(32) box_bin_kernel(const BoxView B) {
   pdl_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= B.n) return;
+  const int seq = B.cnt[BOX_PLACED] + 1;
+  if (k == 0) B.cnt[BOX_PLACING] = seq;
   box_interp(B, k);
-  const int set = B.seq % 3;
+  const int set = seq % 3;
   int* cnt = B.cnt + set * BOX_NCOUNT;
   for (int img = 0; img < 3; img++) {
     int xa, xb, ya, yb;
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(32) box_bin_kernel(const BoxView B) {
         const int c = cy * B.ncx + cx, key = 3 * k + img;
         const int at = atomicAdd(&B.count[c], 1);
         if (at == 0) {
-          B.stamp[c] = B.seq;
+          B.stamp[c] = seq;
           B.cells[(size_t)set * B.lcap + atomicAdd(&cnt[BOX_NCELLS], 1)] = c;
         }
         if (at < BOX_SLOTS) B.slots[(size_t)c * BOX_SLOTS + at] = key;
@@ -217,14 +223,18 @@ __global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B)
   __shared__ int keys[BOX_SLOTS];
   __shared__ int sh[2];
   const int tid = threadIdx.x;
-  const int set = B.seq % 3, last = (B.seq + 2) % 3, next = (B.seq + 1) % 3;
-  const int ncur = B.cnt[set * BOX_NCOUNT + BOX_NCELLS], nlast = B.cnt[last * BOX_NCOUNT + BOX_NCELLS];
+  // (the three sets' counts loaded with the step, not after it)
+  const int seq = B.cnt[BOX_PLACING];
+  const int n0 = B.cnt[BOX_NCELLS], n1 = B.cnt[BOX_NCOUNT + BOX_NCELLS], n2 = B.cnt[2 * BOX_NCOUNT + BOX_NCELLS];
+  const int set = seq % 3, last = (seq + 2) % 3, next = (seq + 1) % 3;
+  const int ncur = set == 0 ? n0 : (set == 1 ? n1 : n2), nlast = last == 0 ? n0 : (last == 1 ? n1 : n2);
   if (blockIdx.x == 0 && tid < BOX_NCOUNT) B.cnt[next * BOX_NCOUNT + tid] = 0;
+  if (blockIdx.x == 0 && tid == 0) B.cnt[BOX_PLACED] = seq;
   const double* Tint = NB(B, NB_TINT);
   for (int it = blockIdx.x; it < ncur + nlast; it += gridDim.x) {
     const bool now = it < ncur;
     const int c = now ? B.cells[(size_t)set * B.lcap + it] : B.cells[(size_t)last * B.lcap + it - ncur];
-    if (!now && B.stamp[c] == B.seq) continue;  // (listed in this step too)
+    if (!now && B.stamp[c] == seq) continue;  // (listed in this step too)
     const int cx = c % B.ncx, cy = c / B.ncx;
     const int i = cx * CELL + (tid % CELL) + 1;  // reference node coordinates (of the domain)
     const int j = B.j0 + cy * CELL + (tid / CELL) + 1;
@@ -290,19 +300,19 @@ __global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B)
 // counts, stamps, slots, three lists, the overflow list, scratch
 static size_t box_lcap(int n, int ncell) { return std::min((size_t)ncell, (size_t)12 * n); }
 size_t box_cell_ints(int n, int ncell) {
-  return 16 + (size_t)ncell * (2 + BOX_SLOTS) + 3 * box_lcap(n, ncell) + (size_t)4 * 12 * n;
+  return BOX_HEAD + (size_t)ncell * (2 + BOX_SLOTS) + 3 * box_lcap(n, ncell) + (size_t)4 * 12 * n;
 }
 
-// `work`: box_cell_ints ints, zero at the start of the run; seq: 1, 2, ... from call to call
+// `work`: box_cell_ints ints, zero at the start of the run
 cudaError_t launch_box_nudge(double* nb, int* nbi, int n, int nx, int ny, int ny_total, int j0, int nt, int istep,
-                             int ncx, int ncy, int* work, int seq, int* nudge_vol, double* tempreadint, int pitch,
+                             int ncx, int ncy, int* work, int* nudge_vol, double* tempreadint, int pitch,
                              cudaStream_t s, bool pdl) {
   const int ncell = ncx * ncy;
   const size_t lcap = box_lcap(n, ncell);
-  BoxView B{nb, nbi, n, nx, ny, nt, istep, ny_total, j0, ncx, ncell, seq};
+  BoxView B{nb, nbi, n, nx, ny, nt, istep, ny_total, j0, ncx, ncell};
   B.cnt = work;
-  B.over = reinterpret_cast<int2*>(work + 16);
-  B.scratch = work + 16 + (size_t)2 * 12 * n;
+  B.over = reinterpret_cast<int2*>(work + BOX_HEAD);
+  B.scratch = work + BOX_HEAD + (size_t)2 * 12 * n;
   B.count = B.scratch + (size_t)2 * 12 * n;
   B.stamp = B.count + ncell;
   B.slots = B.stamp + ncell;
