@@ -171,7 +171,15 @@ LBRB_API int lbrb_set_stream(lbrb_t *h, void *cuda_stream);
  * a two-step launch is faster than a replay of two single steps); 0: off;
  * 1: every grid, ahead of two-step launches.  Not used with nudging,
  * per-kernel timing, a y-slab, the legacy default stream, or while the
- * caller captures the handle's stream.  No counterpart in the reference. */
+ * caller captures the handle's stream.
+ * A caller's capture gets the launches themselves, single and two-step ones
+ * (the launch shapes timed by direct calls before it; a capture makes no
+ * trial launches).  A captured call of a multiple of 12 steps ends in the
+ * buffers that it started from, so its graph can be replayed any number of
+ * times; after direct calls, capture again.  The handle's step count, records
+ * and observation rows are those of the capture.  Once captured, a handle
+ * takes no four-step launches (lbrb_set_pairs) in direct calls either.
+ * No counterpart in the reference. */
 LBRB_API int lbrb_set_graph(lbrb_t *h, int mode);
 /* Two steps per launch inside lbrb_step: the fused kernel computes step n
  * at a tile and a one-node ring into shared memory and step n+1 from there,
@@ -195,7 +203,8 @@ LBRB_API int lbrb_set_graph(lbrb_t *h, int mode);
  * timed faster than two two-step launches and the shape was not fixed by
  * lbrb_set_pair_shape: the same steps, again with identical results, while
  * more than four steps of the call remain and at most one of the four is a
- * record step.
+ * record step; never on a handle whose steps a caller has captured
+ * (lbrb_set_graph).
  * Replaces, for two or four steps at a time, the reference's per-step sweeps
  * (stream, moments, collide: temppart_dump.c:1674-1759). */
 LBRB_API int lbrb_set_pairs(lbrb_t *h, int mode);

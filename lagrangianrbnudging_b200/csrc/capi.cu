@@ -878,6 +878,15 @@ int lbrb_step(lbrb_t* h, int n) {
   const bool f32 = fp32(h);
   const bool refbox = h->p.nudge == LBRB_NUDGE_REFBOX;
   const int nx = h->p.nx, ny = h->p.ny;
+  // A caller that captures steps may replay them, again and again and between
+  // direct calls, wherever the buffers are back where they were: from then on
+  // this handle takes single and two-step launches in the three u, v slots
+  // only, so that where a call of n steps ends follows from n, not from which
+  // launches were timed faster.
+  cudaStreamCaptureStatus capture_status = cudaStreamCaptureStatusNone;
+  CK(h, cudaStreamIsCapturing(h->stream, &capture_status));
+  const bool capturing = capture_status != cudaStreamCaptureStatusNone;
+  h->captured = h->captured || capturing;
   if (h->lb_shape < 0) {
     // autotune the fused kernel's launch shape on this grid (trial launches
     // write only the buffers the real step overwrites)
@@ -950,15 +959,12 @@ int lbrb_step(lbrb_t* h, int n) {
   // Single steps, and what a caller captures, keep beta: their graphs may be
   // replayed with other particles.
   double beta = h->p.beta;
-  if (!h->inertial && h->np > 0 && beta != 0.0) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(h->stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone) beta = 0.0;
-  }
+  if (!h->inertial && h->np > 0 && !capturing) beta = 0.0;
   const bool stencil = beta != 0.0 || h->p.record_full;
   const bool few = 8L * h->np <= (long)nx * ny && !(f32 && stencil);
   auto ride = [&]() {
-    return few && !h->timing && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES && h->quad_shape < 0;
+    return few && !h->timing && !h->captured && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES &&
+           h->quad_shape < 0;
   };
   auto rec_ptr = [&](int slot) -> double* {
     return slot < 0 ? nullptr : h->d_ring + (size_t)slot * h->nrec_fields * h->np;
@@ -1016,10 +1022,17 @@ int lbrb_step(lbrb_t* h, int n) {
     J.nsteps = g.n;
     return J;
   };
-  // k slots for the steps of the next launch, none that the pending group
-  // reads; a pending group that leaves too few, or whose record T the launch
-  // would overwrite (t0, t1: the T buffers it stores to), goes first
+  // k slots for the steps of the next launch.  Two steps go round the three
+  // slots as two single ones do; four take the spare ones first.  With riding
+  // particles, none that the pending group reads; a pending group that leaves
+  // too few, or whose record T the launch would overwrite (t0, t1: the T
+  // buffers it stores to), goes first.
   auto take_slots = [&](int k, const void* t0, const void* t1, int* out) -> int {
+    if (k == 4 || !ride()) {
+      const int in3[2] = {3 - h->uvcur - h->uvprev, h->uvprev};
+      for (int q = 0; q < k; q++) out[q] = q < k - 2 ? 3 + q : in3[q - (k - 2)];
+      return LBRB_OK;
+    }
     bool hit = false;
     for (int q = 0; q < pend.n; q++) hit = hit || (pend.rec[q] >= 0 && (pend.T[q] == t0 || pend.T[q] == t1));
     if (pend.n && (hit || pend.n + 1 + k > h->nuv)) {
@@ -1314,7 +1327,7 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   // four steps per launch where a timed launch beats two timed pair launches
   auto quads_ok = [&]() {
-    return step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed;
+    return step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed && !h->captured;
   };
   auto tune_quads = [&]() -> int {
     h->quad_shape = -1;
@@ -1344,32 +1357,21 @@ int lbrb_step(lbrb_t* h, int n) {
   if (step_pairs_ok(h) && h->pair_shape < 0 && n >= 3) {
     // the pair shape is timed on the first call that can use pairs (trial
     // launches write only what the steps overwrite)
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(h->stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone && !(graphs_on && n - 1 >= GRAPH_STEPS)) {
+    if (!capturing && !(graphs_on && n - 1 >= GRAPH_STEPS)) {
       const int rc = tune_pairs();
       if (rc) return rc;
     }
   }
   if (n >= 5 && h->quad_shape == -2 && quads_ok() && !graphs_on) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(h->stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone) {
-      const int rc = tune_quads();
-      if (rc) return rc;
-    }
+    const int rc = tune_quads();
+    if (rc) return rc;
   }
   // Small grids: a run of GRAPH_STEPS plain steps (no record, not the call's
   // last step) replays a CUDA graph of exactly the launches `one` would
   // issue.  Those launches depend only on the buffer phase (cur, uvcur,
   // uvprev), so one graph per phase is captured on first use.
-  bool graphs = graph_ok(h);
-  if (graphs) {
-    // a caller capturing this stream gets the launches themselves
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(h->stream, &cs));
-    graphs = cs == cudaStreamCaptureStatusNone;
-  }
+  // (a caller capturing this stream gets the launches themselves)
+  const bool graphs = graph_ok(h) && !capturing;
   int s = 0;
   while (s < n) {
     if (graphs && n - 1 - s >= GRAPH_STEPS) {

@@ -67,3 +67,63 @@ def test_box_nudged_interval(nt):
         for k in ma:
             np.testing.assert_array_equal(ma[k], mb[k], err_msg=k)
         del g
+
+
+def free_run(precision, nx, ny, kind):
+    """kind: no particles, few tracers, or few inertial particles (d/dt reads
+    the u, v of the step before)"""
+    n = 0 if kind == "none" else 96
+    r = lb.Run(**lb.closure(nx, ny, Ra=1e6, Pr=1.0, U=0.1), precision=precision, nprtcl=n,
+               beta=0.5 if kind == "inertial" else 0.0)
+    r.set_pairs(1)
+    r.init_conduction(11, 5e-2)
+    if n:
+        rng = np.random.default_rng(5)
+        ptype = np.full(n, 1 if kind == "inertial" else 0, np.int32)
+        z = np.zeros(n)
+        r.set_particles(np.arange(n, dtype=np.int32), rng.uniform(0.5, nx + 0.5, n), rng.uniform(1.0, ny, n), z, z,
+                        ptype, np.where(ptype == 1, 1.0 / 50.0, 0.0))
+    return r
+
+
+def assert_same(a, b):
+    for p, q in zip(a.get_populations(), b.get_populations()):
+        np.testing.assert_array_equal(p, q)
+    ma, mb = a.get_moments(), b.get_moments()
+    for k in ma:
+        np.testing.assert_array_equal(ma[k], mb[k], err_msg=k)
+    if a.np:
+        pa, pb = a.get_particles(), b.get_particles()
+        for k in pa:
+            np.testing.assert_array_equal(pa[k], pb[k], err_msg=k)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("nx,ny", [(128, 64), (2048, 1024)])
+@pytest.mark.parametrize("kind,n,between", [("none", 8, 0), ("none", 24, 0), ("tracers", 12, 12), ("inertial", 12, 12),
+                                            ("inertial", 24, 36)])
+def test_replays_after_tuned_calls(precision, nx, ny, kind, n, between):
+    """a call captured once its launch shapes are timed, whichever they are,
+    over lengths that end in the buffers they started from; with particles
+    also around direct calls of such lengths"""
+    import torch
+
+    with free_run(precision, nx, ny, kind) as a, free_run(precision, nx, ny, kind) as b:
+        stream = torch.cuda.Stream()
+        a.set_stream(stream.cuda_stream)
+        a.step(21)
+        g = capture(a, stream, n)
+        total = 21
+        for q in range(4):
+            with torch.cuda.stream(stream):
+                g.replay()
+            total += n
+            if between and q % 2:
+                a.step(between)
+                total += between
+        torch.cuda.synchronize()
+        a.set_stream(None)
+        b.set_pairs(0)
+        b.step(total)
+        assert_same(a, b)
+        del g
