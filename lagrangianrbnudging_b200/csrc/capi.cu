@@ -76,6 +76,63 @@ static void tuned_put(std::map<TuneKey, TuneVal>& m, const lbrb_t* h, int shape,
   m[tune_key(h)] = {shape, ms};
 }
 
+// The spare u, v slots of a run with particles (lbrb_step: riding particles,
+// four-step launches).  Steps use them and transfers the staging slots, never
+// both at once, so they take the staging memory where they fit (up to about
+// 8 M nodes in FP32, 4 M in FP64; xfer_units waits for the steps).  Larger runs
+// allocate them in the first call that uses them, if they take at most a
+// quarter of what is free, and give them back when that turns out not to use
+// them or when another allocation of the handle fails.  Without them a run
+// steps in pairs, each followed by its particles.
+struct RelaxedCapture {  // (another thread's capture does not concern these allocations)
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&m); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&m); }
+};
+static bool ensure_spare(lbrb_t* h) {
+  if (h->nuv == UV_SLOTS) return true;
+  if (h->spare_denied) return false;
+  constexpr int planes = 2 * (UV_SLOTS - 3);
+  const size_t pb = h->plane * h->esize;
+  char* at = (char*)h->staging;
+  if (planes * pb > h->staging_bytes) {
+    RelaxedCapture relaxed;
+    size_t avail = 0, total = 0;
+    const bool room = cudaMemGetInfo(&avail, &total) == cudaSuccess && planes * pb <= avail / 4;
+    if (!room || cudaMalloc(&h->uv_extra, planes * pb) != cudaSuccess) {
+      cudaGetLastError();
+      h->uv_extra = nullptr;
+      h->spare_denied = true;
+      return false;
+    }
+    at = (char*)h->uv_extra;
+  }
+  for (int q = 0; q < planes; q++) h->uv[3 + q / 2][q % 2] = at + q * pb;
+  h->nuv = UV_SLOTS;
+  return true;
+}
+static void release_spare(lbrb_t* h) {
+  if (!h->uv_extra) return;
+  RelaxedCapture relaxed;
+  cudaFree(h->uv_extra);  // (waits for what still reads them)
+  h->uv_extra = nullptr;
+  for (int q = 3; q < UV_SLOTS; q++) h->uv[q][0] = h->uv[q][1] = nullptr;
+  h->nuv = 3;
+}
+// device memory for one of the handle's calls, at the cost of the spare slots
+// if need be (between calls they hold nothing)
+static cudaError_t dev_alloc(lbrb_t* h, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && h->uv_extra) {
+    cudaGetLastError();
+    release_spare(h);
+    h->spare_denied = true;
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();  // (reported here, not by the next launch)
+  return e;
+}
+
 // the full-size scratch of the rare paths (restart-route moments, post-stream
 // dump), allocated on first use
 static int ensure_big(lbrb_t* h, size_t bytes) {
@@ -83,7 +140,7 @@ static int ensure_big(lbrb_t* h, size_t bytes) {
   if (h->big) cudaFree(h->big);
   h->big = nullptr;
   h->big_bytes = 0;
-  cudaError_t e = cudaMalloc(&h->big, bytes);
+  cudaError_t e = dev_alloc(h, &h->big, bytes);
   if (e != cudaSuccess) return fail(h, LBRB_ERR_NOMEM, "scratch allocation", e);
   h->big_bytes = bytes;
   return LBRB_OK;
@@ -112,6 +169,8 @@ static int xfer_units(lbrb_t* h, bool in, double* host, size_t unit, int ub, int
   double* slot[2] = {(double*)h->staging, (double*)h->staging + h->stage_slot};
   cudaEvent_t* copied = h->xfer_ev;
   cudaEvent_t* converted = h->xfer_ev + 2;
+  if (in && h->nuv == UV_SLOTS)  // (the staging memory may hold u, v slots of steps still running)
+    for (int sl = 0; sl < 2; sl++) CK(h, cudaEventRecord(converted[sl], h->stream));
   int c = 0;
   for (int u0 = ub; u0 < ue; u0 += per, c++) {
     const int u1 = std::min(ue, u0 + per), sl = c & 1;
@@ -256,7 +315,7 @@ static void free_all(lbrb_t* h) {
   auto F = [](void* q) { if (q) cudaFree(q); };
   F(h->pops[0]); F(h->pops[1]); F(h->F[0]); F(h->F[1]);
   F(h->rho[0]); F(h->rho[1]); F(h->T[0]); F(h->T[1]);
-  for (int a = 0; a < 3; a++) for (int b = 0; b < 2; b++) F(h->uv_own[a][b]);
+  for (int a = 0; a < 3; a++) for (int b = 0; b < 2; b++) F(h->uv[a][b]);
   F(h->uv_extra);
   F(h->px); F(h->pid); F(h->ptype); F(h->d_ring);
   if (h->h_ring) cudaFreeHost(h->h_ring);
@@ -342,13 +401,9 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
   void** scal[] = {&h->F[0], &h->F[1], &h->rho[0], &h->rho[1], &h->T[0], &h->T[1],
                    &h->uv[0][0], &h->uv[0][1], &h->uv[1][0], &h->uv[1][1], &h->uv[2][0], &h->uv[2][1]};
   for (void** s : scal) {
-    if (cudaMalloc(s, h->plane * h->esize) != cudaSuccess) {
-      std::memcpy(h->uv_own, h->uv, sizeof h->uv_own);
-      return done(LBRB_ERR_NOMEM);
-    }
+    if (cudaMalloc(s, h->plane * h->esize) != cudaSuccess) return done(LBRB_ERR_NOMEM);
     cudaMemset(*s, 0, h->plane * h->esize);
   }
-  std::memcpy(h->uv_own, h->uv, sizeof h->uv_own);
   h->np = p.nprtcl;
   if (h->np > 0) {
     if (dalloc(&h->px, (size_t)9 * h->np) || dalloc(&h->pid, h->np) || dalloc(&h->ptype, h->np))
@@ -363,23 +418,6 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
       for (int s = 0; s < h->p.record_slots; s++)
         if (cudaEventCreateWithFlags(&h->ring_ev[s], cudaEventDisableTiming) != cudaSuccess)
           return done(LBRB_ERR_CUDA);
-    }
-  }
-  // the extra u, v slots (lbrb_step: particles inside the next launch, and
-  // four-step launches); a run without memory for them steps in pairs, each
-  // followed by its particles.  They take at most a quarter of what is free,
-  // so that they displace nothing that a run allocates later.
-  if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge != LBRB_NUDGE_REFBOX) {
-    constexpr int extra = UV_SLOTS - 3;
-    const size_t pb1 = h->plane * h->esize;
-    size_t avail = 0, total = 0;
-    const bool room = cudaMemGetInfo(&avail, &total) == cudaSuccess && 2 * extra * pb1 <= avail / 4;
-    if (!room || cudaMalloc(&h->uv_extra, 2 * extra * pb1) != cudaSuccess) {
-      cudaGetLastError();
-      h->uv_extra = nullptr;
-    } else {
-      for (int q = 0; q < 2 * extra; q++) h->uv[3 + q / 2][q % 2] = (char*)h->uv_extra + q * pb1;
-      h->nuv = UV_SLOTS;
     }
   }
   h->nobs = p.nobs;
@@ -667,7 +705,7 @@ int lbrb_nudge_obs(lbrb_t* h, int first_step, int nsteps, const double* x, const
     if (h->obs) cudaFree(h->obs);
     h->obs = nullptr;
     h->obs_cap_steps = 0;
-    cudaError_t e = cudaMalloc(&h->obs, (size_t)nsteps * 3 * n * sizeof(double));
+    cudaError_t e = dev_alloc(h, (void**)&h->obs, (size_t)nsteps * 3 * n * sizeof(double));
     if (e != cudaSuccess) return fail(h, LBRB_ERR_NOMEM, "nudge_obs allocation", e);
     h->obs_cap_steps = nsteps;
   }
@@ -887,6 +925,7 @@ int lbrb_step(lbrb_t* h, int n) {
   CK(h, cudaStreamIsCapturing(h->stream, &capture_status));
   const bool capturing = capture_status != cudaStreamCaptureStatusNone;
   h->captured = h->captured || capturing;
+  int s = 0;  // steps of the call queued so far
   if (h->lb_shape < 0) {
     // autotune the fused kernel's launch shape on this grid (trial launches
     // write only the buffers the real step overwrites)
@@ -962,10 +1001,11 @@ int lbrb_step(lbrb_t* h, int n) {
   if (!h->inertial && h->np > 0 && !capturing) beta = 0.0;
   const bool stencil = beta != 0.0 || h->p.record_full;
   const bool few = 8L * h->np <= (long)nx * ny && !(f32 && stencil);
-  auto ride = [&]() {
-    return few && !h->timing && !h->captured && h->nuv == UV_SLOTS && h->pair_shape < NUM_PAIR_TILES &&
-           h->quad_shape < 0;
+  auto may_ride = [&]() {
+    return h->np > 0 && few && !h->captured && h->pair_shape >= 0 && h->pair_shape < NUM_PAIR_TILES &&
+           h->quad_shape < 0 && step_pairs_ok(h);
   };
+  auto ride = [&]() { return may_ride() && !h->timing && h->nuv == UV_SLOTS; };
   auto rec_ptr = [&](int slot) -> double* {
     return slot < 0 ? nullptr : h->d_ring + (size_t)slot * h->nrec_fields * h->np;
   };
@@ -1024,9 +1064,12 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   // k slots for the steps of the next launch.  Two steps go round the three
   // slots as two single ones do; four take the spare ones first.  With riding
-  // particles, none that the pending group reads; a pending group that leaves
-  // too few, or whose record T the launch would overwrite (t0, t1: the T
-  // buffers it stores to), goes first.
+  // particles, none that the pending group reads (the order `rot` of all five,
+  // two at a time, from uvcur on); a pending group that leaves too few, or
+  // whose record T the launch would overwrite (t0, t1: the T buffers it stores
+  // to), goes first.  An order is chosen so that the last two steps of the
+  // call's pairs are in slots 0-2, where the next call expects them.
+  int rot[UV_SLOTS] = {}, at = 0;
   auto take_slots = [&](int k, const void* t0, const void* t1, int* out) -> int {
     if (k == 4 || !ride()) {
       const int in3[2] = {3 - h->uvcur - h->uvprev, h->uvprev};
@@ -1035,37 +1078,43 @@ int lbrb_step(lbrb_t* h, int n) {
     }
     bool hit = false;
     for (int q = 0; q < pend.n; q++) hit = hit || (pend.rec[q] >= 0 && (pend.T[q] == t0 || pend.T[q] == t1));
-    if (pend.n && (hit || pend.n + 1 + k > h->nuv)) {
-      const int rc = flush();
-      if (rc) return rc;
+    if (hit)
+      if (const int rc = flush()) return rc;
+    if (!pend.n) {
+      const int m = h->p.nudge == LBRB_NUDGE_BILINEAR ? (n - s - 1) / 2 * 2 : (n - s) / 2 * 2;  // steps in pairs
+      bool used[UV_SLOTS] = {};
+      auto put = [&](int q) {
+        int i = 0;
+        while (used[i]) i++;
+        used[rot[q] = i] = true;
+      };
+      used[rot[0] = h->uvcur] = true;
+      const int e1 = m % UV_SLOTS, e0 = (m + UV_SLOTS - 1) % UV_SLOTS;
+      for (int q = 1; q < UV_SLOTS; q++)
+        if (q == e0 || q == e1) put(q);
+      for (int q = 1; q < UV_SLOTS; q++)
+        if (q != e0 && q != e1) put(q);
+      at = 0;
     }
-    unsigned busy = 1u << h->uvcur;
-    if (pend.n) busy |= 1u << pend.prev;
-    for (int q = 0; q < pend.n; q++) busy |= 1u << pend.slot[q];
-    for (int q = 0, at = 0; q < k; at++)
-      if (!(busy >> at & 1u)) out[q++] = at;
+    for (int q = 0; q < k; q++) out[q] = rot[at = (at + 1) % UV_SLOTS];
     return LBRB_OK;
   };
-  // uvcur and uvprev back among slots 0-2 (graphs of single steps hold slot
-  // pointers: captured again)
-  auto settle_slots = [&]() {
-    bool moved = false;
-    for (int* s : {&h->uvcur, &h->uvprev}) {
-      if (*s < 3) continue;
-      const int other = s == &h->uvcur ? h->uvprev : h->uvcur;
-      const int j = other == 0 ? 1 : 0;
-      std::swap(h->uv[*s][0], h->uv[j][0]);
-      std::swap(h->uv[*s][1], h->uv[j][1]);
-      *s = j;
-      moved = true;
+  // uvcur and uvprev back among slots 0-2 where a call ended otherwise than its
+  // pairs' order foresaw: copied, as graphs of steps hold the slots' addresses
+  auto settle_slots = [&]() -> int {
+    for (int* p : {&h->uvcur, &h->uvprev}) {
+      if (*p < 3) continue;
+      int j = 0;
+      while (j == h->uvcur || j == h->uvprev) j++;
+      for (int c = 0; c < 2; c++)
+        CK(h, cudaMemcpyAsync(h->uv[j][c], h->uv[*p][c], h->plane * h->esize, cudaMemcpyDeviceToDevice, h->stream));
+      *p = j;
     }
-    if (!moved) return;
-    for (cudaGraphExec_t& g : h->graph_exec)
-      if (g) cudaGraphExecDestroy(g), g = nullptr;
+    return LBRB_OK;
   };
   auto one = [&](bool last) -> int {
     if (const int rc = flush()) return rc;
-    settle_slots();
+    if (const int rc = settle_slots()) return rc;
     const int istep = h->istep + 1;
     const bool rec = h->np > 0 && h->p.noutconfig > 0 && istep % h->p.noutconfig == 0;
     if (rec && !h->slab && (h->rec_head - h->rec_tail) >= h->p.record_slots)
@@ -1331,10 +1380,10 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   auto tune_quads = [&]() -> int {
     h->quad_shape = -1;
-    if (h->np > 0 && h->nuv < UV_SLOTS) return LBRB_OK;  // (no memory for the slots: pairs)
     float ms = 0.f;
     int sh = 0;
     if (!tuned_get(g_tuned_quad, h, &sh, &ms)) {
+      if (h->np > 0 && !ensure_spare(h)) return LBRB_OK;  // (no memory for the slots: pairs)
       const bool none[4] = {};
       const int slot[4] = {3, 4, 3 - h->uvcur - h->uvprev, h->uvprev};
       if (f32) {
@@ -1366,13 +1415,18 @@ int lbrb_step(lbrb_t* h, int n) {
     const int rc = tune_quads();
     if (rc) return rc;
   }
+  bool quads = h->quad_shape >= 0 && quads_ok();
+  if (h->np > 0 && !graphs_on && n >= 3) {
+    if (quads || may_ride()) ensure_spare(h);
+    else if (!capturing) release_spare(h);
+    quads = quads && h->nuv == UV_SLOTS;
+  }
   // Small grids: a run of GRAPH_STEPS plain steps (no record, not the call's
   // last step) replays a CUDA graph of exactly the launches `one` would
   // issue.  Those launches depend only on the buffer phase (cur, uvcur,
   // uvprev), so one graph per phase is captured on first use.
   // (a caller capturing this stream gets the launches themselves)
   const bool graphs = graph_ok(h) && !capturing;
-  int s = 0;
   while (s < n) {
     if (graphs && n - 1 - s >= GRAPH_STEPS) {
       bool plain = true;
@@ -1417,7 +1471,7 @@ int lbrb_step(lbrb_t* h, int n) {
         continue;
       }
     }
-    if (!graphs && n - s >= 5 && h->quad_shape >= 0 && quads_ok()) {
+    if (!graphs && n - s >= 5 && quads) {
       // (a group with two record steps, or whose record would not fit in the
       // ring, goes in pairs or single steps, which report the overflow)
       int need = 0;
@@ -1454,7 +1508,7 @@ int lbrb_step(lbrb_t* h, int n) {
     s++;
   }
   if (const int rc = flush()) return rc;
-  settle_slots();
+  if (const int rc = settle_slots()) return rc;
   // the caller's stream sees the record copies as part of the steps
   if (h->join_pending) {
     CK(h, cudaEventRecord(h->join_ev, h->copy_stream));
@@ -1480,8 +1534,8 @@ int lbrb_adjoint_set_obs(lbrb_t* h, int nobs_steps, const int* steps, int nobs, 
   delete[] h->adj_steps;
   h->adj_steps = nullptr;
   const size_t n = (size_t)nobs_steps * nobs;
-  if (cudaMalloc(&h->adj_obs, 3 * n * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&h->adj_res, n * sizeof(double)) != cudaSuccess)
+  if (dev_alloc(h, (void**)&h->adj_obs, 3 * n * sizeof(double)) != cudaSuccess ||
+      dev_alloc(h, (void**)&h->adj_res, n * sizeof(double)) != cudaSuccess)
     return fail(h, LBRB_ERR_NOMEM, "adjoint_set_obs: allocation");
   for (int a = 0; a < nobs_steps; a++) {
     double* b = h->adj_obs + (size_t)a * 3 * nobs;
@@ -1502,7 +1556,7 @@ static int grow(lbrb_t* h, void** p, size_t* have, size_t need) {
   if (*p) cudaFree(*p);
   *p = nullptr;
   *have = 0;
-  cudaError_t e = cudaMalloc(p, need);
+  cudaError_t e = dev_alloc(h, p, need);
   if (e != cudaSuccess) return fail(h, LBRB_ERR_NOMEM, "adjoint buffers", e);
   *have = need;
   return LBRB_OK;
@@ -1570,7 +1624,7 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
   // two segment buffers: the backward sweep of one segment reads one while
   // the recompute of the segment before it fills the other
   if (!store && (rc = grow(h, &h->adj_seg, &h->adj_seg_bytes, 2 * (size_t)(K + 1) * sb))) return rc;
-  if (!h->adj_T0 && cudaMalloc(&h->adj_T0, nn * sizeof(double)) != cudaSuccess)
+  if (!h->adj_T0 && dev_alloc(h, (void**)&h->adj_T0, nn * sizeof(double)) != cudaSuccess)
     return fail(h, LBRB_ERR_NOMEM, "adjoint T0");
   CK(h, cudaMemcpyAsync(h->adj_T0, T0, nn * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   const double T0ref = T0_of(h), ng = -h->p.gravity;
@@ -1767,9 +1821,9 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
   }
   // ---- backward pass
   const size_t lp = NPOP * plane;  // one lambda population set (doubles)
-  if (!h->adj_lam && cudaMalloc((void**)&h->adj_lam, (4 * lp + 2 * plane) * sizeof(double)) != cudaSuccess)
+  if (!h->adj_lam && dev_alloc(h, (void**)&h->adj_lam, (4 * lp + 2 * plane) * sizeof(double)) != cudaSuccess)
     return fail(h, LBRB_ERR_NOMEM, "adjoint lambda");
-  if (!h->adj_lT && cudaMalloc((void**)&h->adj_lT, 2 * plane * sizeof(long long)) != cudaSuccess)
+  if (!h->adj_lT && dev_alloc(h, (void**)&h->adj_lT, 2 * plane * sizeof(long long)) != cudaSuccess)
     return fail(h, LBRB_ERR_NOMEM, "adjoint lambda T");
   double* lam[2][2] = {{h->adj_lam, h->adj_lam + lp}, {h->adj_lam + 2 * lp, h->adj_lam + 3 * lp}};
   double* lF[2] = {h->adj_lam + 4 * lp, h->adj_lam + 4 * lp + plane};

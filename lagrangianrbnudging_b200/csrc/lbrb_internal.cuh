@@ -365,13 +365,13 @@ struct Handle {
   void* rho[2] = {nullptr, nullptr};
   void* T[2] = {nullptr, nullptr};
   // nuv slots in all: three between calls (uvcur, uvprev and a free one are
-  // slots 0-2); the others, in uv_extra, hold steps of a four-step launch and
-  // steps whose particles the next launch advances.  lbrb_step may exchange
-  // slots' pointers; uv_own are those that free_all releases.
+  // slots 0-2); the others, in the staging memory or uv_extra where a run uses
+  // them, hold steps of a four-step launch and steps whose particles the next
+  // launch advances.
   void* uv[UV_SLOTS][2] = {};
-  void* uv_own[3][2] = {};
   void* uv_extra = nullptr;
   int nuv = 3;
+  bool spare_denied = false;  // no memory for uv_extra, or given back to another allocation
   int uvcur = 0, uvprev = 1;
   // second stream: the adjoint window's segment recompute (events order it
   // against `stream`)
