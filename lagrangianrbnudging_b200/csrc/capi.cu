@@ -1680,21 +1680,25 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
   auto launch_fwd = [&](const char* src, char* dst, int mom) { return launch_fwd_on(src, dst, mom, h->stream); };
   // two steps per launch where the state between them is not read: not an
   // observation step, not in a segment whose states the backward pass keeps
-  const bool fwd_pairs = pairs_ok(h) && nsteps >= 2;
-  if (fwd_pairs && h->pair_shape < 0) {
-    // the pair tile shape, timed on the window's initial state (trial
-    // launches write two slots that the forward pass overwrites)
-    float ms = 0.f;
-    int sh = 0;
-    // (storing the moments, as the launches of a gradient window mostly do)
+  // (the shape lbrb_step has or was given; else one timed on the window's
+  // initial state, the trial launches writing two slots that the forward pass
+  // overwrites and storing the moments as the launches of a gradient window
+  // mostly do.  What is timed here is the window's own: plain steps store less.)
+  if (pairs_ok(h) && nsteps >= 2 && h->pair_shape < 0 && h->adj_fwd_shape == -1) {
     const int mom = dJdT0 ? 1 : 0;
+    float ms = 0.f, single = 1e30f;
+    int sh = 0;
     if (f32) sh = tune_pair_fp32(seg_view<float>(h, chk, trial1, mom), seg_view<float>(h, chk, trial2, mom), h->stream, &ms);
     else sh = tune_pair_fp64(seg_view<double>(h, chk, trial1, mom), seg_view<double>(h, chk, trial2, mom), h->stream, &ms);
+    if (h->pair_mode < 0 && h->p.autotune)
+      single = f32 ? time_lb_fp32(seg_view<float>(h, chk, trial1, mom), h->p.twall, shape, h->stream)
+                   : time_lb_fp64(seg_view<double>(h, chk, trial1, mom), h->p.twall, shape, h->stream);
     CK(h, cudaGetLastError());
-    h->pair_shape = sh;
-    h->pair_ms = ms;
-    if (h->pair_mode < 0 && h->lb_shape_ms > 0.f && ms >= 2.f * h->lb_shape_ms) h->pair_mode = 0;
+    h->adj_fwd_shape = ms < 2.f * single ? sh : -2;
+    h->adj_fwd_ms = ms;
   }
+  const int fwd_shape = h->pair_fixed || h->adj_fwd_shape == -1 ? h->pair_shape : h->adj_fwd_shape;
+  const bool fwd_pairs = pairs_ok(h) && nsteps >= 2 && fwd_shape >= 0;
   // residual of observation step oi from a moment block's T
   auto residual = [&](int oi, const char* mblock) -> cudaError_t {
     const double* ob = h->adj_obs + (size_t)oi * 3 * nob;
@@ -1732,15 +1736,15 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
       return V;
     };
     for (int s = 0; s < nsteps;) {
-      if (fwd_pairs && h->pair_mode != 0 && s + 2 <= nsteps) {
+      if (fwd_pairs && s + 2 <= nsteps) {
         if (f32) {
           LBView<float> V1 = sview(0.f, s);
           V1.write_F = 1;
-          CK(h, launch_pair_fp32(V1, sview(0.f, s + 1), h->pair_shape, h->stream, true));
+          CK(h, launch_pair_fp32(V1, sview(0.f, s + 1), fwd_shape, h->stream, true));
         } else {
           LBView<double> V1 = sview(0.0, s);
           V1.write_F = 1;
-          CK(h, launch_pair_fp64(V1, sview(0.0, s + 1), h->pair_shape, h->stream, true));
+          CK(h, launch_pair_fp64(V1, sview(0.0, s + 1), fwd_shape, h->stream, true));
         }
         for (int q = 1; q <= 2; q++)
           if (obs_at[s + q] >= 0) CK(h, residual(obs_at[s + q], mblk(s + q)));
@@ -1773,16 +1777,16 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
         if (i + q < len) return keep ? segbuf(c) + (size_t)(i + q) * sb : (cur_state == slot1 ? slot1 + sb : slot1);
         return last ? segbuf(c) + (size_t)K * sb : chk + (size_t)(c + 1) * sb;
       };
-      if (fwd_pairs && h->pair_mode != 0 && !keep && i + 1 < len && obs_at[s] < 0) {
+      if (fwd_pairs && !keep && i + 1 < len && obs_at[s] < 0) {
         char* dst = out(2);
         const int oi = obs_at[s + 1];
         const int mom = (dJdT0 && i + 2 == len) || oi >= 0;
         if (f32)
           CK(h, launch_pair_fp32(seg_view<float>(h, cur_state, dst, 0), seg_view<float>(h, cur_state, dst, mom),
-                                 h->pair_shape, h->stream, true));
+                                 fwd_shape, h->stream, true));
         else
           CK(h, launch_pair_fp64(seg_view<double>(h, cur_state, dst, 0), seg_view<double>(h, cur_state, dst, mom),
-                                 h->pair_shape, h->stream, true));
+                                 fwd_shape, h->stream, true));
         if (oi >= 0) CK(h, residual(oi, mb(dst)));
         cur_state = dst;
         i += 2;
@@ -1910,16 +1914,16 @@ int lbrb_adjoint_window(lbrb_t* h, const double* T0, int nsteps, int K, double* 
       // so two steps go in one launch whose first step stores only those
       for (int i = 0; i + 1 < lenp;) {
         char* s1p = segbuf(cp) + (size_t)(i + 1) * sb;
-        if (fwd_pairs && h->pair_mode != 0 && i + 2 < lenp) {
+        if (fwd_pairs && i + 2 < lenp) {
           char* s2p = s1p + sb;
           if (f32) {
             LBView<float> V1 = seg_view<float>(h, state_in(cp, i), s1p, 1);
             V1.write_F = 1;
-            CK(h, launch_pair_fp32(V1, seg_view<float>(h, s1p, s2p, 1), h->pair_shape, rs, true));
+            CK(h, launch_pair_fp32(V1, seg_view<float>(h, s1p, s2p, 1), fwd_shape, rs, true));
           } else {
             LBView<double> V1 = seg_view<double>(h, state_in(cp, i), s1p, 1);
             V1.write_F = 1;
-            CK(h, launch_pair_fp64(V1, seg_view<double>(h, s1p, s2p, 1), h->pair_shape, rs, true));
+            CK(h, launch_pair_fp64(V1, seg_view<double>(h, s1p, s2p, 1), fwd_shape, rs, true));
           }
           i += 2;
         } else {
@@ -2853,6 +2857,7 @@ int lbrb_set_graph(lbrb_t* h, int mode) {
 int lbrb_set_pairs(lbrb_t* h, int mode) {
   if (!h || mode < -1 || mode > 1) return fail(h, LBRB_ERR_ARG, "set_pairs: mode must be -1, 0 or 1");
   h->pair_mode = mode;
+  h->adj_fwd_shape = -1;
   return LBRB_OK;
 }
 
@@ -2864,6 +2869,7 @@ int lbrb_set_pair_shape(lbrb_t* h, int shape) {
   h->pair_shape = shape;
   h->pair_fixed = shape >= 0;
   h->pair_ms = 0.f;
+  h->adj_fwd_shape = -1;
   return LBRB_OK;
 }
 
@@ -2874,11 +2880,13 @@ int lbrb_get_pair_shape(const lbrb_t* h, int* shape, int* tile_x, int* tile_y, f
   static const int TXS[] = {32, 32, 32, 64, 32, 30, 32, 32, 64, 60, 60, 60, 60, 60, 60},
                    TYS[] = {8, 4, 16, 4, 8, 8, 8, 6, 8, 1, 1, 1, 1, 1, 1};
   static_assert(sizeof(TXS) / sizeof(int) == NUM_PAIR_SHAPES, "pair shape table");
-  const int sh = h->pair_shape;
+  // (after windows alone, theirs)
+  const bool window = h->pair_shape < 0 && h->adj_fwd_shape >= 0;
+  const int sh = window ? h->adj_fwd_shape : h->pair_shape;
   if (shape) *shape = sh;
   if (tile_x) *tile_x = sh < 0 ? 0 : TXS[sh];
   if (tile_y) *tile_y = sh < 0 ? 0 : TYS[sh];
-  if (ms) *ms = h->pair_ms;
+  if (ms) *ms = window ? h->adj_fwd_ms : h->pair_ms;
   return LBRB_OK;
 }
 

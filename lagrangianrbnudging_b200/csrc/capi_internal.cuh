@@ -28,6 +28,8 @@ int tune_lb_fp64(const LBView<double>& V, int twall, cudaStream_t s, float* best
 cudaError_t launch_pull_fp64(const LBView<double>& V, int twall, void* outf, void* outg, cudaStream_t s);
 cudaError_t launch_pull_fp32(const LBView<float>& V, int twall, void* outf, void* outg, cudaStream_t s);
 int tune_lb_fp32(const LBView<float>& V, int twall, cudaStream_t s, float* best_ms);
+float time_lb_fp32(const LBView<float>& V, int twall, int shape, cudaStream_t s);
+float time_lb_fp64(const LBView<double>& V, int twall, int shape, cudaStream_t s);
 // two steps per launch (Dirichlet walls, no ghost rows): V1 = step n, V2 =
 // step n+1; job: particles of earlier steps advanced by the launch (tile
 // shapes only), or null

@@ -402,6 +402,37 @@ int tune_lb_fp32(const LBView<float>& V, int twall, cudaStream_t s, float* best_
   return tune<float>(V, twall, false, s, tune_reps(V), best_ms);
 }
 
+// ms per launch of one shape, storing what the view stores
+template <typename Real>
+static float time_lb(const LBView<Real>& V, int twall, int shape, cudaStream_t s) {
+  cudaEvent_t a, b;
+  cudaEventCreate(&a);
+  cudaEventCreate(&b);
+  const int reps = tune_reps(V);
+  float best = 1e30f;
+  for (int round = 0; round < 2; round++) {
+    for (int r = -1; r < reps; r++) {
+      if (r == 0) cudaEventRecord(a, s);
+      if constexpr (std::is_same<Real, double>::value) launch_lb_fp64(V, twall, false, shape, s, true);
+      else launch_lb_fp32(V, twall, shape, s, true);
+    }
+    cudaEventRecord(b, s);
+    cudaEventSynchronize(b);
+    float ms = 1e30f;
+    cudaEventElapsedTime(&ms, a, b);
+    best = std::min(best, ms);
+  }
+  cudaEventDestroy(a);
+  cudaEventDestroy(b);
+  return best / reps;
+}
+float time_lb_fp32(const LBView<float>& V, int twall, int shape, cudaStream_t s) {
+  return time_lb<float>(V, twall, shape, s);
+}
+float time_lb_fp64(const LBView<double>& V, int twall, int shape, cudaStream_t s) {
+  return time_lb<double>(V, twall, shape, s);
+}
+
 // two steps per launch: V1 is step n (its pops and F outputs unused), V2 step
 // n+1 (its pop and F inputs unused)
 cudaError_t launch_pair_fp32(const LBView<float>& V1, const LBView<float>& V2, int shape, cudaStream_t s, bool pdl,

@@ -424,6 +424,8 @@ struct Handle {
   double* adj_lam = nullptr;         // 2 x 18 lambda planes (ping-pong) + 2 lambda F planes
   long long* adj_lT = nullptr;       // 2 fixed-point lambda T planes (the steps of a pair)
   double* adj_T0 = nullptr;          // [ny*nx] initial temperature / gradient
+  int adj_fwd_shape = -1;            // the forward pass's two-step launch shape: -1 to choose, -2 single steps
+  float adj_fwd_ms = 0.f;
   int adj_pair_variant = -1;         // launch variant of the pair kernel (-1: tune at first use)
   void* adj_store = nullptr;         // every state's moment block (store mode)
   size_t adj_store_bytes = 0;
