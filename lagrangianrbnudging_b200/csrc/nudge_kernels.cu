@@ -40,14 +40,21 @@ enum { NB_OX = 0, NB_OY, NB_OT, NB_FX, NB_FY, NB_FT, NB_XINT, NB_YINT, NB_TINT, 
 enum { NBI_CHK = 0, NBI_BC, NBI_XIDX, NBI_YIDX, NBI_COUNT };
 
 // Contributions of a cell: the first BOX_SLOTS in the cell's own slots, the
-// rest in one list of (cell, key) for all cells.  A step's lists and counters
-// are one of three sets, by `seq` (a count of steps, from 1): this step's, the
-// last one's, and the one that this step leaves cleared for the next.  The
-// count is in device memory, so that replays of a captured step go on from the
-// step before them, whichever it was.  Each of its two words is written by the
-// kernel that does not read it.
-constexpr int BOX_SLOTS = 8;
-enum { BOX_NCELLS = 0, BOX_NOVER, BOX_NSORT, BOX_NCOUNT = 4 };
+// rest in BOX_CHAINS chains of the cell, by turns, linked through `link` (a
+// contribution's place there: 4 key + its cell's number in its box, at most
+// 2 x 2 cells).  A chain's length follows from the cell's count, so heads and
+// links are never cleared, and a chain is read by a thread of its own: work in
+// proportion to a cell's own contributions, however many all cells have.
+// (A whole step with 100,000 observations: 123 us on 512x256 and 196 on
+// 1680x840; with one list for all cells, which every full cell searched, 1314
+// and 4228; with a count, a scan and a fill of all cells 149 and 204.)
+// A step's lists and counters are one of three sets, by `seq` (a count of
+// steps, from 1): this step's, the last one's, and the one that this step
+// leaves cleared for the next.  The count is in device memory, so that replays
+// of a captured step go on from the step before them, whichever it was.  Each
+// of its two words is written by the kernel that does not read it.
+constexpr int BOX_SLOTS = 8, BOX_CHAINS = 16;
+enum { BOX_NCELLS = 0, BOX_NSORT, BOX_NCOUNT = 4 };
 enum { BOX_PLACED = 3 * BOX_NCOUNT, BOX_PLACING, BOX_HEAD = 16 };  // words after the counters: steps done, begun
 
 struct BoxView {
@@ -63,7 +70,8 @@ struct BoxView {
   int* stamp;    // [ncell] the last step that touched a cell
   int* slots;    // [ncell][BOX_SLOTS]
   int* cells;    // [3][lcap] cells touched
-  int2* over;    // [12 n] (cell, key)
+  int* head;     // [ncell][BOX_CHAINS] newest entry of a chain
+  int* link;     // [12 n] the entry before it in its chain
   int* scratch;  // [2][12 n]
   int lcap;
   int* nudge_vol;
@@ -208,8 +216,12 @@ __global__ void __launch_bounds__(32) box_bin_kernel(const BoxView B) {
           B.stamp[c] = seq;
           B.cells[(size_t)set * B.lcap + atomicAdd(&cnt[BOX_NCELLS], 1)] = c;
         }
-        if (at < BOX_SLOTS) B.slots[(size_t)c * BOX_SLOTS + at] = key;
-        else B.over[atomicAdd(&cnt[BOX_NOVER], 1)] = make_int2(c, key);
+        if (at < BOX_SLOTS) {
+          B.slots[(size_t)c * BOX_SLOTS + at] = key;
+        } else {
+          const int e = 4 * key + 2 * (cy - ra) + (cx - ca);
+          B.link[e] = atomicExch(&B.head[(size_t)c * BOX_CHAINS + (at - BOX_SLOTS) % BOX_CHAINS], e);
+        }
       }
   }
 }
@@ -221,7 +233,7 @@ __global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B)
   pdl_wait();
   constexpr int NT = CELL * CELL;
   __shared__ int keys[BOX_SLOTS];
-  __shared__ int sh[2];
+  __shared__ int base;
   const int tid = threadIdx.x;
   // (the three sets' counts loaded with the step, not after it)
   const int seq = B.cnt[BOX_PLACING];
@@ -254,17 +266,18 @@ __global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B)
         __syncthreads();
       } else {
         // more than the slots hold: the cell's keys into scratch, then ranked there
-        if (tid == 0) {
-          sh[0] = atomicAdd(&B.cnt[set * BOX_NCOUNT + BOX_NSORT], cnt);
-          sh[1] = BOX_SLOTS;
-        }
+        if (tid == 0) base = atomicAdd(&B.cnt[set * BOX_NCOUNT + BOX_NSORT], cnt);
         __syncthreads();
-        int* raw = B.scratch + sh[0];
+        int* raw = B.scratch + base;
         int* sorted = raw + (size_t)12 * B.n;
-        for (int a = tid; a < BOX_SLOTS; a += NT) raw[a] = B.slots[(size_t)c * BOX_SLOTS + a];
-        const int nover = B.cnt[set * BOX_NCOUNT + BOX_NOVER];
-        for (int a = tid; a < nover; a += NT)
-          if (B.over[a].x == c) raw[atomicAdd(&sh[1], 1)] = B.over[a].y;
+        if (tid < BOX_SLOTS) raw[tid] = B.slots[(size_t)c * BOX_SLOTS + tid];
+        if (tid < BOX_CHAINS) {
+          int e = B.head[(size_t)c * BOX_CHAINS + tid];
+          for (int a = BOX_SLOTS + tid; a < cnt; a += BOX_CHAINS) {
+            raw[a] = e >> 2;
+            e = B.link[e];
+          }
+        }
         __syncthreads();
         for (int a = tid; a < cnt; a += NT) {
           const int key = raw[a];
@@ -297,10 +310,10 @@ __global__ void __launch_bounds__(CELL * CELL) box_cells_kernel(const BoxView B)
 }
 
 // ints of the cell lists for n observations over ncell cells: counters,
-// counts, stamps, slots, three lists, the overflow list, scratch
+// counts, stamps, slots, chain heads, three lists, links, scratch
 static size_t box_lcap(int n, int ncell) { return std::min((size_t)ncell, (size_t)12 * n); }
 size_t box_cell_ints(int n, int ncell) {
-  return BOX_HEAD + (size_t)ncell * (2 + BOX_SLOTS) + 3 * box_lcap(n, ncell) + (size_t)4 * 12 * n;
+  return BOX_HEAD + (size_t)ncell * (2 + BOX_SLOTS + BOX_CHAINS) + 3 * box_lcap(n, ncell) + (size_t)3 * 12 * n;
 }
 
 // `work`: box_cell_ints ints, zero at the start of the run
@@ -311,12 +324,13 @@ cudaError_t launch_box_nudge(double* nb, int* nbi, int n, int nx, int ny, int ny
   const size_t lcap = box_lcap(n, ncell);
   BoxView B{nb, nbi, n, nx, ny, nt, istep, ny_total, j0, ncx, ncell};
   B.cnt = work;
-  B.over = reinterpret_cast<int2*>(work + BOX_HEAD);
-  B.scratch = work + BOX_HEAD + (size_t)2 * 12 * n;
+  B.link = work + BOX_HEAD;
+  B.scratch = B.link + (size_t)12 * n;
   B.count = B.scratch + (size_t)2 * 12 * n;
   B.stamp = B.count + ncell;
   B.slots = B.stamp + ncell;
-  B.cells = B.slots + (size_t)ncell * BOX_SLOTS;
+  B.head = B.slots + (size_t)ncell * BOX_SLOTS;
+  B.cells = B.head + (size_t)ncell * BOX_CHAINS;
   B.lcap = (int)lcap;
   B.nudge_vol = nudge_vol;
   B.tempreadint = tempreadint;
