@@ -200,8 +200,8 @@ LBRB_API int lbrb_set_graph(lbrb_t *h, int mode);
  * of the same kind, as for autotune); lbrb_get_pair_shape reports it
  * (shape index, tile columns and rows, ms per launch; shape -1 before).
  * Runs without nudging also take four steps per launch where that is
- * timed faster than two two-step launches and the shape was not fixed by
- * lbrb_set_pair_shape: the same steps, again with identical results, while
+ * timed faster than two two-step launches and the pair shape was not fixed by
+ * lbrb_set_pair_shape (or where lbrb_set_quad_shape says so): the same steps, again with identical results, while
  * more than four steps of the call remain and at most one of the four is a
  * record step; never on a handle whose steps a caller has captured
  * (lbrb_set_graph).
@@ -221,6 +221,16 @@ LBRB_API int lbrb_set_pair_shape(lbrb_t *h, int shape);
 /* the number of launch shapes of the two-step kernel (0 .. n-1) */
 LBRB_API int lbrb_pair_shapes(void);
 LBRB_API int lbrb_get_pair_shape(const lbrb_t *h, int *shape, int *tile_x, int *tile_y, float *ms);
+/* fix the launch shape of the four-step kernel: 0 .. lbrb_quad_shapes() - 1,
+ * strips of 56 columns walked up chunks of rows for 1, 2 or 4 waves of warps,
+ * taken wherever the kernel applies (lbrb_set_pairs), beside a fixed pair shape
+ * too; -1: no four-step launches; -2 (the default): timed, and used where
+ * faster.  With particles it needs the memory of two more u, v slots; a run
+ * that cannot have it steps in pairs.  get: the shape in use (-1 none, -2 not
+ * timed yet) and its ms per launch (0 when set rather than timed). */
+LBRB_API int lbrb_set_quad_shape(lbrb_t *h, int shape);
+LBRB_API int lbrb_quad_shapes(void);
+LBRB_API int lbrb_get_quad_shape(const lbrb_t *h, int *shape, float *ms);
 /* Per-kernel device timing with CUDA events around each launch.  Classes:
  * 0 fused stream/collide, 1 particles, 2 nudging, 3 record copies.
  * lbrb_get_timing() waits, returns total milliseconds and launch counts per

@@ -55,6 +55,7 @@ EXPORTS = [
     "lbrb_slab_particles_count", "lbrb_slab_particles_get", "lbrb_slab_record_pending",
     "lbrb_slab_record_drain", "lbrb_slab_particle_format", "lbrb_slab_nudge",
     "lbrb_set_graph", "lbrb_set_pairs", "lbrb_set_pair_shape", "lbrb_get_pair_shape", "lbrb_pair_shapes",
+    "lbrb_set_quad_shape", "lbrb_get_quad_shape", "lbrb_quad_shapes",
 ]
 
 
@@ -172,6 +173,9 @@ def lib() -> C.CDLL:
         "lbrb_set_pair_shape": (C.c_int, [vp, C.c_int]),
         "lbrb_pair_shapes": (C.c_int, []),
         "lbrb_get_pair_shape": (C.c_int, [vp, ip, ip, ip, C.POINTER(C.c_float)]),
+        "lbrb_quad_shapes": (C.c_int, []),
+        "lbrb_set_quad_shape": (C.c_int, [vp, C.c_int]),
+        "lbrb_get_quad_shape": (C.c_int, [vp, ip, C.POINTER(C.c_float)]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(L, name)
@@ -527,6 +531,20 @@ class Run:
         sh, tx, ty, ms = C.c_int(), C.c_int(), C.c_int(), C.c_float()
         self._ck(lib().lbrb_get_pair_shape(self.h, C.byref(sh), C.byref(tx), C.byref(ty), C.byref(ms)))
         return {"shape": sh.value, "tile": [tx.value, ty.value], "tuned_ms": ms.value}
+
+    @staticmethod
+    def quad_shapes() -> int:
+        """launch shapes of the four-step kernel"""
+        return lib().lbrb_quad_shapes()
+
+    def set_quad_shape(self, shape: int):
+        """fixed launch shape of the four-step kernel (0 .. quad_shapes() - 1), -1: not used, or -2: timed on first use"""
+        self._ck(lib().lbrb_set_quad_shape(self.h, int(shape)))
+
+    def quad_shape(self):
+        sh, ms = C.c_int(), C.c_float()
+        self._ck(lib().lbrb_get_quad_shape(self.h, C.byref(sh), C.byref(ms)))
+        return {"shape": sh.value, "tuned_ms": ms.value}
 
     def set_timing(self, enable: bool):
         self._ck(lib().lbrb_set_timing(self.h, int(bool(enable))))

@@ -1376,7 +1376,8 @@ int lbrb_step(lbrb_t* h, int n) {
   };
   // four steps per launch where a timed launch beats two timed pair launches
   auto quads_ok = [&]() {
-    return step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 && !h->pair_fixed && !h->captured;
+    return step_pairs_ok(h) && h->p.nudge == LBRB_NUDGE_NONE && h->pair_shape >= 0 &&
+           (!h->pair_fixed || h->quad_fixed) && !h->captured;
   };
   auto tune_quads = [&]() -> int {
     h->quad_shape = -1;
@@ -1400,6 +1401,7 @@ int lbrb_step(lbrb_t* h, int n) {
       tuned_put(g_tuned_quad, h, sh, ms);
     }
     h->quad_shape = sh;
+    h->quad_ms = sh >= 0 ? ms : 0.f;
     return LBRB_OK;
   };
   bool graphs_on = graph_ok(h);  // (refined below for a caller's capture)
@@ -2887,6 +2889,24 @@ int lbrb_get_pair_shape(const lbrb_t* h, int* shape, int* tile_x, int* tile_y, f
   if (tile_x) *tile_x = sh < 0 ? 0 : TXS[sh];
   if (tile_y) *tile_y = sh < 0 ? 0 : TYS[sh];
   if (ms) *ms = window ? h->adj_fwd_ms : h->pair_ms;
+  return LBRB_OK;
+}
+
+int lbrb_quad_shapes(void) { return NUM_QUAD_SHAPES; }
+
+int lbrb_set_quad_shape(lbrb_t* h, int shape) {
+  if (!h || shape < -2 || shape >= NUM_QUAD_SHAPES)
+    return fail(h, LBRB_ERR_ARG, "set_quad_shape: shape must be -2 (tune), -1 (off) or a shape index");
+  h->quad_shape = shape;
+  h->quad_fixed = shape != -2;
+  h->quad_ms = 0.f;
+  return LBRB_OK;
+}
+
+int lbrb_get_quad_shape(const lbrb_t* h, int* shape, float* ms) {
+  if (!h) return LBRB_ERR_ARG;
+  if (shape) *shape = h->quad_shape;
+  if (ms) *ms = h->quad_ms;
   return LBRB_OK;
 }
 

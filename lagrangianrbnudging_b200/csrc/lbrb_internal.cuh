@@ -343,6 +343,8 @@ struct Handle {
   // (two pair launches are faster, or no memory for the u, v slots), else
   // the launch shape
   int quad_shape = -2;
+  float quad_ms = 0.f;
+  bool quad_fixed = false;  // lbrb_set_quad_shape chose quad_shape
   bool captured = false;  // a caller captured steps: single and two-step launches, three u, v slots (lbrb_step)
   int pair_save[3] = {0, 0, 0};  // y-slab pairs: cur, uvcur, uvprev before the launch
   int graph_mode = -1;
