@@ -178,6 +178,7 @@ __device__ __forceinline__ void equil_ref(double r1, double u, double v, double 
 // the correction step alone gives RN(x / c) for every x != 0 (r = 0 adds
 // nothing) and a zero for x = +-0.  Every quotient of the collision is used
 // this way: it is multiplied, squared, or added to a sum that is not a zero.
+// tests/test_div_sum.py checks it as div_const is checked.
 __device__ __forceinline__ double div_sum(double x, double c, double rc) {
   const double q0 = __dmul_rn(x, rc);
   return __fma_rn(__fma_rn(-q0, c, x), rc, q0);
