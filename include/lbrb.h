@@ -314,8 +314,10 @@ LBRB_API int lbrb_adjoint_set_obs(lbrb_t *h, int nobs_steps, const int *steps, i
 LBRB_API int lbrb_adjoint_window(lbrb_t *h, const double *T0, int nsteps, int checkpoint_every,
                                  double *J, double *dJdT0);
 /* Launch variant of the two-step adjoint kernel, 0 .. lbrb_adjoint_variants()-1:
- * 0-3 the tiled kernel (tile shape, threads, blocks per SM), 4 and up the
- * marching kernel (rows per group, blocks per SM, register prefetch, waves).
+ * the tiled kernel (tile, blocks per SM) 0: 32x4 4, 1: 32x4 6, 2: 32x8 2,
+ * 3: 32x8 3, 10: 32x6 2, 11: 32x16 1; the marching kernel (rows per group,
+ * blocks per SM, groups prefetched, waves of blocks) 4: 7 1 1 2, 5: 6 1 1 2,
+ * 6: 7 1 2 2, 7: 5 2 2 2, 8: 5 2 2 1, 9: 3 3 2 2.
  * -1 (the default): timed on the first step pair of the next window and the
  * fastest kept.  Every variant gives the same gradient, bit for bit. */
 LBRB_API int lbrb_adjoint_variants(void);

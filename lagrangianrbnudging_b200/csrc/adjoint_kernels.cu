@@ -739,10 +739,11 @@ static cudaError_t launch_march_t(const AdjPairView<Real>& P, int waves, cudaStr
   return launch_march_o<Real, RB, MINB, PRE, size_t>(P, waves, s);
 }
 
-// launch variants of the two-step adjoint: 0-3 the tiled pair kernel (tile
-// TX x TY, threads, min blocks per SM), 4-9 the marching kernel (rows per
-// group, blocks per SM, register prefetch; waves of blocks)
-constexpr int ADJ_NPAIR_VARIANTS = 10;
+// launch variants of the two-step adjoint: 0-3, 10, 11 the tiled pair kernel
+// (tile TX x TY, threads, min blocks per SM), 4-9 the marching kernel (rows per
+// group, blocks per SM, register prefetch; waves of blocks).  The indices are
+// the C-ABI's (lbrb_adjoint_set_variant): new variants go at the end.
+constexpr int ADJ_NPAIR_VARIANTS = 12;
 int adjoint_pair_variants() { return ADJ_NPAIR_VARIANTS; }
 
 // steps n and n-1 from the moment blocks (MB_PLANES planes: F, rho, u, v, T)
@@ -773,15 +774,17 @@ cudaError_t launch_adjoint_pair(bool fp32, int variant, const void* after_a, con
     P.lg_in = lg_in;
     P.lF_out = lF_out;
     switch (variant) {
-      case 1: return launch_pair_t<Real, 32, 6, 192, 2>(P, s);
+      case 1: return launch_pair_t<Real, 32, 4, 128, 6>(P, s);
       case 2: return launch_pair_t<Real, 32, 8, 256, 2>(P, s);
-      case 3: return launch_pair_t<Real, 32, 16, 512, 1>(P, s);
+      case 3: return launch_pair_t<Real, 32, 8, 256, 3>(P, s);
       case 4: return launch_march_t<Real, 7, 1, 1>(P, 2, s);
       case 5: return launch_march_t<Real, 6, 1, 1>(P, 2, s);
       case 6: return launch_march_t<Real, 7, 1, 2>(P, 2, s);
       case 7: return launch_march_t<Real, 5, 2, 2>(P, 2, s);
       case 8: return launch_march_t<Real, 5, 2, 2>(P, 1, s);
       case 9: return launch_march_t<Real, 3, 3, 2>(P, 2, s);
+      case 10: return launch_pair_t<Real, 32, 6, 192, 2>(P, s);
+      case 11: return launch_pair_t<Real, 32, 16, 512, 1>(P, s);
       default: return launch_pair_t<Real, 32, 4, 128, 4>(P, s);
     }
   };
