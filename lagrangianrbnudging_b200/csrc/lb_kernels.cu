@@ -408,7 +408,7 @@ static float time_lb(const LBView<Real>& V, int twall, int shape, cudaStream_t s
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
-  const int reps = tune_reps(V);
+  const int reps = std::max(3, tune_reps(V) / 5);  // (compared with twice its time: a coarse look)
   float best = 1e30f;
   for (int round = 0; round < 2; round++) {
     for (int r = -1; r < reps; r++) {
