@@ -242,8 +242,8 @@ struct AdjPairView {
 // Phase 1's lambda comes straight into the shared memory that its results
 // take: a thread starts the copies of all its ring nodes (both rounds) before
 // any arithmetic, and each result replaces the value it was made from.  The
-// launch is bound by latency and the L1 / shared-memory data path (78% busy):
-// 1024x512, window of 400 steps with FP32 forward, in ms: 13.4-13.7 on 32x8
+// launch is bound by latency at 16 warps per SM (L1 / shared-memory data path
+// 52% busy, DRAM 42%, issue 43%, FP64 28%): 1024x512, window of 400 steps with FP32 forward, in ms: 13.4-13.7 on 32x8
 // tiles; 14.1 with the first round through registers; 14.0-14.4 with each
 // lambda read from shared memory twice (fewer registers, more blocks); 14.8
 // with both rounds through registers, one after the other.

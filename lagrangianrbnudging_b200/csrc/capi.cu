@@ -80,10 +80,11 @@ static void tuned_put(std::map<TuneKey, TuneVal>& m, const lbrb_t* h, int shape,
 // four-step launches).  Steps use them and transfers the staging slots, never
 // both at once, so they take the staging memory where they fit (up to about
 // 8 M nodes in FP32, 4 M in FP64; xfer_units waits for the steps).  Larger runs
-// allocate them in the first call that uses them, if they take at most a
-// quarter of what is free, and give them back when that turns out not to use
-// them or when another allocation of the handle fails.  Without them a run
-// steps in pairs, each followed by its particles.
+// allocate them at creation (25 ms of a first call otherwise, at 4096x2048 in
+// FP64), if they take at most a quarter of what is free, and give them back to
+// an ensemble, when the launch shapes turn out not to use them, or when another
+// allocation of the handle fails.  Without them a run steps in pairs, each
+// followed by its particles.
 struct RelaxedCapture {  // (another thread's capture does not concern these allocations)
   cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
   RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&m); }
@@ -111,8 +112,8 @@ static bool ensure_spare(lbrb_t* h) {
   h->nuv = UV_SLOTS;
   return true;
 }
-static void release_spare(lbrb_t* h) {
-  if (!h->uv_extra) return;
+void release_spare(lbrb_t* h) {
+  if (!h->uv_extra) return;  // (staging memory stays)
   RelaxedCapture relaxed;
   cudaFree(h->uv_extra);  // (waits for what still reads them)
   h->uv_extra = nullptr;
@@ -421,6 +422,10 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
     }
   }
   h->nobs = p.nobs;
+  h->stage_slot = stage_slot_doubles(p);
+  h->staging_bytes = 2 * h->stage_slot * sizeof(double);
+  if (cudaMalloc(&h->staging, h->staging_bytes) != cudaSuccess) return done(LBRB_ERR_NOMEM);
+  if (h->np > 0 && p.twall == LBRB_TWALL_DIRICHLET && p.nudge == LBRB_NUDGE_NONE) ensure_spare(h);
   if (p.nudge == LBRB_NUDGE_REFBOX) {
     const int n = h->nobs;
     h->ncx = (p.nx + 7) / 8;
@@ -439,9 +444,6 @@ int lbrb_create(const lbrb_params* pin, lbrb_t** out) {
         dalloc(&h->nmask, (size_t)p.ny * (h->pitch / 32)))
       return done(LBRB_ERR_NOMEM);
   }
-  h->stage_slot = stage_slot_doubles(p);
-  h->staging_bytes = 2 * h->stage_slot * sizeof(double);
-  if (cudaMalloc(&h->staging, h->staging_bytes) != cudaSuccess) return done(LBRB_ERR_NOMEM);
   for (cudaEvent_t& ev : h->xfer_ev)
     if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return done(LBRB_ERR_CUDA);
   if (dalloc(&h->red, (size_t)red_blocks() * 6 + 8 + (size_t)p.ny * 9)) return done(LBRB_ERR_NOMEM);

@@ -210,6 +210,9 @@ inline int fail(lbrb_t* h, int code, const std::string& msg, cudaError_t e = cud
     if (e_ != cudaSuccess) return fail((h), LBRB_ERR_CUDA, #call, e_); \
   } while (0)
 
+// a run's spare u, v slots given back (capi.cu)
+void release_spare(lbrb_t* h);
+
 inline bool fp32(const lbrb_t* h) { return h->p.precision == LBRB_PREC_FP32_SHIFTED; }
 inline double T0_of(const lbrb_t* h) { return 0.5 * (h->p.Tup + h->p.Tdown); }
 

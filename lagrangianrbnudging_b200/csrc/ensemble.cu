@@ -598,6 +598,7 @@ int lbrb_ensemble_create(lbrb_t* const* members, int n, lbrb_ensemble_t** out) {
     c = cudaMemcpy(e->d_och, och.data(), och.size() * sizeof(int2), cudaMemcpyHostToDevice);
   if (c == cudaSuccess) c = cudaMemset(e->d_ctr, 0, 4 * sizeof(int));
   if (c != cudaSuccess) return bad(c);
+  for (int i = 0; i < n; i++) release_spare(members[i]);  // (an ensemble steps in three slots)
   *out = e;
   return LBRB_OK;
 }

@@ -334,7 +334,7 @@ cudaError_t launch_lb_fp32(const LBView<float>& V, int twall, int shape, cudaStr
 // overwrites: the other population buffer, the other F buffer and, when the
 // caller's view stores u, v (runs with particles), the u, v slot of the next
 // step; rho and T are not written.  Box-nudged FP64 steps update nud_term in
-// place and are not tuned (shape 0).
+// place and are not tuned (lbrb_step gives them a shape).
 template <typename Real>
 static int tune(const LBView<Real>& Vin, int twall, bool refnudge, cudaStream_t s, int reps,
                 float* best_ms) {

@@ -32,24 +32,29 @@ def free():
     return torch.cuda.mem_get_info()[0]
 
 
-def test_no_spare_slots_where_nothing_uses_them():
-    with run(64) as r:  # (the library's code on the device before anything is measured)
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_no_spare_slots_where_nothing_uses_them(precision):
+    """FP32: never, as they fit in the staging memory; FP64: not in an
+    ensemble, and not once the launch shapes leave them unused"""
+    plane = PLANE * (2 if precision == "fp64" else 1)
+    with run(64, precision=precision) as r:  # (the library's code on the device before anything is measured)
         r.step(3)
     start = free()
-    with run(0):
+    with run(0, precision=precision):
         plain = start - free()
     start = free()
-    with run(64) as a, run(64) as b:
-        assert start - free() < 2 * plain + PLANE  # created
+    with run(64, precision=precision) as a, run(64, precision=precision) as b:
+        if precision == "fp32":
+            assert start - free() < 2 * plain + plane  # created
         with lb.Ensemble([a, b]) as e:
             e.step(24)
             e.sync()
-        assert start - free() < 2 * plain + PLANE + (64 << 20)  # members (and the ensemble's own lists)
+        assert start - free() < 2 * plain + plane + (64 << 20)  # members (and the ensemble's own lists)
     start = free()
-    with run(64, 9) as r:  # two-step strips: particles in launches of their own
+    with run(64, 9, precision) as r:  # two-step strips: particles in launches of their own
         r.step(30)
         r.sync()
-        assert start - free() < plain + PLANE
+        assert start - free() < plain + plane
 
 
 def test_spare_slots_give_way():
