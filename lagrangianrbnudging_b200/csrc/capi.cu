@@ -1477,11 +1477,14 @@ int lbrb_step(lbrb_t* h, int n) {
     }
     if (!graphs && n - s >= 5 && quads) {
       // (a group with two record steps, or whose record would not fit in the
-      // ring, goes in pairs or single steps, which report the overflow)
+      // ring, goes in pairs or single steps, which report the overflow; so
+      // does one whose next step would report it: get_poststream rebuilds the
+      // last step of a pair, not of four)
+      auto records = [&](int q) { return h->np > 0 && h->p.noutconfig > 0 && (h->istep + q) % h->p.noutconfig == 0; };
       int need = 0;
-      for (int q = 1; q <= 4; q++)
-        need += h->np > 0 && h->p.noutconfig > 0 && (h->istep + q) % h->p.noutconfig == 0;
-      if (need <= 1 && h->rec_head - h->rec_tail + pend_recs() + need <= h->p.record_slots) {
+      for (int q = 1; q <= 4; q++) need += records(q);
+      const long held = h->rec_head - h->rec_tail + pend_recs() + need;
+      if (need <= 1 && held + records(5) <= h->p.record_slots) {
         const int rc = four();
         if (rc) return rc;
         s += 4;

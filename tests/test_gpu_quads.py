@@ -88,6 +88,40 @@ def test_particles_and_records(precision, nx, ny, every, beta):
             assert_launches(b, 9, 3)
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_full_ring_after_four_steps(precision):
+    """a call that a full record ring ends where a four-step launch would be
+    the last: the state that it leaves, post-stream populations included"""
+    nx, ny, n = 116, 40, 30
+    runs = []
+    for shape in (None, 0):
+        r = lb.Run(**lb.closure(nx, ny, Ra=1e5, Pr=1.0, U=0.05), precision=precision, nprtcl=n, noutconfig=8,
+                   record_slots=1)
+        r.set_graph(0)
+        r.set_pairs(0 if shape is None else 1)
+        if shape is not None:
+            r.set_pair_shape(0)
+            r.set_quad_shape(shape)
+        r.init_conduction(7, 5e-2)
+        rng = np.random.default_rng(7)
+        z = np.zeros(n)
+        r.set_particles(np.arange(n, dtype=np.int32), rng.uniform(0.5, nx, n), rng.uniform(1.0, ny, n), z, z,
+                        np.zeros(n, np.int32), z)
+        r.step(3)
+        with pytest.raises(lb.LbrbError):
+            r.step(30)  # records at 8 and 16; the ring holds one
+        runs.append(r)
+    a, b = runs
+    assert a.istep == b.istep == 15
+    for p, q in zip(a.get_poststream() + a.get_populations(), b.get_poststream() + b.get_populations()):
+        np.testing.assert_array_equal(q, p)
+    for p, q in zip(a.drain_records_array(), b.drain_records_array()):
+        np.testing.assert_array_equal(q, p)
+    same(a, b, (4, 3))
+    for r in runs:
+        r.close()
+
+
 def test_modes():
     assert lb.Run.quad_shapes() == 3
     with make("fp32", 256, 128, -1) as r:
