@@ -174,7 +174,8 @@ LBRB_API int lbrb_set_stream(lbrb_t *h, void *cuda_stream);
  * caller captures the handle's stream.
  * A caller's capture gets the launches themselves, single and two-step ones
  * (the launch shapes timed by direct calls before it; a capture makes no
- * trial launches).  A captured call of a multiple of 12 steps ends in the
+ * trial launches).  A captured call of a multiple of 12 steps (with bilinear
+ * nudging 6, 18, 30, ...: its last two steps go one per launch) ends in the
  * buffers that it started from, so its graph can be replayed any number of
  * times; after direct calls, capture again.  The handle's step count, records
  * and observation rows are those of the capture.  Once captured, a handle

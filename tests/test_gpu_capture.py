@@ -69,13 +69,17 @@ def test_box_nudged_interval(nt):
         del g
 
 
-def free_run(precision, nx, ny, kind):
+def free_run(precision, nx, ny, kind, rows=0):
     """kind: no particles, few tracers, or few inertial particles (d/dt reads
-    the u, v of the step before)"""
+    the u, v of the step before); rows: of a repeating series of observations"""
     n = 0 if kind == "none" else 96
+    kw = dict(nudge="bilinear", alpha=0.2, nobs=40, obs_cycle=1) if rows else {}
     r = lb.Run(**lb.closure(nx, ny, Ra=1e6, Pr=1.0, U=0.1), precision=precision, nprtcl=n,
-               beta=0.5 if kind == "inertial" else 0.0)
+               beta=0.5 if kind == "inertial" else 0.0, **kw)
     r.set_pairs(1)
+    if rows:
+        rng = np.random.default_rng(3)
+        r.nudge_obs(1, rng.uniform(0, nx, (rows, 40)), rng.uniform(1, ny, (rows, 40)), rng.uniform(-0.5, 0.5, (rows, 40)))
     r.init_conduction(11, 5e-2)
     if n:
         rng = np.random.default_rng(5)
@@ -125,5 +129,31 @@ def test_replays_after_tuned_calls(precision, nx, ny, kind, n, between):
         a.set_stream(None)
         b.set_pairs(0)
         b.step(total)
+        assert_same(a, b)
+        del g
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("kind", ["none", "inertial"])
+@pytest.mark.parametrize("n", [6, 18])
+@pytest.mark.parametrize("pairs", [0, 1])
+def test_nudged_replays(precision, kind, n, pairs):
+    """bilinear nudging toward a series that repeats every captured call"""
+    import torch
+
+    nx, ny = 128, 64
+    with free_run(precision, nx, ny, kind, rows=6) as a, free_run(precision, nx, ny, kind, rows=6) as b:
+        a.set_pairs(pairs)
+        stream = torch.cuda.Stream()
+        a.set_stream(stream.cuda_stream)
+        a.step(24)
+        g = capture(a, stream, n)
+        with torch.cuda.stream(stream):
+            for _ in range(3):
+                g.replay()
+        torch.cuda.synchronize()
+        a.set_stream(None)
+        b.set_pairs(0)
+        b.step(24 + 3 * n)
         assert_same(a, b)
         del g
