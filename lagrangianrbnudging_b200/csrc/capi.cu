@@ -170,8 +170,10 @@ static int xfer_units(lbrb_t* h, bool in, double* host, size_t unit, int ub, int
   double* slot[2] = {(double*)h->staging, (double*)h->staging + h->stage_slot};
   cudaEvent_t* copied = h->xfer_ev;
   cudaEvent_t* converted = h->xfer_ev + 2;
-  if (in && h->nuv == UV_SLOTS)  // (the staging memory may hold u, v slots of steps still running)
+  if (in && h->spare_busy) {  // (the staging memory may hold u, v slots of steps still running)
     for (int sl = 0; sl < 2; sl++) CK(h, cudaEventRecord(converted[sl], h->stream));
+    h->spare_busy = false;
+  }
   int c = 0;
   for (int u0 = ub; u0 < ue; u0 += per, c++) {
     const int u1 = std::min(ue, u0 + per), sl = c & 1;
@@ -927,6 +929,7 @@ int lbrb_step(lbrb_t* h, int n) {
   CK(h, cudaStreamIsCapturing(h->stream, &capture_status));
   const bool capturing = capture_status != cudaStreamCaptureStatusNone;
   h->captured = h->captured || capturing;
+  h->spare_busy = true;
   int s = 0;  // steps of the call queued so far
   if (h->lb_shape < 0) {
     // autotune the fused kernel's launch shape on this grid (trial launches

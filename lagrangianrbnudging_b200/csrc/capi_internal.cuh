@@ -162,6 +162,7 @@ using namespace lbrb;
 
 struct lbrb_s : public Handle {
   std::vector<int> h_ids;
+  bool spare_busy = false;  // steps (which may use the staging memory) since the last transfer to the device
   // timing: event pool and the (class, begin, end) marks of this window
   std::vector<cudaEvent_t> ev_pool;
   size_t ev_used = 0;
